@@ -195,6 +195,11 @@ struct sf_handle {
     float2* amc[2] = {nullptr, nullptr};
     int* pid[2] = {nullptr, nullptr};
     int cur = 0;
+    // slot-pair positions of the current buffer set, written by the sort stage;
+    // pairsFresh: no position was written since (the density pass checks)
+    float4* pairXY = nullptr;
+    float2* pairZ = nullptr;
+    bool pairsFresh = false;
     // per-substep arrays
     float4 *aux = nullptr, *flow = nullptr, *adh = nullptr, *avgadh = nullptr, *drag = nullptr, *acc = nullptr;
     float2* dp = nullptr;
@@ -202,6 +207,7 @@ struct sf_handle {
     float4* grec4 = nullptr;
     unsigned int *keys = nullptr, *cs = nullptr, *bcs = nullptr;
     unsigned char* bnear = nullptr;  // per cell: a boundary particle within the 27 cells
+    unsigned int* bcell = nullptr;   // per boundary particle: its cell
     unsigned int* nbrCnt = nullptr;
     int* bnbrCnt = nullptr;
     int* cnbrCnt = nullptr;
@@ -233,7 +239,10 @@ struct sf_handle {
     cudaEvent_t stateEvent[2] = {nullptr, nullptr};
     bool statePending[2] = {false, false};
     int64_t listGrowths = 0;
-    int block[kTunedPasses] = {kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign};
+    // the density pass runs fastest with 64-128 threads per block (256 / 275 us
+    // with 128 / 256 on the 1M embankment: smaller blocks even out the lengths
+    // of its walks)
+    int block[kTunedPasses] = {128, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign};
     int lanes = 1;  // threads per slot of the momentum passes and the adjoint pair kernels
     int densityStaged = 0;  // the one-lane density pass stages its candidates in shared memory (tuned)
     unsigned int* dProbe = nullptr;       // neighbour-count probe word
@@ -289,6 +298,7 @@ struct sf_handle {
         b.listsW.cs = cs;
         b.listsW.bcs = bcs;
         b.listsW.bnear = bnear;
+        b.listsW.bcell = bcell;
         b.listsW.M = totalSlots;
         b.listsW.cap = nbrCap;
         b.lists.cnt = nbrCnt;
@@ -303,6 +313,8 @@ struct sf_handle {
         b.lists.M = totalSlots;
         b.lists.cap = nbrCap;
         b.pos4 = pos[cur];
+        b.pairXY = pairXY;
+        b.pairZ = pairZ;
         b.vel4 = vel[cur];
         b.aux4 = aux;
         b.flow4 = flow;
@@ -369,6 +381,8 @@ struct sf_handle {
             devFree(amc[k]);
             devFree(pid[k]);
         }
+        devFree(pairXY);
+        devFree(pairZ);
         devFree(aux);
         devFree(flow);
         devFree(adh);
@@ -388,6 +402,7 @@ struct sf_handle {
         devFree(cs);
         devFree(bcs);
         devFree(bnear);
+        devFree(bcell);
         devFree(sc.keysAlt);
         devFree(sc.vals);
         devFree(sc.valsAlt);
@@ -425,7 +440,8 @@ sf_status runSort(sf_handle* h) {
     const int o = h->cur, t = 1 - h->cur;
     launchReorder(h->stream, h->totalSlots, perm, h->pos[o], h->vel[o], h->col[o], h->mat[o], h->amc[o], h->pid[o],
                   h->pos[t], h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t], h->sortedKeys, h->totalCells,
-                  h->cs);
+                  h->cs, h->pairXY, h->pairZ);
+    h->pairsFresh = true;
     h->cur = t;
     h->sorted = true;
     h->launches += 2 + l;
@@ -437,12 +453,22 @@ sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive) {
     PassBuffers b = h->buffers();
     switch (stage) {
     case SF_STAGE_SORT: return runSort(h);
-    case SF_STAGE_DENSITY: launchDensity(c, b); break;
+    case SF_STAGE_DENSITY:
+        if (!h->pairsFresh) {  // positions written since the sort (stages run by hand)
+            launchPairs2(h->stream, h->totalSlots, h->pos[h->cur], h->pairXY, h->pairZ);
+            h->launches += 1;
+            h->pairsFresh = true;
+        }
+        launchDensity(c, b);
+        break;
     case SF_STAGE_AVGFLOW: launchAvgFlow(c, b); break;
     case SF_STAGE_VOIDAGE_ADHESION: launchVoidageAdhesion(c, b); break;
     case SF_STAGE_SAND_MOMENTUM: launchSandMomentum(c, b); break;
     case SF_STAGE_WATER_MOMENTUM: launchWaterMomentum(c, b); break;
-    case SF_STAGE_INTEGRATE: launchIntegrate(c, b, timeArg, adaptive, h->captureStep ? h->dTimeArg : nullptr); break;
+    case SF_STAGE_INTEGRATE:
+        launchIntegrate(c, b, timeArg, adaptive, h->captureStep ? h->dTimeArg : nullptr);
+        h->pairsFresh = false;
+        break;
     default: return h->fail(SF_ERR_INVALID, "unknown stage");
     }
     h->launches += 1;
@@ -482,6 +508,7 @@ sf_status countNeighborsMax(sf_handle* h, unsigned* maxCount) {
     if (!sorted) {
         h->cur = cur;
         h->sorted = false;
+        h->pairsFresh = false;
     }
     return SF_OK;
 }
@@ -681,6 +708,8 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
         SF_ALLOC(h->amc[k], sizeof(float2) * M);
         SF_ALLOC(h->pid[k], sizeof(int) * M);
     }
+    SF_ALLOC(h->pairXY, F4 / 2);
+    SF_ALLOC(h->pairZ, sizeof(float2) * M / 2);
     SF_ALLOC(h->aux, F4);
     SF_ALLOC(h->flow, F4);
     SF_ALLOC(h->adh, F4);
@@ -717,6 +746,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
     SF_ALLOC(h->cs, sizeof(unsigned) * (size_t(h->totalCells) + 1));
     SF_ALLOC(h->bcs, sizeof(unsigned) * (size_t(h->totalCells) + 1));
     SF_ALLOC(h->bnear, std::max<size_t>(1, size_t(h->totalCells)));
+    SF_ALLOC(h->bcell, sizeof(unsigned) * std::max<size_t>(1, size_t(h->totalB)));
     SF_ALLOC(h->bpos, sizeof(float4) * std::max<size_t>(1, size_t(h->totalB)));
     SF_ALLOC(h->blabel, sizeof(int) * std::max<size_t>(1, size_t(h->totalB)));
     SF_ALLOC(h->dScenes, sizeof(SceneDev) * n_scenes);
@@ -738,6 +768,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
     std::vector<int> hpid(M, -1);
     std::vector<float4> hbpos(std::max(1, h->totalB), make_float4(0, 0, 0, 0));
     std::vector<int> hblabel(std::max(1, h->totalB), 0);
+    std::vector<unsigned> hbcell(std::max(1, h->totalB), 0);
     std::vector<unsigned> hbcs(size_t(h->totalCells) + 1, 0);
     std::vector<unsigned char> hbnear(std::max<size_t>(1, size_t(h->totalCells)), 0);
     std::vector<SceneState> hstate(n_scenes);
@@ -788,6 +819,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
             const int64_t o = order[i];
             hbpos[size_t(S.b_off + i)] = make_float4(in.bpos[3 * o], in.bpos[3 * o + 1], in.bpos[3 * o + 2], 0.f);
             hblabel[size_t(S.b_off + i)] = in.blabel ? in.blabel[o] : 0;
+            hbcell[size_t(S.b_off + i)] = unsigned(S.cell_off + bk[o]);
         }
         hstate[s].n = int(in.n);
         hstate[s].n_sub = 1;
@@ -804,6 +836,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
         up(h->pid[0], hpid.data(), sizeof(int) * M, "upload pid") ||
         up(h->bpos, hbpos.data(), sizeof(float4) * hbpos.size(), "upload bpos") ||
         up(h->blabel, hblabel.data(), sizeof(int) * hblabel.size(), "upload blabel") ||
+        up(h->bcell, hbcell.data(), sizeof(unsigned) * hbcell.size(), "upload bcell") ||
         up(h->bcs, hbcs.data(), sizeof(unsigned) * hbcs.size(), "upload bcs") ||
         up(h->bnear, hbnear.data(), hbnear.size(), "upload bnear") ||
         up(h->dScenes, h->hScenes.data(), sizeof(SceneDev) * n_scenes, "upload scenes") ||
@@ -923,6 +956,7 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
     h->launches += g.nodes;
     h->cur = 1 - h->cur;
     h->sorted = true;
+    h->pairsFresh = false;
     queueStateCopy(h);
     if (ms_out) {
         cudaEventRecord(e1, h->stream);
@@ -1011,6 +1045,7 @@ sf_status queueSubstepsFixed(sf_handle* h, float dt, int64_t n) {
         }
     }
     h->sorted = true;
+    h->pairsFresh = false;
     return SF_OK;
 }
 
@@ -1385,6 +1420,7 @@ sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
         }
     }
     const int c = h->cur;
+    if (field == SF_FIELD_POS) h->pairsFresh = false;
     float4* vec = order == SF_ORDER_SORTED ? vec3Array(h, field) : nullptr;
     if (vec && (reinterpret_cast<uintptr_t>(from) & 15u) == 0)
         kSetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
@@ -1511,6 +1547,7 @@ sf_status sf_add_sph_particles(sf_handle* h, int32_t scene, const float* pos3, i
         return SF_ERR_CUDA;
     h->n[scene] += n;
     h->nextId[scene] += n;
+    h->pairsFresh = false;
     return SF_OK;
 }
 
@@ -1552,6 +1589,7 @@ sf_status sf_reset_order(sf_handle* h) {
     }
     h->cur = t;
     h->sorted = false;
+    h->pairsFresh = false;
     return h->cuda(cudaGetLastError(), "reset order launch");
 }
 
@@ -1759,6 +1797,7 @@ size_t snapStride(const sf_handle* h) {
 }
 
 sf_status snapCopy(sf_handle* h, char* snap, bool save) {
+    if (!save) h->pairsFresh = false;
     const size_t M = size_t(h->totalSlots);
     const int c = h->cur;
     void* arrays[6] = {h->pos[c], h->vel[c], h->col[c], h->mat[c], h->amc[c], h->pid[c]};
@@ -1824,8 +1863,8 @@ PassBuffers slabBuffers(const sf_handle* h, const AdjSlab& s) {
     b.lists.ccnt = s.ccnt;
     b.lists.cnbr = s.cnbr;
     b.lists.cs = s.cs;
-    b.listsW = NbrListsW{s.cnt, s.nbr, s.bcnt, s.bnbr, s.ccnt, s.cnbr, s.cs, h->bcs, h->bnear, b.lists.M,
-                         h->nbrCap};
+    b.listsW = NbrListsW{s.cnt, s.nbr, s.bcnt, s.bnbr, s.ccnt, s.cnbr, s.cs, h->bcs, h->bnear, h->bcell,
+                         b.lists.M, h->nbrCap};
     b.pos4 = s.pos;
     b.vel4 = s.vel;
     b.aux4 = s.aux;
@@ -1922,6 +1961,7 @@ sf_status runSubstepStoreGraphed(sf_handle* h, float dt, int64_t t) {
     h->launches += g.nodes;
     h->cur = 1 - h->cur;
     h->sorted = true;
+    h->pairsFresh = false;
     return SF_OK;
 }
 

@@ -163,7 +163,7 @@ __device__ __forceinline__ void recordListNeed(const NbrListsW& L, unsigned int&
     if ((threadIdx.x & 31u) == unsigned(__ffs(active) - 1)) atomicMax(&need, m);
 }
 
-// Shared-memory staging of a block's stencil candidates (kDensity<true>).
+// Shared-memory staging of a block's stencil candidates (kDensityStaged).
 // The slots of a block are consecutive in the cell order, so their particles
 // lie in one or two (x, y) cell columns for nearly every block; for each such
 // source column the block copies the 9 stencil columns over the z-cells its
@@ -262,22 +262,246 @@ __device__ __forceinline__ int stageBlock(const SceneDev& S, const NbrListsW& L,
     return staged;
 }
 
+// ComputeSFPressureByTait_CUDA (cuda_wcsph_sf_solver_gpu.cuh:19-44) or
+// ComputeSFPressure_CUDA (cuda_sph_sf_solver_gpu.cuh:482-508) of one water particle.
+__device__ __forceinline__ float pressureOf(const SceneDev& S, float density) {
+    float pressure;
+    if (S.tait) {
+        pressure = S.stiff * (powf(density / S.rho0, 7.f) - 1.f);
+        if (pressure < 0.f) pressure *= S.neg_scale;
+    } else {
+        pressure = S.stiff * (density - S.rho0);
+        if (pressure < 0.f) pressure *= 1.f;
+    }
+    return pressure;
+}
+
+// ---- packed two-candidate reach test
+// fma.rn.f32x2 / add.rn.f32x2: two IEEE FP32 operations per instruction, each
+// half rounded like the scalar one.
+__device__ __forceinline__ unsigned long long pack2(float a, float b) {
+    unsigned long long r;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(a), "f"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+    unsigned long long r;
+    asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+    return r;
+}
+__device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigned long long b, unsigned long long c) {
+    unsigned long long r;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+    return r;
+}
+
+// Hits of one slot waiting to be appended: (first candidate, hit mask) of up
+// to kHitChunks chunks of 32 candidates, per thread.
+constexpr int kHitChunks = 12;
+
 // Builds the neighbour lists (sand / water / boundary, each in stencil
 // order, plus the sand-sand contact list) and computes the density, fused
 // with ComputeSFPressureByTait_CUDA (cuda_wcsph_sf_solver_gpu.cuh:19-44) or
 // ComputeSFPressure_CUDA (cuda_sph_sf_solver_gpu.cuh:482-508). The stencil is
 // walked as 9 contiguous ranges (the 3 z-cells of one (dx, dy) column are
 // adjacent in the sorted order), which visits the same particles in the same
-// order as the 27-cell loop with far fewer divergent loop exits. The walk
-// only appends list entries; the contact filter and the density sum then run
-// over the finished lists, where the lanes of a warp stay together.
-// The walk is bound by load latency: a register budget of 40 (6 blocks of
-// kSlotAlign threads per SM) buys occupancy that outweighs the few values it
-// moves to the stack. kStaged reads the candidates from the block's staged
-// copy (stageBlock, stageCap positions of dynamic shared memory; 48
-// registers, since its shared memory already bounds the resident blocks).
-template <bool kStaged>
-__global__ void __launch_bounds__(kSlotAlign, kStaged ? 5 : 6) kDensity(const SceneDev* __restrict__ scenes,
+// order as the 27-cell loop with far fewer divergent loop exits.
+//
+// Two phases per thread. The test phase only marks candidates in reach, 32 to
+// a mask, two per instruction (packed FP32 on the slot-pair positions, 12
+// bytes a candidate), and keeps each non-empty mask in shared memory. The hit
+// phase then takes the marks of all columns as one sequence: the lanes of a
+// warp have nearly equal totals (~33 of ~216 candidates) where their counts
+// per column differ by a factor of two, and everything done per neighbour
+// (append, contact filter, density term) uses one load of its position.
+//
+// Bounds and measurements (GB300, events; 1M embankment / 791k disturbed
+// column / 252k embankment): the test phase alone takes 135 us at 1M and is
+// held by the L1 data pipe (70% busy: every lane receives 12 bytes a
+// candidate, whether or not its neighbour lanes read the same one; the float4
+// positions would be 16), the hit phase by issue. One pass per column that
+// appended from each chunk's mask and walked its lists again for contacts and
+// density: 312 / 295 / 111 us; this form 256 / 232 / 82. Of that, the density
+// terms in the hit phase with the boundary terms merged by the end slot of
+// their cell (instead of 27 cell-table steps over both lists) gave 36 us at
+// 791k, where every water particle is near the floor, and list addresses from
+// 32-bit strides 20 us everywhere. 12 waiting chunks: with 16 the larger shared
+// memory costs L1 (286 us at 1M), with 10 the disturbed column drains in the
+// middle of the walk (304 us). 48 registers: with 40 the spills cost 281 us,
+// with 64 the occupancy 268 us at 1M.
+__global__ void __launch_bounds__(kSlotAlign, 5)
+    kDensity(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, SceneState* __restrict__ state,
+             NbrListsW L, const float4* __restrict__ pos4, const float4* __restrict__ pairXY,
+             const float2* __restrict__ pairZ, const float4* __restrict__ bpos4, float4* __restrict__ vel4,
+             float4* __restrict__ aux4) {
+    SF_SLOT_PROLOGUE
+    extern __shared__ uint2 sHits[];
+    if (slot == S.slot_off) state[sid].amax_bits = 0u;
+    const float4 pi4 = pos4[slot];
+    if (pi4.w == 0.f) return;
+    const float3 pi = xyz(pi4);
+    const int3 c = cellOf(S, pi);
+    const bool water = pi4.w > 0.f;
+    uint2* __restrict__ mine = sHits + threadIdx.x;
+    const int stride = blockDim.x;
+    const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, S.gz - 1) + 1;
+    // no boundary particle within the 27 cells: the boundary ranges are empty
+    const bool nearB = !L.bnear || L.bnear[S.cell_off + localHash(S, c)] != 0;
+    int cS = 0, cW = 0, bc = 0, cc = 0, nq = 0;
+    float d = pi4.w * S.W0;
+    // entry k of the slot's list: one 32 x 32 -> 64 bit multiply-add (the
+    // stride in bytes fits 31 bits: a slot takes over 600 B of device memory)
+    const int rowBytes = int(L.M) * 4;
+    auto entry = [&](unsigned* list, int k) -> unsigned& {
+        return *reinterpret_cast<unsigned*>(reinterpret_cast<char*>(list + slot) + (long long)k * rowBytes);
+    };
+    // boundary particles in reach, in stencil order
+    if (nearB) {
+#pragma unroll 1
+        for (int m = 0; m < 9; ++m) {
+            const int x = c.x + m / 3 - 1, y = c.y + m % 3 - 1;
+            if (x < 0 || x >= S.gx || y < 0 || y >= S.gy) continue;
+            const int cell = S.cell_off + (x * S.gy + y) * S.gz;
+            const unsigned bEnd = L.bcs[cell + z1];
+            for (unsigned j = L.bcs[cell + z0]; j < bEnd; ++j) {
+                if (!inReachFast(S, pi - xyz(bpos4[j]))) continue;
+                if (bc < kMaxBNbr) entry(L.bnbr, bc) = j;
+                ++bc;
+            }
+        }
+    }
+    // the next boundary neighbour's density term: it follows the water
+    // neighbours of its cell (the reference's order), i.e. those of the slots
+    // before bEnd, the end of the cell
+    int kb = 0;
+    unsigned bEnd = ~0u, bNext = 0u;
+    auto nextBoundary = [&]() {
+        if (kb < bc && kb < kMaxBNbr) {
+            bNext = entry(L.bnbr, kb);
+            bEnd = L.cs[L.bcell[bNext] + 1];
+        } else {
+            bEnd = ~0u;
+        }
+    };
+    auto boundaryTerm = [&]() {
+        const float4 bj = bpos4[bNext];
+        d += S.rho0 * fabsf(bj.w) * poly6(S, len3(pi - xyz(bj)));
+        ++kb;
+        nextBoundary();
+    };
+    if (water) nextBoundary();
+    // appends the waiting hits in order; water also sums its density (m_i W(0),
+    // then cell by cell the water and the boundary neighbours), sand its
+    // contacts (DEM + liquid-bridge reach, itself excluded)
+    auto drain = [&]() {
+        unsigned base = 0u, mask = 0u;
+        for (int q = 0;;) {
+            if (mask == 0u) {
+                if (q == nq) break;
+                const uint2 h = mine[q * stride];
+                ++q;
+                base = h.x;
+                mask = h.y;
+            }
+            const unsigned j = base + unsigned(__ffs(mask) - 1);
+            mask &= mask - 1u;
+            const float4 pj = pos4[j];
+            const float3 dij = pi - xyz(pj);
+            // the list overflows when its two parts meet: from then on
+            // nothing reads it, so the order of the two appends is free
+            const bool room = cS + cW < L.cap;
+            if (pj.w < 0.f) {
+                if (room) entry(L.nbr, cS) = j;
+                ++cS;
+                if (!water && j != unsigned(slot) && dot3(dij, dij) < S.dem_reach2) {
+                    if (cc < kMaxContact) entry(L.cnbr, cc) = j;
+                    ++cc;
+                }
+            } else {
+                if (room) entry(L.nbr, L.cap - 1 - cW) = j;
+                ++cW;
+                if (water) {
+                    while (j >= bEnd) boundaryTerm();
+                    d += pj.w * poly6(S, len3(dij));
+                }
+            }
+        }
+        nq = 0;
+    };
+    const unsigned long long nx = pack2(-pi.x, -pi.x), ny = pack2(-pi.y, -pi.y), nz = pack2(-pi.z, -pi.z),
+                             nr = pack2(-S.reach2, -S.reach2);
+    const ulonglong2* __restrict__ pxy = reinterpret_cast<const ulonglong2*>(pairXY);
+    const unsigned long long* __restrict__ pz = reinterpret_cast<const unsigned long long*>(pairZ);
+    // the column ranges are loaded one column ahead
+    auto range = [&](int m, unsigned& b, unsigned& e) {
+        const int x = c.x + m / 3 - 1, y = c.y + m % 3 - 1;
+        b = e = 0u;
+        if (x >= 0 && x < S.gx && y >= 0 && y < S.gy) {
+            const int cell = S.cell_off + (x * S.gy + y) * S.gz;
+            b = L.cs[cell + z0];
+            e = L.cs[cell + z1];
+        }
+    };
+    unsigned nextBeg, nextEnd;
+    range(0, nextBeg, nextEnd);
+#pragma unroll 1
+    for (int m = 0; m < 9; ++m) {
+        const unsigned jBeg = nextBeg, jEnd = nextEnd;
+        if (m < 8) range(m + 1, nextBeg, nextEnd);
+        // chunks of 32 candidates from an even slot on (a candidate before
+        // jBeg or behind jEnd is masked out)
+#pragma unroll 1
+        for (unsigned j0 = jBeg & ~1u; j0 < jEnd; j0 += 32u) {
+            const int n = int(min(32u, jEnd - j0)), pairs = (n + 1) >> 1;
+            const ulonglong2* __restrict__ q = pxy + (j0 >> 1);
+            const unsigned long long* __restrict__ qz = pz + (j0 >> 1);
+            unsigned rev = 0u;
+#pragma unroll 4
+            for (int t = 0; t < pairs; ++t) {
+                const ulonglong2 a = q[t];
+                const unsigned long long dx = add2(a.x, nx), dy = add2(a.y, ny), dz = add2(qz[t], nz);
+                const unsigned long long r = fma2(dx, dx, fma2(dy, dy, fma2(dz, dz, nr)));
+                rev = __funnelshift_l(unsigned(r), rev, 1);
+                rev = __funnelshift_l(unsigned(r >> 32), rev, 1);
+            }
+            // candidate t of the chunk ended at bit 2 * pairs - 1 - t
+            unsigned hit = __brev(rev) >> (32 - 2 * pairs);
+            if (n < 32) hit &= (1u << n) - 1u;
+            if (j0 < jBeg) hit &= ~1u;
+            if (hit) {
+                mine[nq * stride] = make_uint2(j0, hit);
+                if (++nq == kHitChunks) drain();
+            }
+        }
+    }
+    drain();
+    if (water)
+        while (kb < bc && kb < kMaxBNbr) boundaryTerm();
+    L.cnt[slot] = unsigned(min(cS, 0xFFFF)) | (unsigned(min(cW, 0xFFFF)) << 16);
+    L.bcnt[slot] = bc;
+    L.ccnt[slot] = cc;
+    // a list more than 7/8 full asks the host to grow the capacity before it
+    // overflows; a full one walks the stencil until then (same results,
+    // slower)
+    recordListNeed(L, state[sid].list_need, cS + cW);
+    float density, pressure = 0.f;
+    if (!water) {
+        density = S.rho1;
+    } else {
+        // more boundary neighbours than the list holds: the stencil is walked again
+        density = bc <= kMaxBNbr ? d : exactDensity(S, L, pi, pi4.w, pos4, bpos4);
+        pressure = pressureOf(S, density);
+    }
+    vel4[slot].w = density;
+    aux4[slot].x = pressure;
+}
+
+// kDensity with one pass per column that appends as it tests, from the block's
+// staged copy of its candidates (stageBlock, stageCap positions of dynamic
+// shared memory); the contact filter and the density sum run over the
+// finished lists. 48 registers: its shared memory already bounds the resident
+// blocks.
+__global__ void __launch_bounds__(kSlotAlign, 5) kDensityStaged(const SceneDev* __restrict__ scenes,
                                                                      const int* __restrict__ blockScene,
                                                                      SceneState* __restrict__ state, NbrListsW L,
                                                                      const float4* __restrict__ pos4,
@@ -289,8 +513,7 @@ __global__ void __launch_bounds__(kSlotAlign, kStaged ? 5 : 6) kDensity(const Sc
     __shared__ StageTable T;
     if (slot == S.slot_off) state[sid].amax_bits = 0u;
     const float4 pi4 = pos4[slot];
-    int staged = 0;
-    if constexpr (kStaged) staged = stageBlock(S, L, pos4, pi4.w != 0.f, cellOf(S, xyz(pi4)), T, sPos, stageCap);
+    const int staged = stageBlock(S, L, pos4, pi4.w != 0.f, cellOf(S, xyz(pi4)), T, sPos, stageCap);
     if (pi4.w == 0.f) return;
     const float3 pi = xyz(pi4);
     const int3 c = cellOf(S, pi);
@@ -301,8 +524,7 @@ __global__ void __launch_bounds__(kSlotAlign, kStaged ? 5 : 6) kDensity(const Sc
     int cS = 0, cW = 0, bc = 0;
     const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, S.gz - 1) + 1;
     // staged columns of this particle's source column
-    int src9 = 0;
-    if constexpr (kStaged) src9 = (staged == 2 && c.x * S.gy + c.y != T.red[0]) ? 9 : 0;
+    const int src9 = (staged == 2 && c.x * S.gy + c.y != T.red[0]) ? 9 : 0;
     // no boundary particle within the 27 cells: the boundary ranges are empty
     const bool nearB = !L.bnear || L.bnear[S.cell_off + localHash(S, c)] != 0;
 #pragma unroll 1
@@ -323,7 +545,7 @@ __global__ void __launch_bounds__(kSlotAlign, kStaged ? 5 : 6) kDensity(const Sc
             for (unsigned j0 = L.cs[base + z0]; j0 < jEnd; j0 += 32u) {
                 const int n = int(min(32u, jEnd - j0));
                 unsigned rev = 0u, srev = 0u;
-                if (kStaged && staged) {
+                if (staged) {
                     const int k = src9 + (dx + 1) * 3 + (dy + 1);
                     const float4* sp = sPos + (int(j0) + int(T.o[k]) - int(T.g[k]));
 #pragma unroll 4
@@ -414,13 +636,7 @@ __global__ void __launch_bounds__(kSlotAlign, kStaged ? 5 : 6) kDensity(const Sc
         // complete lists the stencil is walked again
         density = listed && bc <= kMaxBNbr ? listDensity(S, L, slot, cW, bc, pi, pi4.w, pos4, bpos4)
                                            : exactDensity(S, L, pi, pi4.w, pos4, bpos4);
-        if (S.tait) {
-            pressure = S.stiff * (powf(density / S.rho0, 7.f) - 1.f);
-            if (pressure < 0.f) pressure *= S.neg_scale;
-        } else {
-            pressure = S.stiff * (density - S.rho0);
-            if (pressure < 0.f) pressure *= 1.f;
-        }
+        pressure = pressureOf(S, density);
     }
     vel4[slot].w = density;
     aux4[slot].x = pressure;
@@ -634,13 +850,7 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     recordListNeed(L, state[sid].list_need, cS + cW);
     float pressure = 0.f;
     if (water) {
-        if (S.tait) {
-            pressure = S.stiff * (powf(density / S.rho0, 7.f) - 1.f);
-            if (pressure < 0.f) pressure *= S.neg_scale;
-        } else {
-            pressure = S.stiff * (density - S.rho0);
-            if (pressure < 0.f) pressure *= 1.f;
-        }
+        pressure = pressureOf(S, density);
     }
     vel4[slot].w = density;
     aux4[slot].x = pressure;
@@ -984,11 +1194,12 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
             // 14 positions per thread (a block of 128 consecutive slots
             // needs ~10.4 on the 1M embankment), within 48 KB per block
             const int cap = std::min(14 * c.block[kPassDensity], kDensityStageMax);
-            kDensity<true><<<grid(c, kPassDensity), c.block[kPassDensity], size_t(cap) * sizeof(float4), c.stream>>>(
+            kDensityStaged<<<grid(c, kPassDensity), c.block[kPassDensity], size_t(cap) * sizeof(float4), c.stream>>>(
                 c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4, cap);
         } else {
-            kDensity<false><<<grid(c, kPassDensity), c.block[kPassDensity], 0, c.stream>>>(
-                c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4, 0);
+            const size_t hits = size_t(kHitChunks) * c.block[kPassDensity] * sizeof(uint2);
+            kDensity<<<grid(c, kPassDensity), c.block[kPassDensity], hits, c.stream>>>(
+                c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4);
         }
         break;
     }

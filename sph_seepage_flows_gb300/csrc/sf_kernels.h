@@ -71,6 +71,7 @@ struct NbrListsW {
     const unsigned int* cs;
     const unsigned int* bcs;
     const unsigned char* bnear;
+    const unsigned int* bcell;  // cell of each boundary particle
     long long M;
     int cap;
 };
@@ -80,6 +81,10 @@ struct PassBuffers {
     NbrLists lists;
     NbrListsW listsW;
     float4* pos4;
+    // positions of slot pairs (2p, 2p + 1), written by the sort: (x0, x1, y0, y1)
+    // and (z0, z1), the operands of the density pass's packed reach tests
+    const float4* pairXY;
+    const float2* pairZ;
     float4* vel4;
     float4* aux4;
     float4* flow4;
@@ -167,10 +172,13 @@ void launchKeysHist(const LaunchCtx& c, int n, const float4* pos4, unsigned int*
 void launchCellStart(cudaStream_t s, int n, int nCells, const unsigned int* sortedKeys, unsigned int* cellStart);
 // Gather the persistent per-slot arrays into sorted order (n a multiple of
 // 32) and write the cell table cellStart of the sorted keys (as
-// launchCellStart) in the same launch.
+// launchCellStart) and the slot-pair positions in the same launch.
 void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4* pos, const float4* vel,
                    const float4* col, const float4* mat, const float2* amc, const int* pid, float4* posOut,
                    float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
-                   const unsigned int* sortedKeys, int nCells, unsigned int* cellStart);
+                   const unsigned int* sortedKeys, int nCells, unsigned int* cellStart, float4* pairXY,
+                   float2* pairZ);
+// The slot-pair positions of n slots (a multiple of 32), as launchReorder writes them.
+void launchPairs2(cudaStream_t s, int n, const float4* pos, float4* pairXY, float2* pairZ);
 
 }  // namespace sfg

@@ -346,12 +346,34 @@ __device__ __forceinline__ void fillCellRuns(unsigned int* __restrict__ cs, unsi
     }
 }
 
+// The positions of one slot pair in structure-of-arrays form, written by the
+// pair's two lanes (the whole warp calls it; slots are warp-aligned).
+__device__ __forceinline__ void writePair(int i, float4 p, float4* __restrict__ pairXY, float2* __restrict__ pairZ) {
+    const float qx = __shfl_xor_sync(0xffffffffu, p.x, 1), qy = __shfl_xor_sync(0xffffffffu, p.y, 1),
+                qz = __shfl_xor_sync(0xffffffffu, p.z, 1);
+    if (i & 1)
+        pairZ[i >> 1] = make_float2(qz, p.z);
+    else
+        pairXY[i >> 1] = make_float4(p.x, qx, p.y, qy);
+}
+
+__global__ void kPairs(int n, const float4* __restrict__ pos, float4* __restrict__ pairXY,
+                       float2* __restrict__ pairZ) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) writePair(i, pos[i], pairXY, pairZ);  // n is a multiple of 32: whole warps
+}
+
+void launchPairs2(cudaStream_t s, int n, const float4* pos, float4* pairXY, float2* pairZ) {
+    kPairs<<<(n + 255) / 256, 256, 0, s>>>(n, pos, pairXY, pairZ);
+}
+
 __global__ void kReorder(int n, const unsigned int* __restrict__ perm, const float4* __restrict__ pos,
                          const float4* __restrict__ vel, const float4* __restrict__ col,
                          const float4* __restrict__ mat, const float2* __restrict__ amc, const int* __restrict__ pid,
                          float4* __restrict__ posOut, float4* __restrict__ velOut, float4* __restrict__ colOut,
                          float4* __restrict__ matOut, float2* __restrict__ amcOut, int* __restrict__ pidOut,
-                         const unsigned int* __restrict__ sk, int nCells, unsigned int* __restrict__ cs) {
+                         const unsigned int* __restrict__ sk, int nCells, unsigned int* __restrict__ cs,
+                         float4* __restrict__ pairXY, float2* __restrict__ pairZ) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;  // n is a multiple of 32: whole warps stay
     // cell table (the lower bound of every cell in the sorted keys): index i
@@ -364,7 +386,9 @@ __global__ void kReorder(int n, const unsigned int* __restrict__ perm, const flo
     fillCellRuns(cs, i == 0 ? 0u : min(sk[i - 1], top) + 1u, k + 1u, unsigned(i));
     fillCellRuns(cs, k + 1u, i == n - 1 ? unsigned(nCells) + 1u : k + 1u, unsigned(n));
     const unsigned int o = perm[i];
-    posOut[i] = pos[o];
+    const float4 p = pos[o];
+    posOut[i] = p;
+    writePair(i, p, pairXY, pairZ);
     velOut[i] = vel[o];
     colOut[i] = col[o];
     matOut[i] = mat[o];
@@ -375,9 +399,10 @@ __global__ void kReorder(int n, const unsigned int* __restrict__ perm, const flo
 void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4* pos, const float4* vel,
                    const float4* col, const float4* mat, const float2* amc, const int* pid, float4* posOut,
                    float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
-                   const unsigned int* sortedKeys, int nCells, unsigned int* cellStart) {
+                   const unsigned int* sortedKeys, int nCells, unsigned int* cellStart, float4* pairXY,
+                   float2* pairZ) {
     kReorder<<<(n + 255) / 256, 256, 0, s>>>(n, perm, pos, vel, col, mat, amc, pid, posOut, velOut, colOut, matOut,
-                                            amcOut, pidOut, sortedKeys, nCells, cellStart);
+                                            amcOut, pidOut, sortedKeys, nCells, cellStart, pairXY, pairZ);
 }
 
 }  // namespace sfg
