@@ -642,16 +642,27 @@ __global__ void __launch_bounds__(kSlotAlign, 5) kDensityStaged(const SceneDev* 
     aux4[slot].x = pressure;
 }
 
+// Candidates per chunk of the lane-split density pass: short chunks, so that
+// the ~9 columns of ~24 candidates fill every lane of a round, and all loads
+// of a chunk are in flight at once (40k scene, 8 lanes: 52 us with chunks of
+// 32, 49 with 16, 48 with 8, which cost 2 us on the 20k column).
+constexpr int kLaneChunk = 16;
+
 // The density pass with G lanes per slot (small scenes), with lists, counts,
-// density and pressure identical to kDensity's. The 32-candidate chunks of
-// the stencil walk, in stencil order, are dealt round-robin to the lanes; in
-// each round every lane tests its chunk at the same time, and the round's
-// hits are appended at the positions a single thread would have given them
-// (prefix counts over the lanes in chunk order, then the rank within the
-// chunk). Boundary candidates and the entries of the contact filter are
-// dealt one per lane and ranked by a ballot; the water density folds the
-// round's terms in list order. The rare paths (water with boundary
-// neighbours, overflowed lists) run in lane 0.
+// density and pressure identical to kDensity's. The chunks of the stencil
+// walk, in stencil order, are dealt round-robin to the lanes; in each round
+// every lane tests its chunk at the same time, and the round's hits are
+// appended at the positions a single thread would have given them (prefix
+// counts over the lanes in chunk order, then the rank within the chunk).
+// Particles and boundary particles are walked the same way. The entries of
+// the contact filter are dealt one per lane and ranked by a ballot; the
+// density terms are evaluated G at a time and folded in order, the boundary
+// terms between the water terms by the end slot of their cell. Only
+// particles with more boundary neighbours than the list holds are left to
+// lane 0 alone. Bound by the latency of its chain of loads: 1,770 particles
+// 28.0 -> 17.6 us, 20k column 41 -> 33 (its flooded base is near the floor:
+// lane 0 used to fold all its water and boundary terms by cell-table steps),
+// 40k scene 52 -> 43.
 template <int G>
 __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __restrict__ scenes,
                                                             const int* __restrict__ blockScene,
@@ -668,130 +679,120 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     const bool water = pi4.w > 0.f;
     const long long M = L.M;
     unsigned* __restrict__ nb = L.nbr + slot;
+    unsigned* __restrict__ bnb = L.bnbr + slot;
     const unsigned lane = threadIdx.x & 31u, gbase = lane & ~unsigned(G - 1);
     const unsigned gmask = ((1u << G) - 1u) << gbase;
-    int cS = 0, cW = 0;
+    int cS = 0, cW = 0, bc = 0;
     const int z0 = max(c.z - 1, 0), z1 = min(c.z + 1, S.gz - 1) + 1;
-    unsigned myJ0 = 0u, myHit = 0u, mySand = 0u;
-    // appends the round's hits at their single-thread positions
-    auto flush = [&]() {
-        const int ns = __popc(myHit & mySand), nw = __popc(myHit & ~mySand);
-        int ps = ns, pw = nw;  // inclusive prefix over the lanes, in chunk order
-#pragma unroll
-        for (int o = 1; o < G; o <<= 1) {
-            const int ts = __shfl_up_sync(gmask, ps, o, G), tw = __shfl_up_sync(gmask, pw, o, G);
-            if (part >= o) {
-                ps += ts;
-                pw += tw;
-            }
-        }
-        ps -= ns;
-        pw -= nw;
-        for (unsigned m = myHit; m; m &= m - 1u) {
-            const int t = __ffs(m) - 1;
-            const unsigned low = myHit & ((1u << t) - 1u);
-            if (cS + cW + ps + pw + __popc(low) < L.cap) {  // the single thread's overflow test
-                if ((mySand >> t) & 1u)
-                    nb[(cS + ps + __popc(low & mySand)) * M] = myJ0 + unsigned(t);
-                else
-                    nb[(L.cap - 1 - (cW + pw + __popc(low & ~mySand))) * M] = myJ0 + unsigned(t);
-            }
-        }
-        // round totals: the last lane's inclusive prefix
-        cS += __shfl_sync(gmask, ps + ns, int(gbase) + G - 1);
-        cW += __shfl_sync(gmask, pw + nw, int(gbase) + G - 1);
-        myHit = mySand = 0u;
-    };
-    // the 9 column ranges of the stencil (particles and boundary), loaded
-    // together up front: on a small scene the walk is a latency chain
-    // (the boundary ranges only where a boundary particle is within the 27
-    // cells; elsewhere they are empty)
+    // the 9 column ranges of the stencil, loaded together up front: on a small
+    // scene the walk is a latency chain (the boundary ranges only where a
+    // boundary particle is within the 27 cells; elsewhere they are empty)
     const bool nearB = !L.bnear || L.bnear[S.cell_off + localHash(S, c)] != 0;
-    unsigned cb[9], ce[9], bb[9], be[9];
-#pragma unroll
-    for (int m = 0; m < 9; ++m) {
-        const int x = c.x + m / 3 - 1, y = c.y + m % 3 - 1;
-        cb[m] = ce[m] = bb[m] = be[m] = 0u;
-        if (x >= 0 && x < S.gx && y >= 0 && y < S.gy) {
-            const int base = S.cell_off + (x * S.gy + y) * S.gz;
-            cb[m] = L.cs[base + z0];
-            ce[m] = L.cs[base + z1];
-            if (nearB) {
-                bb[m] = L.bcs[base + z0];
-                be[m] = L.bcs[base + z1];
-            }
-        }
-    }
-    // chunk q of the stencil order: column m with pre[m] <= q < pre[m + 1]
-    int pre[10];
-    pre[0] = 0;
-#pragma unroll
-    for (int m = 0; m < 9; ++m) pre[m + 1] = pre[m] + int((ce[m] - cb[m] + 31u) / 32u);
-    const int nq = pre[9];
-    // round r: lane part tests chunk r * G + part (all lanes at once)
-#pragma unroll 1
-    for (int r0 = 0; r0 < nq; r0 += G) {
-        const int qq = r0 + part;
-        if (qq < nq) {
-            unsigned j0 = 0u, jEnd = 0u;
-#pragma unroll
-            for (int m = 0; m < 9; ++m)
-                if (qq >= pre[m] && qq < pre[m + 1]) {
-                    j0 = cb[m] + 32u * unsigned(qq - pre[m]);
-                    jEnd = ce[m];
-                }
-            const int n = int(min(32u, jEnd - j0));
-            unsigned rev = 0u, srev = 0u;
-#pragma unroll 8
-            for (int t = 0; t < n; ++t) {
-                const float4 qv = pos4[j0 + unsigned(t)];
-                rev = __funnelshift_l(__float_as_uint(reachSign(S, pi - xyz(qv))), rev, 1);
-                srev = __funnelshift_l(__float_as_uint(qv.w), srev, 1);
-            }
-            if (n > 0) {  // always, as every chunk index maps to a non-empty column
-                myJ0 = j0;
-                myHit = __brev(rev) >> (32 - n);
-                mySand = __brev(srev) >> (32 - n);
-            }
-        }
-        flush();
-    }
-    __syncwarp(gmask);  // the group's list entries are visible to every lane
-    const bool listed = cS + cW <= L.cap;
-    int bc = 0;
-    {
-        // boundary candidates dealt to the lanes one at a time, in stencil
-        // order; a ballot ranks the hits
-        unsigned* __restrict__ bnb = L.bnbr + slot;
+    // walks the ranges of one cell table: test(j) gives the reach sign and
+    // the label sign of candidate j, append(first, hits, labelled) takes the
+    // hits of this lane's chunk of a round (every lane calls it)
+    auto walk = [&](const unsigned* __restrict__ table, auto&& test, auto&& append) {
+        unsigned cb[9];
+        int len[9], pre[10];
+        pre[0] = 0;
 #pragma unroll
         for (int m = 0; m < 9; ++m) {
-#pragma unroll 1
-            for (unsigned j0 = bb[m]; j0 < be[m]; j0 += unsigned(G)) {
-                const unsigned j = j0 + unsigned(part);
-                const bool in = j < be[m] && inReachFast(S, pi - xyz(bpos4[j]));
-                const unsigned ball = __ballot_sync(gmask, in) >> gbase;
-                if (in) {
-                    const int r = bc + __popc(ball & ((1u << part) - 1u));
-                    if (r < kMaxBNbr) bnb[r * M] = j;
-                }
-                bc += __popc(ball);
+            const int x = c.x + m / 3 - 1, y = c.y + m % 3 - 1;
+            cb[m] = 0u;
+            len[m] = 0;
+            if (x >= 0 && x < S.gx && y >= 0 && y < S.gy) {
+                const int base = S.cell_off + (x * S.gy + y) * S.gz;
+                cb[m] = table[base + z0];
+                len[m] = int(table[base + z1] - cb[m]);
             }
         }
-    }
+#pragma unroll
+        for (int m = 0; m < 9; ++m) pre[m + 1] = pre[m] + (len[m] + kLaneChunk - 1) / kLaneChunk;
+        // round r: lane part tests chunk r * G + part (all lanes at once);
+        // chunk q lies in the column m with pre[m] <= q < pre[m + 1]
+#pragma unroll 1
+        for (int r0 = 0; r0 < pre[9]; r0 += G) {
+            const int q = r0 + part;
+            unsigned j0 = 0u, hit = 0u, lab = 0u;
+            int n = 0;
+#pragma unroll
+            for (int m = 0; m < 9; ++m)
+                if (q >= pre[m] && q < pre[m + 1]) {
+                    j0 = cb[m] + unsigned(kLaneChunk * (q - pre[m]));
+                    n = min(kLaneChunk, len[m] - kLaneChunk * (q - pre[m]));
+                }
+            if (n > 0) {
+                unsigned rev = 0u, lrev = 0u;
+#pragma unroll
+                for (int t = 0; t < kLaneChunk; ++t) {
+                    const float2 s = test(j0 + unsigned(min(t, n - 1)));
+                    rev = __funnelshift_l(__float_as_uint(s.x), rev, 1);
+                    lrev = __funnelshift_l(__float_as_uint(s.y), lrev, 1);
+                }
+                // candidate t ended at bit kLaneChunk - 1 - t
+                const unsigned in = (1u << n) - 1u;
+                hit = (__brev(rev) >> (32 - kLaneChunk)) & in;
+                lab = __brev(lrev) >> (32 - kLaneChunk);
+            }
+            append(j0, hit, lab);
+        }
+    };
+    // inclusive prefix of v over the group's lanes
+    auto prefix = [&](int v) {
+#pragma unroll
+        for (int o = 1; o < G; o <<= 1) {
+            const int t = __shfl_up_sync(gmask, v, o, G);
+            if (part >= o) v += t;
+        }
+        return v;
+    };
+    walk(
+        L.cs,
+        [&](unsigned j) {
+            const float4 q = pos4[j];
+            return make_float2(reachSign(S, pi - xyz(q)), q.w);
+        },
+        [&](unsigned j0, unsigned hit, unsigned sand) {
+            // sand and water counts share one prefix sum (16 bits each: a
+            // round has at most G * kLaneChunk hits)
+            const int mine = __popc(hit & sand) | (__popc(hit & ~sand) << 16);
+            const int incl = prefix(mine), before = incl - mine;
+            const int ps = cS + (before & 0xffff), pw = cW + (before >> 16);
+            for (unsigned m = hit; m; m &= m - 1u) {
+                const int t = __ffs(m) - 1;
+                const unsigned low = hit & ((1u << t) - 1u);
+                const int ks = ps + __popc(low & sand), kw = pw + __popc(low & ~sand);
+                if (ks + kw < L.cap)  // the single thread's overflow test
+                    nb[((sand >> t) & 1u ? ks : L.cap - 1 - kw) * M] = j0 + unsigned(t);
+            }
+            const int total = __shfl_sync(gmask, incl, int(gbase) + G - 1);
+            cS += total & 0xffff;
+            cW += total >> 16;
+        });
+    if (nearB)
+        walk(
+            L.bcs, [&](unsigned j) { return make_float2(reachSign(S, pi - xyz(bpos4[j])), 0.f); },
+            [&](unsigned j0, unsigned hit, unsigned) {
+                const int incl = prefix(__popc(hit));
+                int k = bc + incl - __popc(hit);
+                for (unsigned m = hit; m; m &= m - 1u, ++k)
+                    if (k < kMaxBNbr) bnb[k * M] = j0 + unsigned(__ffs(m) - 1);
+                bc += __shfl_sync(gmask, incl, int(gbase) + G - 1);
+            });
+    __syncwarp(gmask);  // the group's list entries are visible to every lane
+    const bool listed = cS + cW <= L.cap;
     int cc = 0;
     if (!water) {
         unsigned* __restrict__ cnb = L.cnbr + slot;
         if (listed) {
+            unsigned jn = part < cS ? nb[part * M] : unsigned(slot);  // a round ahead
             for (int k0 = 0; k0 < cS; k0 += G) {
-                const int k = k0 + part;
+                const unsigned j = jn;
+                if (k0 + G + part < cS) jn = nb[(k0 + G + part) * M];
                 bool in = false;
-                unsigned j = 0u;
-                if (k < cS) {
-                    j = nb[k * M];
-                    if (j != unsigned(slot)) {
-                        const float3 dij = pi - xyz(pos4[j]);
-                        in = dot3(dij, dij) < S.dem_reach2;
-                    }
+                if (k0 + part < cS && j != unsigned(slot)) {
+                    const float3 dij = pi - xyz(pos4[j]);
+                    in = dot3(dij, dij) < S.dem_reach2;
                 }
                 const unsigned ball = __ballot_sync(gmask, in) >> gbase;
                 if (in) {
@@ -818,26 +819,55 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     }
     float density = S.rho1;
     if (water) {
-        if (listed && bc == 0) {
-            // m_i W(0), then the water list in order, G entries per round
+        if (listed && bc <= kMaxBNbr) {
+            // m_i W(0), then G water terms a round in list order; the G boundary
+            // terms at hand, with the end slots of their cells, go in before
+            // the first water neighbour behind them
             float d = pi4.w * S.W0;
             const unsigned* __restrict__ wp = L.nbr + slot + size_t(L.cap - 1) * M;
+            int kb = 0;
+            float bt = 0.f;
+            unsigned be = ~0u;
+            auto boundaryRound = [&]() {
+                be = ~0u;
+                if (kb + part < bc) {
+                    const unsigned b = bnb[(kb + part) * M];
+                    const float4 bj = bpos4[b];
+                    be = L.cs[L.bcell[b] + 1];
+                    bt = S.rho0 * fabsf(bj.w) * poly6(S, len3(pi - xyz(bj)));
+                }
+            };
+            if (bc > 0) boundaryRound();
+            unsigned beNext = __shfl_sync(gmask, be, int(gbase));
+            auto boundaryTerm = [&]() {
+                d += __shfl_sync(gmask, bt, int(gbase) + kb % G);
+                ++kb;
+                if (kb % G == 0) boundaryRound();
+                beNext = __shfl_sync(gmask, be, int(gbase) + kb % G);
+            };
+            unsigned jn = part < cW ? wp[-part * M] : 0u;  // a round ahead
             for (int k0 = 0; k0 < cW; k0 += G) {
+                const unsigned j = jn;
+                if (k0 + G + part < cW) jn = wp[-(k0 + G + part) * M];
                 float t = 0.f;
                 if (k0 + part < cW) {
-                    const float4 pj = pos4[wp[-(k0 + part) * M]];
+                    const float4 pj = pos4[j];
                     t = pj.w * poly6(S, len3(pi - xyz(pj)));
                 }
 #pragma unroll
                 for (int g = 0; g < G; ++g) {
                     const float u = __shfl_sync(gmask, t, int(gbase) + g);
-                    if (k0 + g < cW) d += u;
+                    const unsigned ju = __shfl_sync(gmask, j, int(gbase) + g);
+                    if (k0 + g < cW) {
+                        while (ju >= beNext) boundaryTerm();
+                        d += u;
+                    }
                 }
             }
+            while (kb < bc) boundaryTerm();
             density = d;
         } else if (part == 0) {
-            density = listed && bc <= kMaxBNbr ? listDensity(S, L, slot, cW, bc, pi, pi4.w, pos4, bpos4)
-                                               : exactDensity(S, L, pi, pi4.w, pos4, bpos4);
+            density = exactDensity(S, L, pi, pi4.w, pos4, bpos4);
         }
     }
     if (part != 0) return;
@@ -849,9 +879,7 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     // slower)
     recordListNeed(L, state[sid].list_need, cS + cW);
     float pressure = 0.f;
-    if (water) {
-        pressure = pressureOf(S, density);
-    }
+    if (water) pressure = pressureOf(S, density);
     vel4[slot].w = density;
     aux4[slot].x = pressure;
 }
