@@ -322,7 +322,8 @@ sf_status sf_set_tuning(sf_handle* h, int32_t block_size, int32_t items_per_thre
 /* Threads per particle of the neighbour passes and of the adjoint pair
  * kernels (no reference counterpart): 1, 2, 4 or 8, or 0 for the automatic
  * choice (doubled up to 8 while fewer than 2048 threads per SM would run,
- * i.e. 1 for large scenes). The density, average-flow and voidage/adhesion
+ * i.e. 1 for large scenes; the density and average-flow passes use 8 or 4
+ * only while no more than 1152 threads per SM run, else 1). The density, average-flow and voidage/adhesion
  * results and the neighbour lists are the same for every value; the
  * momentum sums are grouped differently (FP32 rounding only). Takes effect
  * at the next substep (captured graphs are dropped). */
@@ -347,15 +348,16 @@ sf_status sf_get_density_staging(const sf_handle* h, int32_t* staged);
  * particle, each neighbour pass with 64, 128 and 256 threads per block
  * (density, average flow, voidage/adhesion, sand momentum, water momentum;
  * the integrator keeps its size; with one thread per particle the density
- * pass with and without its shared-memory staging); it keeps the fastest sort tiles and the
- * lane count with the smallest sum of its passes' best times, with those
- * block sizes. The state is not advanced. block_sizes_out (6 entries, in
+ * pass with and without its shared-memory staging); it keeps the fastest sort tiles, the
+ * fastest lane count of each pass up to voidage/adhesion (their results do
+ * not depend on it) and the lane count with the smaller sum of the two
+ * momentum passes, with those block sizes. The state is not advanced. block_sizes_out (6 entries, in
  * that pass order then the integrator) and list_capacity_out may be NULL;
  * sf_get_tuning reads every choice back. */
 sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t* list_capacity_out);
 
 /* The current launch configuration (no reference counterpart): block sizes
- * (6 entries, as sf_autotune), threads per particle of the neighbour passes,
+ * (6 entries, as sf_autotune), threads per particle of the momentum passes,
  * keys per thread of the radix sort tiles and bits per radix digit (8, or
  * 9-11 where wider digits save a pass). Any pointer may be NULL. */
 sf_status sf_get_tuning(const sf_handle* h, int32_t* block_sizes_out, int32_t* lanes_out, int32_t* sort_items_out,

@@ -244,6 +244,8 @@ struct sf_handle {
     // of its walks)
     int block[kTunedPasses] = {128, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign};
     int lanes = 1;  // threads per slot of the momentum passes and the adjoint pair kernels
+    // threads per slot of the passes before them, whose results do not depend on it
+    int listLanes[3] = {1, 1, 1};  // density, average flow, voidage / adhesion
     int densityStaged = 0;  // the one-lane density pass stages its candidates in shared memory (tuned)
     unsigned int* dProbe = nullptr;       // neighbour-count probe word
     // reverse-mode buffers, allocated by the first sf_adjoint_run
@@ -283,7 +285,11 @@ struct sf_handle {
         c.errWord = dErr;
         c.slotBlocks = slotBlocks;
         for (int k = 0; k < kTunedPasses; ++k) c.block[k] = block[k];
-        c.lanes = lanes;
+        c.lanes[kPassDensity] = listLanes[0];
+        c.lanes[kPassAvgFlow] = listLanes[1];
+        c.lanes[kPassVoidage] = listLanes[2];
+        c.lanes[kPassSand] = c.lanes[kPassWater] = lanes;
+        c.lanes[kPassIntegrate] = 1;
         c.densityStaged = densityStaged;
         return c;
     }
@@ -329,6 +335,11 @@ struct sf_handle {
         b.vrec2 = vrec2;
         b.grec4 = grec4;
         return b;
+    }
+    void setLanes(int all) { lanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
+    void setAutomaticLanes(int smCount) {
+        setLanes(lanesForSlots(totalSlots, smCount));
+        listLanes[0] = listLanes[1] = listLanesForSlots(totalSlots, smCount);
     }
     // Drop the captured substep graphs (after a change of buffers or launch shapes).
     void dropGraphs() {
@@ -734,7 +745,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
             h->cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"))
             return bail(SF_ERR_CUDA);
         h->sc.items = sortItemsFor(h->totalSlots, sms);
-        h->lanes = lanesForSlots(h->totalSlots, sms);
+        h->setAutomaticLanes(sms);
     }
     h->sc.tiles = sortTiles(h->totalSlots, h->sc.items);
     // digits of 8 bits, or 9-11 when that saves a pass; room for the widest
@@ -1657,9 +1668,10 @@ sf_status sf_set_lanes(sf_handle* h, int32_t lanes) {
         if (h->cuda(cudaGetDevice(&dev), "cudaGetDevice") ||
             h->cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"))
             return SF_ERR_CUDA;
-        lanes = lanesForSlots(h->totalSlots, sms);
+        h->setAutomaticLanes(sms);
+    } else {
+        h->setLanes(lanes);
     }
-    h->lanes = lanes;
     h->dropGraphs();
     return SF_OK;
 }
@@ -1723,14 +1735,18 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
                                           SF_STAGE_SAND_MOMENTUM, SF_STAGE_WATER_MOMENTUM};
     for (int s = SF_STAGE_DENSITY; s <= SF_STAGE_WATER_MOMENTUM && st == SF_OK; ++s) st = runStage(h, s, dt, 0);
     // (with one lane the density pass is timed with and without its
-    // shared-memory staging as well)
-    float bestTotal = 0.f;
-    int bestLanes = h->lanes, bestBlock[kTunedPasses - 1], bestStaged = 0;
+    // shared-memory staging as well). The passes up to voidage / adhesion give
+    // the same results for every lane count, so each keeps its own fastest;
+    // the two momentum passes share the one of their smaller sum.
+    constexpr int kFirstMomentum = kPassSand;
+    float bestMomentum = 0.f, bestList[kFirstMomentum] = {};
+    int bestLanes = h->lanes, bestListLanes[kFirstMomentum], bestBlock[kTunedPasses - 1], bestStaged = 0;
     for (int p = 0; p < kTunedPasses - 1; ++p) bestBlock[p] = h->block[p];
+    for (int p = 0; p < kFirstMomentum; ++p) bestListLanes[p] = h->listLanes[p];
     for (int lanes : {1, 2, 4, 8}) {
         if (st) break;
-        h->lanes = lanes;
-        float total = 0.f;
+        h->setLanes(lanes);
+        float momentum = 0.f;
         int block[kTunedPasses - 1], staged = 0;
         for (int p = 0; p < kTunedPasses - 1 && st == SF_OK; ++p) {
             float best = 0.f;
@@ -1751,16 +1767,23 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
             }
             h->densityStaged = 0;
             h->block[p] = block[p];
-            total += best;
+            if (p >= kFirstMomentum) {
+                momentum += best;
+            } else if (st == SF_OK && (bestList[p] == 0.f || best < bestList[p])) {
+                bestList[p] = best;
+                bestListLanes[p] = lanes;
+                bestBlock[p] = block[p];
+                if (p == kPassDensity) bestStaged = staged;
+            }
         }
-        if (st == SF_OK && (bestTotal == 0.f || total < bestTotal)) {
-            bestTotal = total;
+        if (st == SF_OK && (bestMomentum == 0.f || momentum < bestMomentum)) {
+            bestMomentum = momentum;
             bestLanes = lanes;
-            bestStaged = staged;
-            for (int p = 0; p < kTunedPasses - 1; ++p) bestBlock[p] = block[p];
+            for (int p = kFirstMomentum; p < kTunedPasses - 1; ++p) bestBlock[p] = block[p];
         }
     }
     h->lanes = bestLanes;
+    for (int p = 0; p < kFirstMomentum; ++p) h->listLanes[p] = bestListLanes[p];
     h->densityStaged = bestStaged;
     for (int p = 0; p < kTunedPasses - 1; ++p) h->block[p] = bestBlock[p];
     cudaEventDestroy(e0);

@@ -1195,6 +1195,12 @@ int lanesForSlots(long long totalSlots, int smCount) {
     return g;
 }
 
+int listLanesForSlots(long long totalSlots, int smCount) {
+    for (int g = 8; g > 2; g /= 2)
+        if (totalSlots * g <= 1152LL * smCount) return g;
+    return 1;
+}
+
 // Blocks of a tuned pass over all slots.
 static inline int grid(const LaunchCtx& c, int pass) { return c.slotBlocks * (kSlotAlign / c.block[pass]); }
 
@@ -1213,7 +1219,7 @@ template <int G> void launchDensityLanes(const LaunchCtx& c, const PassBuffers& 
         c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4);
 }
 void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
-    switch (c.lanes) {
+    switch (c.lanes[kPassDensity]) {
     case 2: launchDensityLanes<2>(c, b); break;
     case 4: launchDensityLanes<4>(c, b); break;
     case 8: launchDensityLanes<8>(c, b); break;
@@ -1238,7 +1244,7 @@ template <int G> void launchAvgFlowG(const LaunchCtx& c, const PassBuffers& b) {
         c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4, b.flow4, b.vrec2, b.grec4);
 }
 void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b) {
-    switch (c.lanes) {
+    switch (c.lanes[kPassAvgFlow]) {
     case 2: launchAvgFlowG<2>(c, b); break;
     case 4: launchAvgFlowG<4>(c, b); break;
     case 8: launchAvgFlowG<8>(c, b); break;
@@ -1252,7 +1258,7 @@ template <int G> void launchVoidageAdhesionG(const LaunchCtx& c, const PassBuffe
         b.grec4);
 }
 void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b) {
-    switch (c.lanes) {
+    switch (c.lanes[kPassVoidage]) {
     case 2: launchVoidageAdhesionG<2>(c, b); break;
     case 4: launchVoidageAdhesionG<4>(c, b); break;
     case 8: launchVoidageAdhesionG<8>(c, b); break;

@@ -22,7 +22,7 @@ struct LaunchCtx {
     unsigned int* errWord;    // device error word
     int slotBlocks;           // total slots / kSlotAlign
     int block[kTunedPasses];  // threads per block of each tuned pass
-    int lanes;                // threads per slot of the momentum passes (1, 2, 4 or 8)
+    int lanes[kTunedPasses];  // threads per slot of each neighbour pass (1, 2, 4 or 8)
     int densityStaged;        // 1: the one-lane density pass stages its candidates in shared memory
 };
 
@@ -117,10 +117,16 @@ struct PassBuffers {
     float4* grec4;
 };
 
-// Threads per slot of the lane-split passes (momentum passes and the adjoint
-// pair kernels) for totalSlots slots on a GPU with smCount SMs: doubled, up
-// to 8, while fewer than 2048 threads per SM would run.
+// Threads per slot of the voidage / adhesion and momentum passes and of the
+// adjoint pair kernels for totalSlots slots on a GPU with smCount SMs:
+// doubled, up to 8, while fewer than 2048 threads per SM would run.
 int lanesForSlots(long long totalSlots, int smCount);
+// Threads per slot of the density and average-flow passes, whose one-lane
+// forms do the least work in all: 8 or 4 as long as no more than 1152 threads
+// per SM run, else 1. Density / average flow in us with 1, 4 and 8 lanes:
+// 20k column 64, 33, 33 / 25, 18, 14; 40k 45, 43, 49 / 18, 12, 13; 120k 65,
+// 92, 117 / 23, 29, 33; 252k 82, 223, 272 / 26, 47, 60 (2 lanes 226 / 47).
+int listLanesForSlots(long long totalSlots, int smCount);
 
 void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, const int* blabel,
                           const unsigned int* bcs);

@@ -214,7 +214,7 @@ template <int G> void launchSandMomentumG(const LaunchCtx& c, const PassBuffers&
         b.drag4, b.acc4);
 }
 void launchSandMomentum(const LaunchCtx& c, const PassBuffers& b) {
-    switch (c.lanes) {
+    switch (c.lanes[kPassSand]) {
     case 2: launchSandMomentumG<2>(c, b); break;
     case 4: launchSandMomentumG<4>(c, b); break;
     case 8: launchSandMomentumG<8>(c, b); break;
@@ -228,7 +228,7 @@ template <int G> void launchWaterMomentumG(const LaunchCtx& c, const PassBuffers
         b.acc4, c.errWord);
 }
 void launchWaterMomentum(const LaunchCtx& c, const PassBuffers& b) {
-    switch (c.lanes) {
+    switch (c.lanes[kPassWater]) {
     case 2: launchWaterMomentumG<2>(c, b); break;
     case 4: launchWaterMomentumG<4>(c, b); break;
     case 8: launchWaterMomentumG<8>(c, b); break;
