@@ -215,6 +215,9 @@ struct sf_handle {
     unsigned int *nbr = nullptr, *bnbr = nullptr;
     unsigned int* sortedKeys = nullptr;  // points into keys/scratch after a sort
     SortScratch sc{};
+    bool countingSort = false;  // by cell count and slot count (useCountingSort), else the radix sort
+    unsigned int *cellCount = nullptr, *tileCount = nullptr;
+    uint2* keyRank = nullptr;
     float4* bpos = nullptr;
     int* blabel = nullptr;
     // staging for field access
@@ -419,6 +422,9 @@ struct sf_handle {
         devFree(sc.valsAlt);
         devFree(sc.hist);
         devFree(sc.digitTotal);
+        devFree(cellCount);
+        devFree(keyRank);
+        devFree(tileCount);
         devFree(bpos);
         devFree(blabel);
         devFree(dScenes);
@@ -441,10 +447,24 @@ struct sf_handle {
 
 namespace {
 
-// The sort stage: keys (with the first radix pass's tile histograms), stable
-// radix sort, reorder into the other buffer set (with the cell table).
+// The sort stage: the counting sort by cell, or keys (with the first radix
+// pass's tile histograms), stable radix sort and reorder into the other buffer
+// set (with the cell table).
 sf_status runSort(sf_handle* h) {
     LaunchCtx c = h->ctx();
+    if (h->countingSort) {
+        const CountScratch cc{h->cellCount, h->tileCount, h->keyRank, h->sc.vals, h->keys,
+                              countTileShift(h->totalCells)};
+        const int o = h->cur, t = 1 - h->cur;
+        h->launches += launchCountingSort(c, h->totalSlots, h->totalCells, cc, h->pos[o], h->vel[o], h->col[o],
+                                          h->mat[o], h->amc[o], h->pid[o], h->pos[t], h->vel[t], h->col[t], h->mat[t],
+                                          h->amc[t], h->pid[t], h->cs, h->pairXY, h->pairZ);
+        h->sortedKeys = cc.sortedKeys;
+        h->pairsFresh = true;
+        h->cur = t;
+        h->sorted = true;
+        return h->cuda(cudaGetLastError(), "sort stage launch");
+    }
     launchKeysHist(c, h->totalSlots, h->pos[h->cur], h->keys, h->sc);
     unsigned int* perm = nullptr;
     int l = radixSort(h->stream, h->totalSlots, h->sortBits, h->keys, h->sc, &h->sortedKeys, &perm, true);
@@ -736,9 +756,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
     SF_ALLOC(h->bnbr, sizeof(unsigned) * M * kMaxBNbr);
     SF_ALLOC(h->cnbrCnt, sizeof(int) * M);
     SF_ALLOC(h->cnbr, sizeof(unsigned) * M * kMaxContact);
-    SF_ALLOC(h->sc.keysAlt, sizeof(unsigned) * M);
     SF_ALLOC(h->sc.vals, sizeof(unsigned) * M);
-    SF_ALLOC(h->sc.valsAlt, sizeof(unsigned) * M);
     {
         int dev = 0, sms = 0;
         if (h->cuda(cudaGetDevice(&dev), "cudaGetDevice") ||
@@ -752,8 +770,17 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
     // digits and the smallest tiles, so that the tuner can change both
     h->sc.digitBits = sortDigitBits(h->sortBits);
     const int maxRadix = 1 << std::max(8, h->sc.digitBits);
-    SF_ALLOC(h->sc.hist, sizeof(unsigned) * size_t(maxRadix) * size_t(sortTiles(h->totalSlots, 1)));
-    SF_ALLOC(h->sc.digitTotal, sizeof(unsigned) * size_t(maxRadix));
+    h->countingSort = useCountingSort(h->totalSlots, h->totalCells);
+    if (h->countingSort) {
+        SF_ALLOC(h->cellCount, sizeof(unsigned) * (size_t(h->totalCells) + 4));
+        SF_ALLOC(h->tileCount, sizeof(unsigned) * kMaxCountTiles);
+        SF_ALLOC(h->keyRank, sizeof(uint2) * M);
+    } else {
+        SF_ALLOC(h->sc.keysAlt, sizeof(unsigned) * M);
+        SF_ALLOC(h->sc.valsAlt, sizeof(unsigned) * M);
+        SF_ALLOC(h->sc.hist, sizeof(unsigned) * size_t(maxRadix) * size_t(sortTiles(h->totalSlots, 1)));
+        SF_ALLOC(h->sc.digitTotal, sizeof(unsigned) * size_t(maxRadix));
+    }
     SF_ALLOC(h->cs, sizeof(unsigned) * (size_t(h->totalCells) + 1));
     SF_ALLOC(h->bcs, sizeof(unsigned) * (size_t(h->totalCells) + 1));
     SF_ALLOC(h->bnear, std::max<size_t>(1, size_t(h->totalCells)));
@@ -1701,8 +1728,8 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
             return SF_ERR_CUDA;
         return SF_OK;
     };
-    // sort tile size and digit width: sorting the sorted state again is the identity
-    {
+    // radix sort: tile size and digit width (sorting the sorted state again is the identity)
+    if (!h->countingSort) {
         float best = 0.f;
         int bestItems = h->sc.items, bestDigit = h->sc.digitBits;
         const int wide = sortDigitBits(h->sortBits);

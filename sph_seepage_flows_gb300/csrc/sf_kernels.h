@@ -184,6 +184,30 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
                    float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
                    const unsigned int* sortedKeys, int nCells, unsigned int* cellStart, float4* pairXY,
                    float2* pairZ);
+// ---- counting sort by cell (sf_sort.cu) ----
+// Scratch of the counting sort; n: slots, a multiple of 256.
+struct CountScratch {
+    unsigned int* count;       // nCells rounded up to a multiple of 4, zero between sorts
+    unsigned int* tileCount;   // kMaxCountTiles: slots per table tile
+    uint2* keyRank;            // n: key of each slot before the sort, place among the slots counted into its cell
+    unsigned int* arrived;     // n: slots of each cell, in arrival order
+    unsigned int* sortedKeys;  // n: keys after the sort
+    int tileShift;             // log2 of the cells per table tile (countTileShift)
+};
+constexpr int kMaxCountTiles = 1024;
+// Whether the counting sort is used: its table passes cost 12 B per cell, which
+// stays behind the radix sort's cost while there are at most 8 cells per slot
+// (or a million cells, which the L2 holds).
+bool useCountingSort(int slots, int cells);
+// log2 of the cells per table tile: 1024 cells, doubled until at most
+// kMaxCountTiles tiles are left (every block of the scatter scans the tile sums).
+int countTileShift(int cells);
+// The sort stage in four launches: keys, cell table, stable order and gather of
+// the persistent arrays (with the slot-pair positions). Returns kernels launched.
+int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch& cc, const float4* pos,
+                       const float4* vel, const float4* col, const float4* mat, const float2* amc, const int* pid,
+                       float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
+                       unsigned int* cellStart, float4* pairXY, float2* pairZ);
 // The slot-pair positions of n slots (a multiple of 32), as launchReorder writes them.
 void launchPairs2(cudaStream_t s, int n, const float4* pos, float4* pairXY, float2* pairZ);
 
