@@ -479,7 +479,8 @@ sf_status runSort(sf_handle* h) {
     return h->cuda(cudaGetLastError(), "sort stage launch");
 }
 
-sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive) {
+// chained: called for one stage after the other of a whole substep.
+sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive, bool chained = false) {
     LaunchCtx c = h->ctx();
     PassBuffers b = h->buffers();
     switch (stage) {
@@ -492,7 +493,7 @@ sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive) {
         }
         launchDensity(c, b);
         break;
-    case SF_STAGE_AVGFLOW: launchAvgFlow(c, b); break;
+    case SF_STAGE_AVGFLOW: launchAvgFlow(c, b, chained); break;
     case SF_STAGE_VOIDAGE_ADHESION: launchVoidageAdhesion(c, b); break;
     case SF_STAGE_SAND_MOMENTUM: launchSandMomentum(c, b); break;
     case SF_STAGE_WATER_MOMENTUM: launchWaterMomentum(c, b); break;
@@ -508,7 +509,7 @@ sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive) {
 
 sf_status runSubstep(sf_handle* h, float timeArg, int adaptive) {
     for (int s = 0; s < SF_STAGE_COUNT; ++s) {
-        sf_status st = runStage(h, s, timeArg, adaptive);
+        sf_status st = runStage(h, s, timeArg, adaptive, true);
         if (st != SF_OK) return st;
     }
     return SF_OK;
@@ -1950,7 +1951,7 @@ sf_status runSubstepStore(sf_handle* h, float dt, const AdjSlab& s) {
     h->flow = s.flow;
     h->drag = s.drag;
     sf_status st = SF_OK;
-    for (int k = SF_STAGE_SORT; k <= SF_STAGE_WATER_MOMENTUM && st == SF_OK; ++k) st = runStage(h, k, dt, 0);
+    for (int k = SF_STAGE_SORT; k <= SF_STAGE_WATER_MOMENTUM && st == SF_OK; ++k) st = runStage(h, k, dt, 0, true);
     if (st == SF_OK) {
         launchAdjStore(h->ctx(), h->buffers(), h->pid[h->cur], s);
         h->launches += 1;

@@ -295,6 +295,16 @@ __device__ __forceinline__ unsigned long long fma2(unsigned long long a, unsigne
     return r;
 }
 
+// One sand neighbour's term of the sand volume around a particle
+// (ComputeSFSandVolume, cuda_sph_sf_solver_gpu.cuh:111-130): m_j / rho_j W(r),
+// with wj = -m_j and the sand density rho1 that this pass writes. vol is
+// m / rho1 of the sand particle with position w component wi; neighbours of
+// the same mass share the quotient.
+__device__ __forceinline__ float sandVolumeTerm(const SceneDev& S, float wj, float wi, float vol, float r) {
+    if (S.rho1 == 0.f) return 0.f;
+    return (wj == wi ? vol : -wj / S.rho1) * poly6(S, r);
+}
+
 // Hits of one slot waiting to be appended: (first candidate, hit mask) of up
 // to kHitChunks chunks of 32 candidates, per thread.
 constexpr int kHitChunks = 12;
@@ -348,7 +358,9 @@ __global__ void __launch_bounds__(kSlotAlign, 5)
     // no boundary particle within the 27 cells: the boundary ranges are empty
     const bool nearB = !L.bnear || L.bnear[S.cell_off + localHash(S, c)] != 0;
     int cS = 0, cW = 0, bc = 0, cc = 0, nq = 0;
-    float d = pi4.w * S.W0;
+    // water: density, sand: volume of the sand neighbours (itself included)
+    float sum = water ? pi4.w * S.W0 : 0.f;
+    const float vol = fabsf(pi4.w) / S.rho1;
     // entry k of the slot's list: one 32 x 32 -> 64 bit multiply-add (the
     // stride in bytes fits 31 bits: a slot takes over 600 B of device memory)
     const int rowBytes = int(L.M) * 4;
@@ -385,14 +397,15 @@ __global__ void __launch_bounds__(kSlotAlign, 5)
     };
     auto boundaryTerm = [&]() {
         const float4 bj = bpos4[bNext];
-        d += S.rho0 * fabsf(bj.w) * poly6(S, len3(pi - xyz(bj)));
+        sum += S.rho0 * fabsf(bj.w) * poly6(S, len3(pi - xyz(bj)));
         ++kb;
         nextBoundary();
     };
     if (water) nextBoundary();
     // appends the waiting hits in order; water also sums its density (m_i W(0),
     // then cell by cell the water and the boundary neighbours), sand its
-    // contacts (DEM + liquid-bridge reach, itself excluded)
+    // contacts (DEM + liquid-bridge reach, itself excluded) and the volume of
+    // the sand around it
     auto drain = [&]() {
         unsigned base = 0u, mask = 0u;
         for (int q = 0;;) {
@@ -413,16 +426,20 @@ __global__ void __launch_bounds__(kSlotAlign, 5)
             if (pj.w < 0.f) {
                 if (room) entry(L.nbr, cS) = j;
                 ++cS;
-                if (!water && j != unsigned(slot) && dot3(dij, dij) < S.dem_reach2) {
-                    if (cc < kMaxContact) entry(L.cnbr, cc) = j;
-                    ++cc;
+                if (!water) {
+                    const float d2 = dot3(dij, dij);
+                    if (j != unsigned(slot) && d2 < S.dem_reach2) {
+                        if (cc < kMaxContact) entry(L.cnbr, cc) = j;
+                        ++cc;
+                    }
+                    sum += sandVolumeTerm(S, pj.w, pi4.w, vol, sqrtf(d2));
                 }
             } else {
                 if (room) entry(L.nbr, L.cap - 1 - cW) = j;
                 ++cW;
                 if (water) {
                     while (j >= bEnd) boundaryTerm();
-                    d += pj.w * poly6(S, len3(dij));
+                    sum += pj.w * poly6(S, len3(dij));
                 }
             }
         }
@@ -489,11 +506,15 @@ __global__ void __launch_bounds__(kSlotAlign, 5)
         density = S.rho1;
     } else {
         // more boundary neighbours than the list holds: the stencil is walked again
-        density = bc <= kMaxBNbr ? d : exactDensity(S, L, pi, pi4.w, pos4, bpos4);
+        density = bc <= kMaxBNbr ? sum : exactDensity(S, L, pi, pi4.w, pos4, bpos4);
         pressure = pressureOf(S, density);
     }
     vel4[slot].w = density;
-    aux4[slot].x = pressure;
+    float4& aux = aux4[slot];
+    if (water)
+        aux.x = pressure;
+    else
+        *reinterpret_cast<float2*>(&aux) = make_float2(pressure, 1.f - sum);
 }
 
 // kDensity with one pass per column that appends as it tests, from the block's
@@ -782,17 +803,23 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     __syncwarp(gmask);  // the group's list entries are visible to every lane
     const bool listed = cS + cW <= L.cap;
     int cc = 0;
+    float sandVolume = 0.f;
     if (!water) {
         unsigned* __restrict__ cnb = L.cnbr + slot;
+        const float vol = -pi4.w / S.rho1;
         if (listed) {
             unsigned jn = part < cS ? nb[part * M] : unsigned(slot);  // a round ahead
             for (int k0 = 0; k0 < cS; k0 += G) {
                 const unsigned j = jn;
                 if (k0 + G + part < cS) jn = nb[(k0 + G + part) * M];
                 bool in = false;
-                if (k0 + part < cS && j != unsigned(slot)) {
-                    const float3 dij = pi - xyz(pos4[j]);
-                    in = dot3(dij, dij) < S.dem_reach2;
+                float t = 0.f;
+                if (k0 + part < cS) {
+                    const float4 pj = pos4[j];
+                    const float3 dij = pi - xyz(pj);
+                    const float d2 = dot3(dij, dij);
+                    in = j != unsigned(slot) && d2 < S.dem_reach2;
+                    t = sandVolumeTerm(S, pj.w, pi4.w, vol, sqrtf(d2));
                 }
                 const unsigned ball = __ballot_sync(gmask, in) >> gbase;
                 if (in) {
@@ -800,6 +827,11 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
                     if (r < kMaxContact) cnb[r * M] = j;
                 }
                 cc += __popc(ball);
+#pragma unroll
+                for (int g = 0; g < G; ++g) {
+                    const float u = __shfl_sync(gmask, t, int(gbase) + g);
+                    if (k0 + g < cS) sandVolume += u;
+                }
             }
         } else if (part == 0) {
             for (int x = max(c.x - 1, 0); x <= min(c.x + 1, S.gx - 1); ++x)
@@ -807,12 +839,14 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
                     const int base = S.cell_off + (x * S.gy + y) * S.gz;
                     for (unsigned j = L.cs[base + z0]; j < L.cs[base + z1]; ++j) {
                         const float4 pj = pos4[j];
-                        if (!(pj.w < 0.f) || !inReachFast(S, pi - xyz(pj)) || j == unsigned(slot)) continue;
+                        if (!(pj.w < 0.f) || !inReachFast(S, pi - xyz(pj))) continue;
                         const float3 dij = pi - xyz(pj);
-                        if (dot3(dij, dij) < S.dem_reach2) {
+                        const float d2 = dot3(dij, dij);
+                        if (j != unsigned(slot) && d2 < S.dem_reach2) {
                             if (cc < kMaxContact) cnb[cc * M] = j;
                             ++cc;
                         }
+                        sandVolume += sandVolumeTerm(S, pj.w, pi4.w, vol, sqrtf(d2));
                     }
                 }
         }
@@ -882,6 +916,7 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     if (water) pressure = pressureOf(S, density);
     vel4[slot].w = density;
     aux4[slot].x = pressure;
+    if (!water) aux4[slot].y = 1.f - sandVolume;
 }
 
 // ------------------------------------------------------------ avg-flow stage
@@ -890,8 +925,12 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
 // disjoint accumulators, so one sweep keeps every sum's reference order.
 // Small scenes run G lanes per slot: the lanes share the term evaluations
 // and fold the terms in list order (forLabelNeighborsOrdered), so the sums
-// stay bit-identical.
-template <int G>
+// stay bit-identical. kSummed: the density pass, run just before on the same
+// state, left the fluid voidage of sand in aux.y, so sand has no sand
+// neighbours to visit (a stage run by itself sums them from the densities it
+// finds). That was most of this pass's work: 93 -> 30 us on
+// the 1M embankment, for 26 us more in the density pass.
+template <int G, bool kSummed>
 __global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restrict__ scenes,
                                                        const int* __restrict__ blockScene, NbrLists L,
                                                        const float4* __restrict__ pos4,
@@ -906,34 +945,36 @@ __global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restric
     float v_s = 0.f, v_w = 0.f, sand_volume = 0.f;
     float3 avg_s = mk3(0.f, 0.f, 0.f), avg_w = avg_s;
     // sand neighbours: sand volume (every i) and, for water i, the sand average flow
-    forLabelNeighborsOrdered<true, G, 6>(
-        S, L, slot, pi, pos4, part,
-        [&](int j) {
-            const float4 pj = pos4[j];
-            const float4 vj4 = vel4[j];
-            const float mj = -pj.w;
-            const float wij = poly6(S, len3(pi - xyz(pj)));
-            Terms<6> t;
-            t.v[0] = vj4.w != 0.f ? mj / vj4.w * wij : 0.f;
-            t.v[1] = vj4.w != 0.f ? 1.f : 0.f;
-            t.v[2] = t.v[3] = t.v[4] = t.v[5] = 0.f;
-            if (!sandI) {
-                const float vj = mj / vj4.w;
-                const float3 a = xyz(vj4) * vj * wij;
-                t.v[2] = a.x;
-                t.v[3] = a.y;
-                t.v[4] = a.z;
-                t.v[5] = vj * wij;
-            }
-            return t;
-        },
-        [&](const Terms<6>& t) {
-            if (t.v[1] != 0.f) sand_volume += t.v[0];
-            if (!sandI) {
-                avg_w += mk3(t.v[2], t.v[3], t.v[4]);
-                v_w += t.v[5];
-            }
-        });
+    if (!kSummed || !sandI) {
+        forLabelNeighborsOrdered<true, G, 6>(
+            S, L, slot, pi, pos4, part,
+            [&](int j) {
+                const float4 pj = pos4[j];
+                const float4 vj4 = vel4[j];
+                const float mj = -pj.w;
+                const float wij = poly6(S, len3(pi - xyz(pj)));
+                Terms<6> t;
+                t.v[0] = vj4.w != 0.f ? mj / vj4.w * wij : 0.f;
+                t.v[1] = vj4.w != 0.f ? 1.f : 0.f;
+                t.v[2] = t.v[3] = t.v[4] = t.v[5] = 0.f;
+                if (!sandI) {
+                    const float vj = mj / vj4.w;
+                    const float3 a = xyz(vj4) * vj * wij;
+                    t.v[2] = a.x;
+                    t.v[3] = a.y;
+                    t.v[4] = a.z;
+                    t.v[5] = vj * wij;
+                }
+                return t;
+            },
+            [&](const Terms<6>& t) {
+                if (t.v[1] != 0.f) sand_volume += t.v[0];
+                if (!sandI) {
+                    avg_w += mk3(t.v[2], t.v[3], t.v[4]);
+                    v_w += t.v[5];
+                }
+            });
+    }
     // water neighbours of sand i: the water average flow and the saturation
     if (sandI) {
         forLabelNeighborsOrdered<false, G, 4>(
@@ -969,7 +1010,7 @@ __global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restric
     const float bz = sandI ? bezier(S.adhG, v_s) : 0.f;
     flow4[slot] = make_float4(avg.x, avg.y, avg.z, bz);
     float4 a = aux4[slot];
-    a.y = 1.f - sand_volume;
+    if (!kSummed || !sandI) a.y = 1.f - sand_volume;
     a.z = v_s;
     a.w = a.y;  // the reference's voidage array holds the fluid voidage until the sand pass
     aux4[slot] = a;
@@ -1239,16 +1280,23 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
     }
 }
 
-template <int G> void launchAvgFlowG(const LaunchCtx& c, const PassBuffers& b) {
-    kAvgFlow<G><<<grid(c, kPassAvgFlow) * G, c.block[kPassAvgFlow], 0, c.stream>>>(
-        c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4, b.flow4, b.vrec2, b.grec4);
+template <int G> void launchAvgFlowG(const LaunchCtx& c, const PassBuffers& b, bool summed) {
+    const int blocks = grid(c, kPassAvgFlow) * G, threads = c.block[kPassAvgFlow];
+    if (summed)
+        kAvgFlow<G, true><<<blocks, threads, 0, c.stream>>>(c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4,
+                                                            b.flow4, b.vrec2, b.grec4);
+    else
+        kAvgFlow<G, false><<<blocks, threads, 0, c.stream>>>(c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4,
+                                                             b.flow4, b.vrec2, b.grec4);
 }
-void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b) {
+void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b, bool chained) {
+    // the staged form of the density pass does not sum the sand volume
+    const bool summed = chained && !(c.lanes[kPassDensity] == 1 && c.densityStaged);
     switch (c.lanes[kPassAvgFlow]) {
-    case 2: launchAvgFlowG<2>(c, b); break;
-    case 4: launchAvgFlowG<4>(c, b); break;
-    case 8: launchAvgFlowG<8>(c, b); break;
-    default: launchAvgFlowG<1>(c, b); break;
+    case 2: launchAvgFlowG<2>(c, b, summed); break;
+    case 4: launchAvgFlowG<4>(c, b, summed); break;
+    case 8: launchAvgFlowG<8>(c, b, summed); break;
+    default: launchAvgFlowG<1>(c, b, summed); break;
     }
 }
 

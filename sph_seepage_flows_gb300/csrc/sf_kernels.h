@@ -131,7 +131,8 @@ int listLanesForSlots(long long totalSlots, int smCount);
 void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, const int* blabel,
                           const unsigned int* bcs);
 void launchDensity(const LaunchCtx& c, const PassBuffers& b);
-void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b);
+// chained: the density pass ran just before, with nothing set in between
+void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b, bool chained);
 void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b);
 void launchSandMomentum(const LaunchCtx& c, const PassBuffers& b);
 void launchWaterMomentum(const LaunchCtx& c, const PassBuffers& b);
