@@ -1118,17 +1118,37 @@ sf_status sf_substeps_fixed(sf_handle* h, float dt, int64_t n) {
 // ---------------------------------------------------------------- fields
 namespace {
 
-__global__ void kGetField(int field, int n, int slotOff, int cellOff, int order, const float4* __restrict__ pos,
-                          const float4* __restrict__ vel, const float4* __restrict__ col,
-                          const float4* __restrict__ mat, const float2* __restrict__ amc,
-                          const int* __restrict__ pid, const float4* __restrict__ aux, const float4* __restrict__ flow,
-                          const float4* __restrict__ adh, const float4* __restrict__ avgadh,
-                          const float4* __restrict__ drag, const float4* __restrict__ acc,
-                          const unsigned int* __restrict__ keys, const unsigned int* __restrict__ cnt, void* out) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int s = slotOff + i;
-    const int o = order == SF_ORDER_ID ? pid[s] : i;
+// The per-slot arrays behind the fields.
+struct FieldArrays {
+    float4 *pos, *vel, *col, *mat;
+    float2* amc;
+    int* pid;
+    float4 *aux, *flow, *adh, *avgadh, *drag, *acc;
+    float2 *dp, *vrec2;
+    float4* grec4;
+    const unsigned int *keys, *cnt;  // null before the first sort
+};
+
+FieldArrays fieldArrays(const sf_handle* h) {
+    const int c = h->cur;
+    return FieldArrays{h->pos[c], h->vel[c],  h->col[c],  h->mat[c], h->amc[c], h->pid[c],
+                       h->aux,    h->flow,    h->adh,     h->avgadh, h->drag,   h->acc,
+                       h->dp,     h->vrec2,   h->grec4,   h->sorted ? h->sortedKeys : nullptr,
+                       h->sorted ? h->nbrCnt : nullptr};
+}
+
+// The fields of one call that are moved by one launch (device buffers): a
+// launch costs the caller 2-4 us, more than the fields of a small scene take
+// (1,770 particles, four fields set and eight read: 33 us of launches, now 5;
+// 64 scenes of 17k, three read and four set each: 2.2 ms, now 0.5).
+constexpr int kFieldsPerLaunch = 16;
+struct FieldList {
+    int n;
+    int field[kFieldsPerLaunch];
+    void* buf[kFieldsPerLaunch];
+};
+
+__device__ __forceinline__ void getField(int field, int s, int o, int cellOff, const FieldArrays& A, void* out) {
     float* f = static_cast<float*>(out);
     int* iv = static_cast<int*>(out);
     auto put3 = [&](float4 v) {
@@ -1137,32 +1157,40 @@ __global__ void kGetField(int field, int n, int slotOff, int cellOff, int order,
         f[3 * o + 2] = v.z;
     };
     switch (field) {
-    case SF_FIELD_POS: put3(pos[s]); break;
-    case SF_FIELD_VEL: put3(vel[s]); break;
-    case SF_FIELD_ACC: put3(acc[s]); break;
-    case SF_FIELD_COL: put3(col[s]); break;
-    case SF_FIELD_LABEL: iv[o] = pos[s].w < 0.f ? SF_LABEL_SAND : SF_LABEL_WATER; break;
-    case SF_FIELD_RADIUS: f[o] = mat[s].w; break;
-    case SF_FIELD_MASS: f[o] = fabsf(pos[s].w); break;
-    case SF_FIELD_DENSITY: f[o] = vel[s].w; break;
-    case SF_FIELD_PRESSURE: f[o] = aux[s].x; break;
-    case SF_FIELD_VOIDAGE: f[o] = aux[s].w; break;
-    case SF_FIELD_SATURATION: f[o] = aux[s].z; break;
-    case SF_FIELD_MAX_SATURATION: f[o] = col[s].w; break;
-    case SF_FIELD_AVG_FLOW: put3(flow[s]); break;
-    case SF_FIELD_AVG_DRAG: put3(drag[s]); break;
-    case SF_FIELD_ADHESION: put3(adh[s]); break;
-    case SF_FIELD_AVG_ADHESION: put3(avgadh[s]); break;
-    case SF_FIELD_CDA0ASAT: put3(mat[s]); break;
+    case SF_FIELD_POS: put3(A.pos[s]); break;
+    case SF_FIELD_VEL: put3(A.vel[s]); break;
+    case SF_FIELD_ACC: put3(A.acc[s]); break;
+    case SF_FIELD_COL: put3(A.col[s]); break;
+    case SF_FIELD_LABEL: iv[o] = A.pos[s].w < 0.f ? SF_LABEL_SAND : SF_LABEL_WATER; break;
+    case SF_FIELD_RADIUS: f[o] = A.mat[s].w; break;
+    case SF_FIELD_MASS: f[o] = fabsf(A.pos[s].w); break;
+    case SF_FIELD_DENSITY: f[o] = A.vel[s].w; break;
+    case SF_FIELD_PRESSURE: f[o] = A.aux[s].x; break;
+    case SF_FIELD_VOIDAGE: f[o] = A.aux[s].w; break;
+    case SF_FIELD_SATURATION: f[o] = A.aux[s].z; break;
+    case SF_FIELD_MAX_SATURATION: f[o] = A.col[s].w; break;
+    case SF_FIELD_AVG_FLOW: put3(A.flow[s]); break;
+    case SF_FIELD_AVG_DRAG: put3(A.drag[s]); break;
+    case SF_FIELD_ADHESION: put3(A.adh[s]); break;
+    case SF_FIELD_AVG_ADHESION: put3(A.avgadh[s]); break;
+    case SF_FIELD_CDA0ASAT: put3(A.mat[s]); break;
     case SF_FIELD_AMCAMCP:
-        f[2 * o] = amc[s].x;
-        f[2 * o + 1] = amc[s].y;
+        f[2 * o] = A.amc[s].x;
+        f[2 * o + 1] = A.amc[s].y;
         break;
-    case SF_FIELD_ID: iv[o] = pid[s]; break;
-    case SF_FIELD_KEY: iv[o] = keys ? int(keys[s]) - cellOff : -1; break;
-    case SF_FIELD_NEIGHBORS: iv[o] = cnt ? int(cnt[s] & 0xFFFFu) + int(cnt[s] >> 16) : 0; break;
+    case SF_FIELD_ID: iv[o] = A.pid[s]; break;
+    case SF_FIELD_KEY: iv[o] = A.keys ? int(A.keys[s]) - cellOff : -1; break;
+    case SF_FIELD_NEIGHBORS: iv[o] = A.cnt ? int(A.cnt[s] & 0xFFFFu) + int(A.cnt[s] >> 16) : 0; break;
     default: break;
     }
+}
+
+__global__ void kGetFields(FieldList list, int n, int slotOff, int cellOff, int order, FieldArrays A) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int s = slotOff + i;
+    const int o = order == SF_ORDER_ID ? A.pid[s] : i;
+    for (int k = 0; k < list.n; ++k) getField(list.field[k], s, o, cellOff, A, list.buf[k]);
 }
 
 // The values the passes derive from a slot's fields for later passes (the
@@ -1190,14 +1218,8 @@ __device__ void refreshDerived(int s, const float4* pos, const float4* vel, cons
     }
 }
 
-__global__ void kSetField(int field, int n, int slotOff, int order, float4* pos, float4* vel, float4* col,
-                          float4* mat, float2* amc, const int* __restrict__ pid, float4* aux, float4* flow,
-                          float4* adh, float4* avgadh, float4* drag, float4* acc, float2* dp, float2* vrec2,
-                          float4* grec4, const void* in, const SceneDev* __restrict__ scene) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int s = slotOff + i;
-    const int o = order == SF_ORDER_ID ? pid[s] : i;
+__device__ __forceinline__ void setField(int field, int s, int o, const FieldArrays& A, const void* in,
+                                         const SceneDev& S) {
     const float* f = static_cast<const float*>(in);
     const int* iv = static_cast<const int*>(in);
     auto set3 = [&](float4* a) {
@@ -1208,37 +1230,47 @@ __global__ void kSetField(int field, int n, int slotOff, int order, float4* pos,
         a[s] = v;
     };
     switch (field) {
-    case SF_FIELD_POS: set3(pos); break;
-    case SF_FIELD_VEL: set3(vel); break;
-    case SF_FIELD_ACC: set3(acc); break;
-    case SF_FIELD_COL: set3(col); break;
+    case SF_FIELD_POS: set3(A.pos); break;
+    case SF_FIELD_VEL: set3(A.vel); break;
+    case SF_FIELD_ACC: set3(A.acc); break;
+    case SF_FIELD_COL: set3(A.col); break;
     case SF_FIELD_LABEL: {
-        const float m = fabsf(pos[s].w);
-        pos[s].w = iv[o] == SF_LABEL_SAND ? -m : m;
+        const float m = fabsf(A.pos[s].w);
+        A.pos[s].w = iv[o] == SF_LABEL_SAND ? -m : m;
         break;
     }
-    case SF_FIELD_RADIUS: mat[s].w = f[o]; break;
-    case SF_FIELD_MASS: pos[s].w = pos[s].w < 0.f ? -f[o] : f[o]; break;
-    case SF_FIELD_DENSITY: vel[s].w = f[o]; break;
-    case SF_FIELD_PRESSURE: aux[s].x = f[o]; break;
-    case SF_FIELD_VOIDAGE: aux[s].w = f[o]; aux[s].y = f[o]; break;
-    case SF_FIELD_SATURATION: aux[s].z = f[o]; break;
-    case SF_FIELD_MAX_SATURATION: col[s].w = f[o]; break;
-    case SF_FIELD_AVG_FLOW: set3(flow); break;
-    case SF_FIELD_AVG_DRAG: set3(drag); break;
-    case SF_FIELD_ADHESION: set3(adh); break;
-    case SF_FIELD_AVG_ADHESION: set3(avgadh); break;
-    case SF_FIELD_CDA0ASAT: set3(mat); break;
-    case SF_FIELD_AMCAMCP: amc[s] = make_float2(f[2 * o], f[2 * o + 1]); break;
+    case SF_FIELD_RADIUS: A.mat[s].w = f[o]; break;
+    case SF_FIELD_MASS: A.pos[s].w = A.pos[s].w < 0.f ? -f[o] : f[o]; break;
+    case SF_FIELD_DENSITY: A.vel[s].w = f[o]; break;
+    case SF_FIELD_PRESSURE: A.aux[s].x = f[o]; break;
+    case SF_FIELD_VOIDAGE: A.aux[s].w = f[o]; A.aux[s].y = f[o]; break;
+    case SF_FIELD_SATURATION: A.aux[s].z = f[o]; break;
+    case SF_FIELD_MAX_SATURATION: A.col[s].w = f[o]; break;
+    case SF_FIELD_AVG_FLOW: set3(A.flow); break;
+    case SF_FIELD_AVG_DRAG: set3(A.drag); break;
+    case SF_FIELD_ADHESION: set3(A.adh); break;
+    case SF_FIELD_AVG_ADHESION: set3(A.avgadh); break;
+    case SF_FIELD_CDA0ASAT: set3(A.mat); break;
+    case SF_FIELD_AMCAMCP: A.amc[s] = make_float2(f[2 * o], f[2 * o + 1]); break;
     default: break;
     }
     switch (field) {
     case SF_FIELD_VEL: case SF_FIELD_LABEL: case SF_FIELD_MASS: case SF_FIELD_DENSITY: case SF_FIELD_PRESSURE:
     case SF_FIELD_VOIDAGE: case SF_FIELD_SATURATION:
-        refreshDerived(s, pos, vel, aux, flow, avgadh, drag, dp, vrec2, grec4, *scene);
+        refreshDerived(s, A.pos, A.vel, A.aux, A.flow, A.avgadh, A.drag, A.dp, A.vrec2, A.grec4, S);
         break;
     default: break;
     }
+}
+
+// The fields of the list in order, each as if set by a call of its own.
+__global__ void kSetFields(FieldList list, int n, int slotOff, int order, FieldArrays A,
+                           const SceneDev* __restrict__ scene) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    const int s = slotOff + i;
+    const int o = order == SF_ORDER_ID ? A.pid[s] : i;
+    for (int k = 0; k < list.n; ++k) setField(list.field[k], s, o, A, list.buf[k], *scene);
 }
 
 int fieldWidth(int field) {
@@ -1364,20 +1396,49 @@ __global__ void kGetBoundary(int field, int n, int bOff, const float4* __restric
 
 namespace {
 
+// Whether a field call's arguments are valid; bytes: of the caller's buffer.
+sf_status checkField(sf_handle* h, int32_t scene, int32_t field, int32_t order, const void* buf, int64_t count,
+                     bool set, size_t* bytes) {
+    if (!h || !buf || scene < 0 || scene >= h->nScenes) return SF_ERR_INVALID;
+    const int w = fieldWidth(field);
+    if (set) {
+        if (w == 0 || field >= SF_BFIELD_POS || field == SF_FIELD_ID || field == SF_FIELD_KEY ||
+            field == SF_FIELD_NEIGHBORS)
+            return h->fail(SF_ERR_INVALID, "field cannot be set");
+    } else if (w == 0) {
+        return h->fail(SF_ERR_INVALID, "unknown field");
+    }
+    if (order != SF_ORDER_SORTED && order != SF_ORDER_ID) return h->fail(SF_ERR_INVALID, "unknown order");
+    const int64_t n = field >= SF_BFIELD_POS ? h->hScenes[scene].nb : h->n[scene];
+    if (count != n) return h->fail(SF_ERR_INVALID, "count must equal the scene's particle count");
+    *bytes = size_t(n) * size_t(w) * 4;
+    return SF_OK;
+}
+
+FieldList oneField(int field, const void* buf) {
+    FieldList l;
+    l.n = 1;
+    l.field[0] = field;
+    l.buf[0] = const_cast<void*>(buf);
+    return l;
+}
+
+sf_status launchGetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
+    const SceneDev& S = h->hScenes[scene];
+    kGetFields<<<int((n + 255) / 256), 256, 0, h->stream>>>(list, int(n), S.slot_off, S.cell_off, order,
+                                                           fieldArrays(h));
+    return h->cuda(cudaGetLastError(), "get_field launch");
+}
+
 // sf_get_field without its final host synchronisation (the copy is queued on
 // the handle's stream).
-sf_status getFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t order, void* dst, int64_t count,
+sf_status getFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t order, void* dst, int64_t n,
                          int32_t dst_on_device) {
-    if (!h || !dst || scene < 0 || scene >= h->nScenes) return SF_ERR_INVALID;
-    const int w = fieldWidth(field);
-    if (w == 0) return h->fail(SF_ERR_INVALID, "unknown field");
-    if (order != SF_ORDER_SORTED && order != SF_ORDER_ID) return h->fail(SF_ERR_INVALID, "unknown order");
+    size_t bytes = 0;
+    if (sf_status st = checkField(h, scene, field, order, dst, n, false, &bytes)) return st;
+    if (n == 0) return SF_OK;
     const SceneDev& S = h->hScenes[scene];
     const bool bfield = field >= SF_BFIELD_POS;
-    const int64_t n = bfield ? S.nb : h->n[scene];
-    if (count != n) return h->fail(SF_ERR_INVALID, "count must equal the scene's particle count");
-    const size_t bytes = size_t(n) * size_t(w) * 4;
-    if (n == 0) return SF_OK;
     void* target = dst;
     // pinned host memory in sorted order is written by the gather kernel
     // directly (coalesced); anything else goes through the device stage
@@ -1390,19 +1451,14 @@ sf_status getFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
             target = h->stage;
         }
     }
-    const int blocks = int((n + 255) / 256);
     float4* vec = bfield || order != SF_ORDER_SORTED ? nullptr : vec3Array(h, field);
     if (vec && (reinterpret_cast<uintptr_t>(target) & 15u) == 0) {
         kGetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
             int(n), S.slot_off, vec, static_cast<float4*>(target));
     } else if (bfield) {
-        kGetBoundary<<<blocks, 256, 0, h->stream>>>(field, int(n), S.b_off, h->bpos, h->blabel, target);
-    } else {
-        const int c = h->cur;
-        kGetField<<<blocks, 256, 0, h->stream>>>(field, int(n), S.slot_off, S.cell_off, order, h->pos[c], h->vel[c],
-                                                 h->col[c], h->mat[c], h->amc[c], h->pid[c], h->aux, h->flow,
-                                                 h->adh, h->avgadh, h->drag, h->acc, h->sorted ? h->sortedKeys : nullptr,
-                                                 h->sorted ? h->nbrCnt : nullptr, target);
+        kGetBoundary<<<int((n + 255) / 256), 256, 0, h->stream>>>(field, int(n), S.b_off, h->bpos, h->blabel, target);
+    } else if (launchGetFields(h, scene, oneField(field, target), order, n)) {
+        return SF_ERR_CUDA;
     }
     if (h->cuda(cudaGetLastError(), "get_field launch")) return SF_ERR_CUDA;
     if (!dst_on_device && !mapped &&
@@ -1423,28 +1479,51 @@ sf_status sf_get_field(sf_handle* h, int32_t scene, int32_t field, int32_t order
 sf_status sf_get_fields(sf_handle* h, int32_t scene, int32_t n_fields, const int32_t* fields, int32_t order,
                         void* const* dsts, int64_t count, int32_t dst_on_device) {
     if (!h || n_fields < 0 || (n_fields > 0 && (!fields || !dsts))) return SF_ERR_INVALID;
+    // device buffers: one launch for (up to kFieldsPerLaunch) fields
+    if (dst_on_device) {
+        FieldList list;
+        list.n = 0;
+        for (int32_t k = 0; k < n_fields; ++k) {
+            size_t bytes = 0;
+            sf_status st = checkField(h, scene, fields[k], order, dsts[k], count, false, &bytes);
+            const bool own = st == SF_OK && fields[k] >= SF_BFIELD_POS;  // boundary fields
+            if (!own && st == SF_OK) {
+                list.field[list.n] = fields[k];
+                list.buf[list.n++] = dsts[k];
+            }
+            // the fields before an invalid one are copied, as by calls of their own
+            if (list.n > 0 && (st || own || list.n == kFieldsPerLaunch || k == n_fields - 1)) {
+                const sf_status ls = count > 0 ? launchGetFields(h, scene, list, order, count) : SF_OK;
+                list.n = 0;
+                if (ls) return ls;
+            }
+            if (st) return st;
+            if (own && (st = getFieldQueued(h, scene, fields[k], order, dsts[k], count, 1))) return st;
+        }
+        return SF_OK;
+    }
     for (int32_t k = 0; k < n_fields; ++k)
         if (sf_status st = getFieldQueued(h, scene, fields[k], order, dsts[k], count, dst_on_device)) return st;
-    if (dst_on_device || n_fields == 0) return SF_OK;
+    if (n_fields == 0) return SF_OK;
     return h->cuda(cudaStreamSynchronize(h->stream), "get_fields sync");
 }
 
 namespace {
 
+sf_status launchSetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
+    for (int k = 0; k < list.n; ++k)
+        if (list.field[k] == SF_FIELD_POS) h->pairsFresh = false;
+    kSetFields<<<int((n + 255) / 256), 256, 0, h->stream>>>(list, int(n), h->hScenes[scene].slot_off, order,
+                                                           fieldArrays(h), h->dScenes + scene);
+    return h->cuda(cudaGetLastError(), "set_field launch");
+}
+
 // sf_set_field without its final host synchronisation.
-sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t order, const void* src, int64_t count,
+sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t order, const void* src, int64_t n,
                          int32_t src_on_device) {
-    if (!h || !src || scene < 0 || scene >= h->nScenes) return SF_ERR_INVALID;
-    const int w = fieldWidth(field);
-    if (w == 0 || field >= SF_BFIELD_POS || field == SF_FIELD_ID || field == SF_FIELD_KEY ||
-        field == SF_FIELD_NEIGHBORS)
-        return h->fail(SF_ERR_INVALID, "field cannot be set");
-    if (order != SF_ORDER_SORTED && order != SF_ORDER_ID) return h->fail(SF_ERR_INVALID, "unknown order");
-    const SceneDev& S = h->hScenes[scene];
-    const int64_t n = h->n[scene];
-    if (count != n) return h->fail(SF_ERR_INVALID, "count must equal the scene's particle count");
+    size_t bytes = 0;
+    if (sf_status st = checkField(h, scene, field, order, src, n, true, &bytes)) return st;
     if (n == 0) return SF_OK;
-    const size_t bytes = size_t(n) * size_t(w) * 4;
     const void* from = src;
     // pinned host memory in sorted order is read by the scatter kernel directly
     void* mapped = (!src_on_device && order == SF_ORDER_SORTED) ? mappedHostPointer(src) : nullptr;
@@ -1458,17 +1537,13 @@ sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
             from = h->stage;
         }
     }
-    const int c = h->cur;
-    if (field == SF_FIELD_POS) h->pairsFresh = false;
     float4* vec = order == SF_ORDER_SORTED ? vec3Array(h, field) : nullptr;
-    if (vec && (reinterpret_cast<uintptr_t>(from) & 15u) == 0)
-        kSetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
-            int(n), S.slot_off, vec, static_cast<const float4*>(from), field == SF_FIELD_VEL ? h->grec4 : nullptr);
-    else
-        kSetField<<<int((n + 255) / 256), 256, 0, h->stream>>>(field, int(n), S.slot_off, order, h->pos[c],
-                                                               h->vel[c], h->col[c], h->mat[c], h->amc[c], h->pid[c],
-                                                               h->aux, h->flow, h->adh, h->avgadh, h->drag, h->acc,
-                                                               h->dp, h->vrec2, h->grec4, from, h->dScenes + scene);
+    if (!vec || (reinterpret_cast<uintptr_t>(from) & 15u) != 0)
+        return launchSetFields(h, scene, oneField(field, from), order, n);
+    if (field == SF_FIELD_POS) h->pairsFresh = false;
+    kSetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
+        int(n), h->hScenes[scene].slot_off, vec, static_cast<const float4*>(from),
+        field == SF_FIELD_VEL ? h->grec4 : nullptr);
     return h->cuda(cudaGetLastError(), "set_field launch");
 }
 
@@ -1484,9 +1559,30 @@ sf_status sf_set_field(sf_handle* h, int32_t scene, int32_t field, int32_t order
 sf_status sf_set_fields(sf_handle* h, int32_t scene, int32_t n_fields, const int32_t* fields, int32_t order,
                         const void* const* srcs, int64_t count, int32_t src_on_device) {
     if (!h || n_fields < 0 || (n_fields > 0 && (!fields || !srcs))) return SF_ERR_INVALID;
+    // device buffers: one launch for (up to kFieldsPerLaunch) fields
+    if (src_on_device) {
+        FieldList list;
+        list.n = 0;
+        for (int32_t k = 0; k < n_fields; ++k) {
+            size_t bytes = 0;
+            const sf_status st = checkField(h, scene, fields[k], order, srcs[k], count, true, &bytes);
+            if (st == SF_OK) {
+                list.field[list.n] = fields[k];
+                list.buf[list.n++] = const_cast<void*>(srcs[k]);
+            }
+            // the fields before an invalid one are set, as by calls of their own
+            if (list.n > 0 && (st || list.n == kFieldsPerLaunch || k == n_fields - 1)) {
+                const sf_status ls = count > 0 ? launchSetFields(h, scene, list, order, count) : SF_OK;
+                list.n = 0;
+                if (ls) return ls;
+            }
+            if (st) return st;
+        }
+        return SF_OK;
+    }
     for (int32_t k = 0; k < n_fields; ++k)
         if (sf_status st = setFieldQueued(h, scene, fields[k], order, srcs[k], count, src_on_device)) return st;
-    if (src_on_device || n_fields == 0) return SF_OK;
+    if (n_fields == 0) return SF_OK;
     return h->cuda(cudaStreamSynchronize(h->stream), "set_fields sync");
 }
 
@@ -1592,23 +1688,22 @@ sf_status sf_add_sph_particles(sf_handle* h, int32_t scene, const float* pos3, i
 
 namespace {
 
-// Scatters one scene's persistent arrays from buffer set o to t by particle
-// id: live slot s goes to slotOff + pid[s]; parked slots keep their place.
-__global__ void kResetOrder(int slots, int n, int slotOff, const float4* __restrict__ pos, const float4* __restrict__ vel,
-                            const float4* __restrict__ col, const float4* __restrict__ mat,
-                            const float2* __restrict__ amc, const int* __restrict__ pid, float4* __restrict__ pos2,
-                            float4* __restrict__ vel2, float4* __restrict__ col2, float4* __restrict__ mat2,
-                            float2* __restrict__ amc2, int* __restrict__ pid2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= slots) return;
-    const int s = slotOff + i;
-    const int id = pid[s];
-    const int d = (i < n && id >= 0 && id < n) ? slotOff + id : s;
-    pos2[d] = pos[s];
-    vel2[d] = vel[s];
-    col2[d] = col[s];
-    mat2[d] = mat[s];
-    amc2[d] = amc[s];
+// Scatters the persistent arrays of every scene from one buffer set to the
+// other by particle id: live slot s goes to slot_off + pid[s]; parked slots
+// (pid -1) keep their place.
+__global__ void __launch_bounds__(kSlotAlign) kResetOrder(const SceneDev* __restrict__ scenes,
+                                                          const int* __restrict__ blockScene, FieldArrays from,
+                                                          float4* __restrict__ pos2, float4* __restrict__ vel2,
+                                                          float4* __restrict__ col2, float4* __restrict__ mat2,
+                                                          float2* __restrict__ amc2, int* __restrict__ pid2) {
+    const int s = blockIdx.x * kSlotAlign + threadIdx.x;
+    const int id = from.pid[s];
+    const int d = id >= 0 ? scenes[blockScene[blockIdx.x]].slot_off + id : s;
+    pos2[d] = from.pos[s];
+    vel2[d] = from.vel[s];
+    col2[d] = from.col[s];
+    mat2[d] = from.mat[s];
+    amc2[d] = from.amc[s];
     pid2[d] = id;
 }
 
@@ -1616,16 +1711,10 @@ __global__ void kResetOrder(int slots, int n, int slotOff, const float4* __restr
 
 sf_status sf_reset_order(sf_handle* h) {
     if (!h) return SF_ERR_INVALID;
-    const int o = h->cur, t = 1 - h->cur;
-    for (int sc = 0; sc < h->nScenes; ++sc) {
-        const SceneDev& S = h->hScenes[sc];
-        const int slots = S.slot_cap;
-        if (slots <= 0) continue;
-        kResetOrder<<<(slots + 255) / 256, 256, 0, h->stream>>>(
-            slots, int(h->n[sc]), S.slot_off, h->pos[o], h->vel[o], h->col[o], h->mat[o], h->amc[o], h->pid[o],
-            h->pos[t], h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t]);
-        h->launches += 1;
-    }
+    const int t = 1 - h->cur;
+    kResetOrder<<<h->slotBlocks, kSlotAlign, 0, h->stream>>>(h->dScenes, h->dBlockScene, fieldArrays(h), h->pos[t],
+                                                             h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t]);
+    h->launches += 1;
     h->cur = t;
     h->sorted = false;
     h->pairsFresh = false;
