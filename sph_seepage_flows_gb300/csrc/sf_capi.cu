@@ -234,6 +234,7 @@ struct sf_handle {
     // the render interval from dTimeArg, written before each replay
     GraphCache graphStep[2];
     float* dTimeArg = nullptr;
+    float timeArg = 0.f;  // what dTimeArg holds (a NaN or zero is written again)
     bool captureStep = false;  // runStage passes dTimeArg to the integrator while capturing graphStep
     int nbrCap = kMinNbr;                 // particle neighbour list capacity (per slot)
     // list growth: copies of the scene states queued behind the substeps and
@@ -982,12 +983,16 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
         cudaEventCreate(&e1);
         cudaEventRecord(e0, h->stream);
     }
-    // the substep is replayed from a captured graph; its render interval goes
-    // to the device first (a pageable source: the copy is staged before the
-    // call returns)
+    // the substep is replayed from a captured graph; a render interval other
+    // than the last call's goes to the device first (a pageable source: the
+    // copy is staged before the call returns)
     const float t = render_interval;
-    if (h->cuda(cudaMemcpyAsync(h->dTimeArg, &t, sizeof(float), cudaMemcpyHostToDevice, h->stream), "step time"))
-        return SF_ERR_CUDA;
+    if (t != h->timeArg || t == 0.f) {
+        h->timeArg = 0.f;
+        if (h->cuda(cudaMemcpyAsync(h->dTimeArg, &t, sizeof(float), cudaMemcpyHostToDevice, h->stream), "step time"))
+            return SF_ERR_CUDA;
+        h->timeArg = t;
+    }
     GraphCache& g = h->graphStep[h->cur];
     sf_status st = ensureStepGraph(h, g);
     if (st != SF_OK) return st;
@@ -996,7 +1001,7 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
     h->cur = 1 - h->cur;
     h->sorted = true;
     h->pairsFresh = false;
-    queueStateCopy(h);
+    const int copy = queueStateCopy(h);
     if (ms_out) {
         cudaEventRecord(e1, h->stream);
         cudaEventSynchronize(e1);
@@ -1004,7 +1009,11 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
         cudaEventDestroy(e0);
         cudaEventDestroy(e1);
     }
-    if (n_substeps_out) {
+    if (n_substeps_out && copy >= 0) {
+        // the count is in the state copy queued for the list check
+        if (h->cuda(cudaEventSynchronize(h->stateEvent[copy]), "state copy")) return SF_ERR_CUDA;
+        *n_substeps_out = h->stateHost[copy][0].n_sub;
+    } else if (n_substeps_out) {
         SceneState s0;
         st = h->cuda(cudaMemcpyAsync(&s0, h->dState, sizeof(SceneState), cudaMemcpyDeviceToHost, h->stream),
                      "read n_sub");
