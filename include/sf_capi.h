@@ -424,11 +424,12 @@ sf_status sf_set_adjoint_seed_scale(sf_handle* h, int32_t scene, float scale);
  *   cell_start_out_dev  out: G + 1 ints, device, G = grid cells:
  *                            first sorted index with cell >= c; entry G = n
  *   stream              the CUDA stream to use (NULL = the legacy default stream)
- * Every call copies a flag word to host memory and waits for its stream
- * before returning, and returns SF_ERR_DEVICE when a position is not finite;
- * the output buffers then hold unspecified values. The first call on a
- * device looks up the scratch address (cudaGetSymbolAddress), which may load
- * the module: make the first call before any stream capture. The lookup is
+ * Every call waits for its stream before returning, and returns
+ * SF_ERR_DEVICE when a position is not finite (its kernels report that
+ * through pinned host memory); the output buffers then hold unspecified
+ * values. The first call on a device looks up the scratch address
+ * (cudaGetSymbolAddress), which may load the module, and takes the pinned
+ * words: make the first call before any stream capture. The lookup is
  * repeated when the cached address no longer belongs to the device (after
  * cudaDeviceReset). Calls that overlap on the GPU (two streams or host
  * threads) share the scratch and race: serialise them. Errors are reported

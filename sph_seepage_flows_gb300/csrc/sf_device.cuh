@@ -35,6 +35,7 @@
 namespace sfg {
 
 constexpr int kSlotAlign = 256;
+constexpr int kSortThreads = 256;  // threads per block of the sort kernels
 constexpr float kEps = 1e-6f;  // KIRI_EPSILON (kiri_pbs_pch.cuh:52)
 
 struct BezierDev {  // QuadraticBezierCoeff (cuda_sf_utils.cuh:36-83)
@@ -199,6 +200,30 @@ __device__ __forceinline__ float3 capillaryForce(const SceneDev& S, float3 dij, 
         f = -N * (ncp + stf);
     }
     return f;
+}
+
+// Exclusive scan of one value per thread over a block of kSortThreads; total:
+// the block's sum. Every thread of the block calls it.
+__device__ __forceinline__ unsigned int blockScan(unsigned int v, unsigned int& total) {
+    __shared__ unsigned int warpSum[kSortThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    unsigned int incl = v;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const unsigned int u = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += u;
+    }
+    __syncthreads();  // the sums of the call before have been read
+    if (lane == 31) warpSum[warp] = incl;
+    __syncthreads();
+    unsigned int before = 0u;
+    total = 0u;
+#pragma unroll
+    for (int w = 0; w < kSortThreads / 32; ++w) {
+        if (w < warp) before += warpSum[w];
+        total += warpSum[w];
+    }
+    return before + incl - v;
 }
 
 }  // namespace sfg

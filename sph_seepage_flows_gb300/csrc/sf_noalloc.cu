@@ -1,18 +1,24 @@
-// Allocation-free cell sort (sf_cell_sort_noalloc): the key computation,
-// stable radix sort and cell-start table of the sort stage, with every
-// scratch word in one static device array instead of handle memory.
+// Allocation-free cell sort (sf_cell_sort_noalloc): the sort stage of a
+// single-scene handle on caller buffers, with every scratch word in one static
+// device array instead of handle memory.
 //
-// The scratch (g_noallocScratch) holds the keys, the ping-pong key and
-// permutation buffers, the digit histograms and totals of the radix sort and
-// a non-finite-position flag. Its device address is looked up once per
-// device with cudaGetSymbolAddress (the first call on a device does it, and
-// the first call after that device's context was reset, which is detected
-// by asking the runtime whether the cached address is still a device
-// address), so the call itself issues only kernels, one memset,
-// device-to-device copies and one small device-to-host read. Every
-// histogram and total is written before it is read; the flag is the only
-// word that must start at zero and is cleared by every call. Calls that
-// overlap on the GPU share the scratch and race.
+// Two forms, as in the handle's sort stage. The counting sort counts in the
+// caller's cell table: clear, keys and counts, scan of each table tile, tiles
+// added up (the table is then final), slots of each cell in arrival order,
+// stable order. The radix sort (keys, digit passes, table by binary search)
+// is for grids with many more cells than particles, and for input with a cell
+// of more than kCrowded particles: finding their order slot by slot would cost
+// the square of their number, so the last kernel reports such a cell instead.
+// The call is a chain of short launches and a wait: 200k particles 84 -> 33 us.
+//
+// The scratch (g_noallocScratch) holds the keys and the arrays of either form.
+// Its device address is looked up once per device with cudaGetSymbolAddress
+// (the first call on a device does it, and the first call after that device's
+// context was reset, which is detected by asking the runtime whether the
+// cached address is still a device address); the same lookup takes one page
+// of pinned host memory for the words that a call reports through, which its
+// kernels write directly. Every scratch word is written before it is read.
+// Calls that overlap on the GPU share the scratch and race.
 #include "../../include/sf_capi.h"
 #include "sf_device.cuh"
 #include "sf_kernels.h"
@@ -29,22 +35,115 @@ namespace {
 using namespace sfg;
 
 constexpr int kMaxN = SF_NOALLOC_MAX_PARTICLES;
-constexpr size_t kFlagWords = 64;               // keeps the arrays behind it 256-byte aligned
 constexpr size_t kHistWords = 256 * size_t(kMaxN / 1024);  // >= 256 digit counts per sort tile
-constexpr size_t kWords = kFlagWords + 4 * size_t(kMaxN) + 256 + kHistWords;
+constexpr size_t kWords = 4 * size_t(kMaxN) + 256 + kHistWords;
+constexpr unsigned int kCrowded = 256;          // most particles of a cell that the counting sort orders
 constexpr int kMaxDevices = 64;
 
 __device__ __align__(256) unsigned int g_noallocScratch[kWords];
 
-// Pos2GridHash of every position (the key of the sort stage for a
-// single-scene handle); non-finite positions set the flag.
-__global__ void kNoAllocKeys(SceneDev S, const float* __restrict__ pos, int n, unsigned int* __restrict__ keys,
-                             unsigned int* flag) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
+// What a call's kernels report, in pinned host memory: cleared by the host
+// before the launches, set to 1 by any thread that finds the condition.
+struct Report {
+    unsigned int nonFinite, crowded;
+};
+
+// Pos2GridHash of a position (the key of the sort stage for a single-scene
+// handle); a non-finite one is reported.
+__device__ __forceinline__ unsigned int keyOf(const SceneDev& S, const float* __restrict__ pos, int i,
+                                              Report* report) {
     const float3 q = mk3(pos[3 * i], pos[3 * i + 1], pos[3 * i + 2]);
-    if (!(isfinite(q.x) && isfinite(q.y) && isfinite(q.z))) atomicOr(flag, 1u);
-    keys[i] = unsigned(localHash(S, cellOf(S, q)));
+    if (!(isfinite(q.x) && isfinite(q.y) && isfinite(q.z))) report->nonFinite = 1u;
+    return unsigned(localHash(S, cellOf(S, q)));
+}
+
+__global__ void kNoAllocKeys(SceneDev S, const float* __restrict__ pos, int n, unsigned int* __restrict__ keys,
+                             Report* report) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) keys[i] = keyOf(S, pos, i, report);
+}
+
+constexpr int kThreads = kSortThreads, kItems = 4;  // 1024 cells per turn of a scan block
+
+// (key, place among the particles counted into its cell), counting in the
+// table; runs of equal keys in a warp take one atomic.
+__global__ void __launch_bounds__(kThreads) kNoAllocCount(SceneDev S, const float* __restrict__ pos, int n,
+                                                          unsigned int* table, uint2* __restrict__ keyRank,
+                                                          Report* report) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    const unsigned int lane = threadIdx.x & 31u;
+    const unsigned int key = i < n ? keyOf(S, pos, i, report) : 0xffffffffu;
+    const unsigned int prev = __shfl_up_sync(0xffffffffu, key, 1);
+    const unsigned int heads = __ballot_sync(0xffffffffu, lane == 0u || prev != key);
+    unsigned int at = 0u;
+    if (i < n && ((heads >> lane) & 1u)) {
+        const unsigned int behind = lane == 31u ? 0u : heads >> (lane + 1u);
+        at = atomicAdd(&table[key], behind ? unsigned(__ffs(behind)) : 32u - lane);
+    }
+    const int leader = 31 - __clz(heads & (0xffffffffu >> (31u - lane)));
+    at = __shfl_sync(0xffffffffu, at, leader) + (lane - unsigned(leader));
+    if (i < n) keyRank[i] = make_uint2(key, at);
+}
+
+// Block b: exclusive scan of table tile b (2^shift cells) in place, and its sum.
+__global__ void __launch_bounds__(kThreads) kNoAllocScan(unsigned int* table, int nCells, int shift,
+                                                         unsigned int* __restrict__ tileSum) {
+    const int beg = int(blockIdx.x) << shift, end = min(beg + (1 << shift), nCells);
+    unsigned int carry = 0u, total;
+    for (int base = beg; base < end; base += kThreads * kItems) {
+        const int c = base + int(threadIdx.x) * kItems;
+        unsigned int v[kItems], sum = 0u;
+#pragma unroll
+        for (int u = 0; u < kItems; ++u) sum += v[u] = c + u < end ? table[c + u] : 0u;
+        unsigned int a = carry + blockScan(sum, total);
+#pragma unroll
+        for (int u = 0; u < kItems; ++u) {
+            if (c + u < end) table[c + u] = a;
+            a += v[u];
+        }
+        carry += total;
+    }
+    if (threadIdx.x == 0) tileSum[blockIdx.x] = carry;
+}
+
+// Adds the sums of the tiles before to every tile but the first (one block per
+// tile); the table is then final.
+__global__ void __launch_bounds__(kThreads) kNoAllocAddTiles(unsigned int* table, int nCells, int n, int shift,
+                                                             const unsigned int* __restrict__ tileSum) {
+    unsigned int before = 0u, total;
+    for (int t = threadIdx.x; t < int(blockIdx.x); t += kThreads) before += tileSum[t];
+    blockScan(before, total);
+    const int beg = int(blockIdx.x) << shift, end = min(beg + (1 << shift), nCells);
+    if (total)
+        for (int c = beg + int(threadIdx.x); c < end; c += kThreads) table[c] += total;
+    if (end == nCells && threadIdx.x == 0) table[nCells] = unsigned(n);
+}
+
+__global__ void __launch_bounds__(kThreads) kNoAllocScatter(int n, const unsigned int* __restrict__ table,
+                                                            const uint2* __restrict__ keyRank,
+                                                            unsigned int* __restrict__ arrived) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= n) return;
+    const uint2 kr = keyRank[i];
+    arrived[table[kr.x] + kr.y] = unsigned(i);
+}
+
+// The stable order: a particle's place in its cell is the number of the cell's
+// particles with a smaller index.
+__global__ void __launch_bounds__(kThreads) kNoAllocOrder(int n, const unsigned int* __restrict__ table,
+                                                          const uint2* __restrict__ keyRank,
+                                                          const unsigned int* __restrict__ arrived,
+                                                          int* __restrict__ perm, Report* report) {
+    const int i = blockIdx.x * kThreads + threadIdx.x;
+    if (i >= n) return;
+    const unsigned int o = arrived[i], key = keyRank[o].x, beg = table[key], end = table[key + 1];
+    if (end - beg > kCrowded) {
+        report->crowded = 1u;
+        return;
+    }
+    unsigned int d = beg;
+    for (unsigned int q = beg; q < end; ++q) d += arrived[q] < o ? 1u : 0u;
+    perm[d] = int(o);
 }
 
 sf_status failWith(sf_status st, const std::string& msg) {
@@ -65,11 +164,13 @@ bool stillDeviceAddress(const void* p, int device) {
     return a.type == cudaMemoryTypeDevice && a.device == device;
 }
 
-// Device address of the scratch on the current device: looked up on the first
-// call on a device and again whenever the cached address went stale.
-unsigned int* scratchAddress(int device, std::string& why) {
+// Device address of the scratch on the current device, and the device's report
+// words: looked up on the first call on a device and again whenever the cached
+// address went stale (a reset of the context frees the pinned memory as well).
+unsigned int* scratchAddress(int device, Report*& report, std::string& why) {
     static std::mutex mu;
     static unsigned int* addr[kMaxDevices] = {};
+    static Report* reports[kMaxDevices] = {};
     std::lock_guard<std::mutex> lock(mu);
     if (device < 0 || device >= kMaxDevices) {
         why = "device index out of range";
@@ -83,8 +184,16 @@ unsigned int* scratchAddress(int device, std::string& why) {
             why = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e);
             return nullptr;
         }
+        void* r = nullptr;
+        const cudaError_t he = cudaHostAlloc(&r, sizeof(Report), cudaHostAllocPortable | cudaHostAllocMapped);
+        if (he != cudaSuccess) {
+            why = std::string("cudaHostAlloc: ") + cudaGetErrorString(he);
+            return nullptr;
+        }
+        reports[device] = static_cast<Report*>(r);
         addr[device] = static_cast<unsigned int*>(p);
     }
+    report = reports[device];
     return addr[device];
 }
 
@@ -108,7 +217,8 @@ extern "C" sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const 
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return failWith(SF_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     std::string why;
-    unsigned int* base = scratchAddress(device, why);
+    Report* report = nullptr;
+    unsigned int* base = scratchAddress(device, report, why);
     if (!base) return failWith(SF_ERR_CUDA, "sf_cell_sort_noalloc: " + why);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int ncell = int(cells);
@@ -116,15 +226,6 @@ extern "C" sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const 
         e = cudaMemsetAsync(cell_start_out_dev, 0, sizeof(int32_t) * (size_t(ncell) + 1), s);
         return e == cudaSuccess ? SF_OK : failWith(SF_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
     }
-    unsigned int* flag = base;
-    unsigned int* keys = base + kFlagWords;
-    SortScratch sc{};
-    sc.keysAlt = keys + kMaxN;
-    sc.vals = keys + 2 * size_t(kMaxN);
-    sc.valsAlt = keys + 3 * size_t(kMaxN);
-    sc.digitTotal = keys + 4 * size_t(kMaxN);
-    sc.hist = sc.digitTotal + 256;
-    sc.tiles = sortTiles(int(n));
     // grid of the sort stage (the cell fields of the scene description)
     SceneDev S{};
     S.lpx = grid->lowest_point[0];
@@ -135,23 +236,50 @@ extern "C" sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const 
     S.gy = grid->grid_size[1];
     S.gz = grid->grid_size[2];
     S.ncell = ncell;
-    int bits = 1;
-    while ((int64_t(1) << bits) <= int64_t(ncell)) ++bits;
-    if ((e = cudaMemsetAsync(flag, 0, sizeof(unsigned int), s)) != cudaSuccess)
-        return failWith(SF_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-    kNoAllocKeys<<<int((n + 255) / 256), 256, 0, s>>>(S, pos_dev, int(n), keys, flag);
-    unsigned int *sortedKeys = nullptr, *perm = nullptr;
-    radixSort(s, int(n), bits, keys, sc, &sortedKeys, &perm);
-    launchCellStart(s, int(n), ncell, sortedKeys, reinterpret_cast<unsigned int*>(cell_start_out_dev));
-    if ((e = cudaGetLastError()) != cudaSuccess)
-        return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc launch: ") + cudaGetErrorString(e));
-    if ((e = cudaMemcpyAsync(perm_out_dev, perm, sizeof(int32_t) * size_t(n), cudaMemcpyDeviceToDevice, s)) !=
-        cudaSuccess)
-        return failWith(SF_ERR_CUDA, std::string("permutation copy: ") + cudaGetErrorString(e));
-    unsigned int flagHost = 0;
-    if ((e = cudaMemcpyAsync(&flagHost, flag, sizeof(unsigned int), cudaMemcpyDeviceToHost, s)) != cudaSuccess ||
-        (e = cudaStreamSynchronize(s)) != cudaSuccess)
-        return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc sync: ") + cudaGetErrorString(e));
-    if (flagHost) return failWith(SF_ERR_DEVICE, "sf_cell_sort_noalloc: non-finite particle position");
+    unsigned int* table = reinterpret_cast<unsigned int*>(cell_start_out_dev);
+    const int blocks = int((n + kThreads - 1) / kThreads);
+    report->nonFinite = report->crowded = 0u;
+    bool done = false;
+    if (useCountingSort(int(n), ncell)) {
+        uint2* keyRank = reinterpret_cast<uint2*>(base);
+        unsigned int *arrived = base + 2 * size_t(kMaxN), *tileSum = base + 3 * size_t(kMaxN);
+        const int shift = countTileShift(ncell), tiles = ((ncell - 1) >> shift) + 1;
+        if ((e = cudaMemsetAsync(table, 0, sizeof(int32_t) * size_t(ncell), s)) != cudaSuccess)
+            return failWith(SF_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
+        kNoAllocCount<<<blocks, kThreads, 0, s>>>(S, pos_dev, int(n), table, keyRank, report);
+        kNoAllocScan<<<tiles, kThreads, 0, s>>>(table, ncell, shift, tileSum);
+        kNoAllocAddTiles<<<tiles, kThreads, 0, s>>>(table, ncell, int(n), shift, tileSum);
+        kNoAllocScatter<<<blocks, kThreads, 0, s>>>(int(n), table, keyRank, arrived);
+        kNoAllocOrder<<<blocks, kThreads, 0, s>>>(int(n), table, keyRank, arrived, perm_out_dev, report);
+        if ((e = cudaGetLastError()) != cudaSuccess)
+            return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc launch: ") + cudaGetErrorString(e));
+        if ((e = cudaStreamSynchronize(s)) != cudaSuccess)
+            return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc sync: ") + cudaGetErrorString(e));
+        done = report->crowded == 0u || report->nonFinite != 0u;
+    }
+    if (!done) {
+        unsigned int* keys = base;
+        SortScratch sc{};
+        sc.keysAlt = keys + kMaxN;
+        sc.vals = keys + 2 * size_t(kMaxN);
+        sc.valsAlt = keys + 3 * size_t(kMaxN);
+        sc.digitTotal = keys + 4 * size_t(kMaxN);
+        sc.hist = sc.digitTotal + 256;
+        sc.tiles = sortTiles(int(n));
+        int bits = 1;
+        while ((int64_t(1) << bits) <= int64_t(ncell)) ++bits;
+        kNoAllocKeys<<<blocks, kThreads, 0, s>>>(S, pos_dev, int(n), keys, report);
+        unsigned int *sortedKeys = nullptr, *perm = nullptr;
+        radixSort(s, int(n), bits, keys, sc, &sortedKeys, &perm);
+        launchCellStart(s, int(n), ncell, sortedKeys, table);
+        if ((e = cudaGetLastError()) != cudaSuccess)
+            return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc launch: ") + cudaGetErrorString(e));
+        if ((e = cudaMemcpyAsync(perm_out_dev, perm, sizeof(int32_t) * size_t(n), cudaMemcpyDeviceToDevice, s)) !=
+            cudaSuccess)
+            return failWith(SF_ERR_CUDA, std::string("permutation copy: ") + cudaGetErrorString(e));
+        if ((e = cudaStreamSynchronize(s)) != cudaSuccess)
+            return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc sync: ") + cudaGetErrorString(e));
+    }
+    if (report->nonFinite) return failWith(SF_ERR_DEVICE, "sf_cell_sort_noalloc: non-finite particle position");
     return SF_OK;
 }

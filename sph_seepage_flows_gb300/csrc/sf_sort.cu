@@ -25,8 +25,6 @@
 
 namespace sfg {
 
-constexpr int kSortThreads = 256;
-
 int sortTiles(int n, int items) { return (n + kSortThreads * items - 1) / (kSortThreads * items); }
 
 int sortItemsFor(int n, int smCount) {
@@ -467,29 +465,6 @@ __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restr
     const int leader = 31 - __clz(heads & (0xffffffffu >> (31u - lane)));
     at = __shfl_sync(0xffffffffu, at, leader) + (lane - unsigned(leader));
     cc.keyRank[slot] = make_uint2(key, live ? at : parkedBase + at);
-}
-
-// Exclusive scan of one value per thread over the block; total: the block's sum.
-__device__ __forceinline__ unsigned int blockScan(unsigned int v, unsigned int& total) {
-    __shared__ unsigned int warpSum[kSortThreads / 32];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    unsigned int incl = v;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const unsigned int u = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += u;
-    }
-    __syncthreads();  // the sums of the call before have been read
-    if (lane == 31) warpSum[warp] = incl;
-    __syncthreads();
-    unsigned int before = 0u;
-    total = 0u;
-#pragma unroll
-    for (int w = 0; w < kSortThreads / 32; ++w) {
-        if (w < warp) before += warpSum[w];
-        total += warpSum[w];
-    }
-    return before + incl - v;
 }
 
 // Block b scans table tile b (2^tileShift cells, a multiple of kScanChunk) in

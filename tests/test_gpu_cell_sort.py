@@ -60,3 +60,37 @@ def test_sort_is_the_stable_key_order(cuda_lib, sizes, side, spare, crowd):
             pos[s][move] = rng.uniform(-0.05, side + 0.05, (int(move.sum()), 3)).astype(np.float32)
             sim.set_field("pos", pos[s], order="id", scene=s)
     assert sim.check_error() == 0
+
+
+@pytest.mark.parametrize("n, grid, crowd", [
+    (1, (3, 3, 3), 0), (31, (1, 1, 1), 0), (33, (20, 10, 30), 33), (1025, (16, 8, 8), 256), (1025, (16, 8, 8), 257),
+    (5000, (1, 1, 1), 0), (262144, (64, 50, 61), 0), (4099, (150, 100, 90), 0)])
+def test_noalloc_sort_is_the_stable_key_order(cuda_lib, n, grid, crowd):
+    """Both forms of the allocation-free sort: cells up to and above the size that the counting form orders, one cell for
+    everything, tables of one tile, of many and with more cells than the counting form takes."""
+    torch = pytest.importorskip("torch")
+    import ctypes
+    from sph_seepage_flows_gb300.params import boundary_params
+    h = 0.04
+    b = boundary_params((0.1, -0.2, 0.0), [0.1 + grid[0] * h + 0.01, -0.2 + grid[1] * h + 0.01, grid[2] * h + 0.01], h)
+    assert list(b.grid_size[:]) == list(grid)
+    rng = np.random.default_rng(n)
+    lo = np.float32([0.1, -0.2, 0.0])
+    pos = (lo + rng.uniform(-0.05, 1.05, (n, 3)) * np.float32(grid) * h).astype(np.float32)
+    pos[rng.permutation(n)[:crowd]] = lo + np.float32(0.5 * h)
+    q = ((pos - lo) / np.float32(h)).astype(np.int64)
+    c = np.minimum(np.maximum(q, 0), np.array(grid) - 1)
+    keys = (c[:, 0] * grid[1] + c[:, 1]) * grid[2] + c[:, 2]
+    cells = int(np.prod(grid))
+    want = np.argsort(keys, kind="stable")
+    dpos = torch.from_numpy(pos).cuda()
+    # the table at an odd word: it has no alignment beyond its elements'
+    room = torch.full((cells + 3,), -7, dtype=torch.int32, device="cuda")
+    table, perm = room[1:-1], torch.full((n,), -1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):
+        assert cuda_lib.sf_cell_sort_noalloc(ctypes.byref(b), dpos.data_ptr(), n, perm.data_ptr(), table.data_ptr(),
+                                             None) == 0
+        assert np.array_equal(perm.cpu().numpy(), want)
+        assert np.array_equal(table.cpu().numpy(), np.searchsorted(keys[want], np.arange(cells + 1)))
+        assert int(room[0]) == int(room[-1]) == -7
