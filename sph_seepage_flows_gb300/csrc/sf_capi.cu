@@ -243,10 +243,10 @@ struct sf_handle {
     cudaEvent_t stateEvent[2] = {nullptr, nullptr};
     bool statePending[2] = {false, false};
     int64_t listGrowths = 0;
-    // the density pass runs fastest with 64-128 threads per block (256 / 275 us
-    // with 128 / 256 on the 1M embankment: smaller blocks even out the lengths
-    // of its walks)
-    int block[kTunedPasses] = {128, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign, kSlotAlign};
+    // the neighbour passes run fastest with 64-128 threads per block: smaller
+    // blocks even out the lengths of their walks (1M embankment with 128 / 256:
+    // density 256 / 275 us, average flow 82 / 94, water momentum 115 / 119)
+    int block[kTunedPasses] = {128, 128, 128, 128, 128, kSlotAlign};
     int lanes = 1;  // threads per slot of the momentum passes and the adjoint pair kernels
     // threads per slot of the passes before them, whose results do not depend on it
     int listLanes[3] = {1, 1, 1};  // density, average flow, voidage / adhesion

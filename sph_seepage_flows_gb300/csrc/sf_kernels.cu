@@ -931,7 +931,7 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
 // finds). That was most of this pass's work: 93 -> 30 us on
 // the 1M embankment, for 26 us more in the density pass.
 template <int G, bool kSummed>
-__global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kSlotAlign, 4) kAvgFlow(const SceneDev* __restrict__ scenes,
                                                        const int* __restrict__ blockScene, NbrLists L,
                                                        const float4* __restrict__ pos4,
                                                        const float4* __restrict__ vel4, float4* __restrict__ aux4,
@@ -944,13 +944,16 @@ __global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restric
     const bool sandI = pi4.w < 0.f;
     float v_s = 0.f, v_w = 0.f, sand_volume = 0.f;
     float3 avg_s = mk3(0.f, 0.f, 0.f), avg_w = avg_s;
+    struct Record {
+        float4 p, v;
+    };
+    auto record = [&](int j) { return Record{pos4[j], vel4[j]}; };
     // sand neighbours: sand volume (every i) and, for water i, the sand average flow
     if (!kSummed || !sandI) {
         forLabelNeighborsOrdered<true, G, 6>(
-            S, L, slot, pi, pos4, part,
-            [&](int j) {
-                const float4 pj = pos4[j];
-                const float4 vj4 = vel4[j];
+            S, L, slot, pi, pos4, part, record,
+            [&](const Record& d) {
+                const float4 pj = d.p, vj4 = d.v;
                 const float mj = -pj.w;
                 const float wij = poly6(S, len3(pi - xyz(pj)));
                 Terms<6> t;
@@ -978,10 +981,9 @@ __global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restric
     // water neighbours of sand i: the water average flow and the saturation
     if (sandI) {
         forLabelNeighborsOrdered<false, G, 4>(
-            S, L, slot, pi, pos4, part,
-            [&](int j) {
-                const float4 pj = pos4[j];
-                const float4 vj4 = vel4[j];
+            S, L, slot, pi, pos4, part, record,
+            [&](const Record& d) {
+                const float4 pj = d.p, vj4 = d.v;
                 const float vj = pj.w / vj4.w;
                 const float wij = poly6(S, len3(pi - xyz(pj)));
                 const float3 a = xyz(vj4) * vj * wij;
@@ -1032,7 +1034,7 @@ __global__ void __launch_bounds__(kSlotAlign) kAvgFlow(const SceneDev* __restric
 // of water neighbours and writes the final voidage (aux.w) of sand slots.
 // Lane-split like kAvgFlow (order-preserving sums).
 template <int G>
-__global__ void __launch_bounds__(kSlotAlign) kVoidageAdhesion(
+__global__ void __launch_bounds__(kSlotAlign, 4) kVoidageAdhesion(
     const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, NbrLists L,
     const float4* __restrict__ pos4, const float4* __restrict__ vel4, float4* __restrict__ aux4,
     const float4* __restrict__ flow4, float4* __restrict__ adh4, float4* __restrict__ avgadh4,
@@ -1042,14 +1044,19 @@ __global__ void __launch_bounds__(kSlotAlign) kVoidageAdhesion(
     const float4 pi4 = pos4[slot];
     if (pi4.w == 0.f) return;
     const float3 pi = xyz(pi4);
+    struct Record {
+        float4 p;
+        float2 r;
+    };
+    auto record = [&](int j) { return Record{pos4[j], vrec2[j]}; };
     if (pi4.w < 0.f) {
         const float sat = aux4[slot].z;
         float num = 0.f, den = 0.f;
         forLabelNeighborsOrdered<false, G, 2>(
-            S, L, slot, pi, pos4, part,
-            [&](int j) {
-                const float4 pj = pos4[j];
-                const float2 r = vrec2[j];  // (fluid voidage x volume, volume)
+            S, L, slot, pi, pos4, part, record,
+            [&](const Record& d) {
+                const float4 pj = d.p;
+                const float2 r = d.r;  // (fluid voidage x volume, volume)
                 const float3 dij = pi - xyz(pj);
                 const float wij = poly6(S, len3(dij));
                 Terms<2> t;
@@ -1080,10 +1087,10 @@ __global__ void __launch_bounds__(kSlotAlign) kVoidageAdhesion(
         float v_s = 0.f;
         float3 ad = mk3(0.f, 0.f, 0.f);
         forLabelNeighborsOrdered<true, G, 4>(
-            S, L, slot, pi, pos4, part,
-            [&](int j) {
-                const float4 pj = pos4[j];
-                const float2 r = vrec2[j];  // (adhesion Bezier factor of sat_j, volume)
+            S, L, slot, pi, pos4, part, record,
+            [&](const Record& d) {
+                const float4 pj = d.p;
+                const float2 r = d.r;  // (adhesion Bezier factor of sat_j, volume)
                 const float3 dpij = pi - xyz(pj);
                 const float ldp = len3(dpij);
                 const float wij = poly6(S, ldp);

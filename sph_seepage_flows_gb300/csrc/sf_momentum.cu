@@ -11,16 +11,20 @@
 namespace sfg {
 
 // ---------------------------------------------------------- sand momentum
-// Both momentum passes run with a register budget of 48 (5 blocks of
-// kSlotAlign threads per SM): their neighbour gathers are latency bound and
-// gain more from the occupancy than they lose to the values moved to the stack.
+// The neighbour gathers of both momentum passes are bound by latency. With the
+// next neighbour's data loaded ahead (forLabelNeighbors) and a register budget
+// of 64 for it (4 blocks of kSlotAlign threads per SM), sand / water take 57 /
+// 105 us on the 1M embankment, 62 / 83 on the 791k disturbed column; with 48
+// registers the data ahead spills (58 / 123, 75 / 98), with 80 the occupancy
+// is missing (62 / 111, 66 / 90). Four indices ahead without data, at 48
+// registers, took 64 / 118 and 72 / 94.
 // Compute[Multi]SFSandLinearMomentum_CUDA (cuda_sph_sf_solver_gpu.cuh:723-897):
 // DEM and capillary terms of sand neighbours (21-50, 83-109), buoyancy and
 // adhesion terms of water neighbours (240-273, 314-341), DEM against shape
 // boundary particles (52-81) and ComputeDemWorldBoundaryForces
 // (cuda_dem_solver_common_gpu.cuh:132-199). acc = g + 2 (f + df) / m.
 template <int G>
-__global__ void __launch_bounds__(kSlotAlign, 5) kSandMomentum(
+__global__ void __launch_bounds__(kSlotAlign, 4) kSandMomentum(
     const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, NbrLists L,
     const float4* __restrict__ pos4, const float4* __restrict__ vel4, const float4* __restrict__ aux4,
     const float4* __restrict__ flow4, const float4* __restrict__ avgadh4, const float4* __restrict__ mat4,
@@ -43,29 +47,46 @@ __global__ void __launch_bounds__(kSlotAlign, 5) kSandMomentum(
     float3 f = mk3(0.f, 0.f, 0.f), df = f;
     // DEM and capillary terms vanish beyond contact + liquid-bridge reach:
     // iterate the contact list (or the sand list when it overflowed)
-    auto contact = [&](int j) {
-        const float3 dij = xyz(pos4[j]) - pi;
-        const float4 gj = grec4[j];  // (velocity, saturation)
+    struct Contact {
+        float4 p, g;  // g: (velocity, saturation)
+    };
+    auto record = [&](int j) { return Contact{pos4[j], grec4[j]}; };
+    auto contact = [&](const Contact& d) {
+        const float3 dij = xyz(d.p) - pi;
+        const float4 gj = d.g;
         f += demForce(dij, xyz(gj) - vi, S.rij2, S.kn, S.ks, S.tan2);
         f += capillaryForce(S, dij, (ai.z + gj.w) / 2.f);
     };
     const int cc = L.ccnt[slot];
     if (cc <= kMaxContact) {
+        // all indices of a lane's share are loaded ahead of the first contact
         const unsigned* __restrict__ p = L.cnbr + slot;
-#pragma unroll 2
-        for (int k = part; k < cc; k += G) contact(int(p[k * L.M]));
+        if (part < cc) {
+            int jn = part + G < cc ? int(p[(part + G) * L.M]) : slot;
+            Contact d = record(int(p[part * L.M]));
+#pragma unroll 1
+            for (int k = part; k < cc; k += G) {
+                const Contact dn = record(jn);
+                if (k + 2 * G < cc) jn = int(p[(k + 2 * G) * L.M]);
+                contact(d);
+                d = dn;
+            }
+        }
     } else {
-        forSandNeighbors<G>(S, L, slot, pi, pos4, [&](int j) {
+        forLabelNeighbors<true, G, false>(S, L, slot, pi, pos4, part, record, [&](int j, const Contact& d) {
             if (j == slot) return;
-            const float3 dij = xyz(pos4[j]) - pi;
-            if (dot3(dij, dij) < S.dem_reach2) contact(j);
-        }, part);
+            const float3 dij = xyz(d.p) - pi;
+            if (dot3(dij, dij) < S.dem_reach2) contact(d);
+        });
     }
-    forWaterNeighbors<G, true>(S, L, slot, pi, pos4, [&](int j) {
-        const float4 pj = pos4[j];
+    struct Water {
+        float4 p, a, g;  // g: (average adhesion, D)
+    };
+    auto waterRecord = [&](int j) { return Water{pos4[j], aux4[j], avgadh4[j]}; };
+    forLabelNeighbors<false, G, true>(S, L, slot, pi, pos4, part, waterRecord, [&](int, const Water& d) {
+        const float4 pj = d.p;
         const float3 dij = pi - xyz(pj);
-        const float4 aj = aux4[j];
-        const float4 gj = avgadh4[j];  // (average adhesion, D)
+        const float4 aj = d.a, gj = d.g;
         const float wij = poly6(S, len3(dij));
         if (aj.w > 0.f && aj.w <= 1.f) {
             const float dj = gj.w;
@@ -73,7 +94,7 @@ __global__ void __launch_bounds__(kSlotAlign, 5) kSandMomentum(
             f += -mi * pj.w * aj.x / fmaxf(kEps, di * dj) * spikyGrad(S, dij);
         }
         f += wij * vol_i * xyz(gj);
-    }, part);
+    });
     if (S.shape_boundary) {
         forBoundaryNeighbors<G>(S, L, slot, pi, bpos4, [&](int b) {
             const float4 bj = bpos4[b];
@@ -119,7 +140,7 @@ __global__ void __launch_bounds__(kSlotAlign, 5) kSandMomentum(
 // density). acc = g + (a - F_adh / m). Every thread then contributes |acc|
 // of its slot (sand included) to the scene maximum (cuda_wcsph_sf_solver.cu:43-47).
 template <int G>
-__global__ void __launch_bounds__(kSlotAlign, 5) kWaterMomentum(
+__global__ void __launch_bounds__(kSlotAlign, 4) kWaterMomentum(
     const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, SceneState* __restrict__ state,
     NbrLists L, const float4* __restrict__ pos4, const float4* __restrict__ vel4, const float4* __restrict__ aux4,
     const float4* __restrict__ drag4, const float4* __restrict__ adh4, const float4* __restrict__ bpos4,
@@ -137,15 +158,18 @@ __global__ void __launch_bounds__(kSlotAlign, 5) kWaterMomentum(
         const float pri = aux4[slot].x;
         const float pterm_i = dpi.y;
         float3 a = mk3(0.f, 0.f, 0.f);
-        forWaterNeighbors<G, true>(S, L, slot, pi, pos4, [&](int j) {
+        // D of the neighbour is loaded with its position and record for every
+        // pair (only approaching pairs use it): its latency then overlaps the
+        // pressure term instead of stalling inside the viscosity branch
+        struct Water {
+            float4 p, g;  // g: (velocity, P)
+            float D;
+        };
+        auto waterRecord = [&](int j) { return Water{pos4[j], grec4[j], dp[j].x}; };
+        forLabelNeighbors<false, G, true>(S, L, slot, pi, pos4, part, waterRecord, [&](int j, const Water& d) {
             if (j == slot) return;
-            const float4 pj = pos4[j];
-            const float4 gj = grec4[j];  // (velocity, P)
-            // D of the neighbour, loaded with its position and record for
-            // every pair (only approaching pairs use it): its latency then
-            // overlaps the pressure term instead of stalling inside the
-            // viscosity branch
-            const float dj = dp[j].x;
+            const float4 pj = d.p, gj = d.g;
+            const float dj = d.D;
             const float3 dij = pi - xyz(pj);
             const float3 nab = spikyGrad(S, dij);
             a += -pj.w * (pterm_i + gj.w) * nab;
@@ -154,18 +178,22 @@ __global__ void __launch_bounds__(kSlotAlign, 5) kWaterMomentum(
                 const float pij = -S.nu / (di + dj) * (dd / (dot3(dij, dij) + kEps));
                 a += -pj.w * pij * nab;
             }
-        }, part);
-        forSandNeighbors<G, true>(S, L, slot, pi, pos4, [&](int j) {
-            const float4 pj = pos4[j];
+        });
+        struct Sand {
+            float4 p, drag;  // drag: (average drag, density)
+        };
+        auto sandRecord = [&](int j) { return Sand{pos4[j], drag4[j]}; };
+        forLabelNeighbors<true, G, true>(S, L, slot, pi, pos4, part, sandRecord, [&](int, const Sand& d) {
+            const float4 pj = d.p;
             const float3 dij = pi - xyz(pj);
-            const float4 dragj = drag4[j];  // (average drag, density)
+            const float4 dragj = d.drag;
             const float dj = dragj.w;
             const float wij = poly6(S, len3(dij));
             const float3 nab = spikyGrad(S, dij);
             const float3 buoy = pj.w * pri / fmaxf(kEps, di * dj) * nab;  // -m_j with m_j = -w
             const float3 drag = -wij / di * xyz(dragj);
             a += buoy + drag;
-        }, part);
+        });
         const float bp = pri / fmaxf(kEps, S.rho0 * S.rho0);
         const float bvis = -S.bnu / (2.f * S.rho0);
         forBoundaryNeighbors<G>(S, L, slot, pi, bpos4, [&](int b) {
