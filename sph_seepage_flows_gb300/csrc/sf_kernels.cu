@@ -308,6 +308,8 @@ __device__ __forceinline__ float sandVolumeTerm(const SceneDev& S, float wj, flo
 // Hits of one slot waiting to be appended: (first candidate, hit mask) of up
 // to kHitChunks chunks of 32 candidates, per thread.
 constexpr int kHitChunks = 12;
+// Most slots for the form of the one-lane density pass that loads ahead.
+constexpr int kAheadSlots = 600000;
 
 // Builds the neighbour lists (sand / water / boundary, each in stencil
 // order, plus the sand-sand contact list) and computes the density, fused
@@ -339,7 +341,14 @@ constexpr int kHitChunks = 12;
 // memory costs L1 (286 us at 1M), with 10 the disturbed column drains in the
 // middle of the walk (304 us). 48 registers: with 40 the spills cost 281 us,
 // with 64 the occupancy 268 us at 1M.
-__global__ void __launch_bounds__(kSlotAlign, 5)
+//
+// kAhead: the hit phase loads the position of the next hit before it uses this
+// one's, with 64 registers (4 blocks of kSlotAlign threads per SM). That pays
+// while there are few waves of blocks (kAheadSlots): 40k 48 -> 43 us, 120k
+// 67 -> 63, 252k 90 -> 85, 306k of 12 scenes 147 -> 141; at a million the
+// occupancy is worth more (1M embankment 283 -> 286, 64 scenes 295 -> 306).
+template <bool kAhead>
+__global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
     kDensity(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, SceneState* __restrict__ state,
              NbrListsW L, const float4* __restrict__ pos4, const float4* __restrict__ pairXY,
              const float2* __restrict__ pairZ, const float4* __restrict__ bpos4, float4* __restrict__ vel4,
@@ -406,42 +415,68 @@ __global__ void __launch_bounds__(kSlotAlign, 5)
     // then cell by cell the water and the boundary neighbours), sand its
     // contacts (DEM + liquid-bridge reach, itself excluded) and the volume of
     // the sand around it
+    auto take = [&](unsigned j, float4 pj) {
+        const float3 dij = pi - xyz(pj);
+        // the list overflows when its two parts meet: from then on
+        // nothing reads it, so the order of the two appends is free
+        const bool room = cS + cW < L.cap;
+        if (pj.w < 0.f) {
+            if (room) entry(L.nbr, cS) = j;
+            ++cS;
+            if (!water) {
+                const float d2 = dot3(dij, dij);
+                if (j != unsigned(slot) && d2 < S.dem_reach2) {
+                    if (cc < kMaxContact) entry(L.cnbr, cc) = j;
+                    ++cc;
+                }
+                sum += sandVolumeTerm(S, pj.w, pi4.w, vol, sqrtf(d2));
+            }
+        } else {
+            if (room) entry(L.nbr, L.cap - 1 - cW) = j;
+            ++cW;
+            if (water) {
+                while (j >= bEnd) boundaryTerm();
+                sum += pj.w * poly6(S, len3(dij));
+            }
+        }
+    };
     auto drain = [&]() {
         unsigned base = 0u, mask = 0u;
-        for (int q = 0;;) {
+        int q = 0;
+        // the next waiting hit (its candidate in j), false when there is none
+        auto next = [&](unsigned& j) {
             if (mask == 0u) {
-                if (q == nq) break;
+                if (q == nq) return false;
                 const uint2 h = mine[q * stride];
                 ++q;
                 base = h.x;
                 mask = h.y;
             }
-            const unsigned j = base + unsigned(__ffs(mask) - 1);
+            j = base + unsigned(__ffs(mask) - 1);
             mask &= mask - 1u;
-            const float4 pj = pos4[j];
-            const float3 dij = pi - xyz(pj);
-            // the list overflows when its two parts meet: from then on
-            // nothing reads it, so the order of the two appends is free
-            const bool room = cS + cW < L.cap;
-            if (pj.w < 0.f) {
-                if (room) entry(L.nbr, cS) = j;
-                ++cS;
-                if (!water) {
-                    const float d2 = dot3(dij, dij);
-                    if (j != unsigned(slot) && d2 < S.dem_reach2) {
-                        if (cc < kMaxContact) entry(L.cnbr, cc) = j;
-                        ++cc;
+            return true;
+        };
+        unsigned j = 0u;
+        if constexpr (kAhead) {
+            if (next(j)) {
+                float4 pj = pos4[j];
+                unsigned jn = 0u;
+                bool more = next(jn);
+                for (;;) {
+                    const unsigned ji = j;
+                    const float4 p = pj;
+                    const bool go = more;
+                    if (go) {
+                        j = jn;
+                        pj = pos4[jn];
+                        more = next(jn);
                     }
-                    sum += sandVolumeTerm(S, pj.w, pi4.w, vol, sqrtf(d2));
-                }
-            } else {
-                if (room) entry(L.nbr, L.cap - 1 - cW) = j;
-                ++cW;
-                if (water) {
-                    while (j >= bEnd) boundaryTerm();
-                    sum += pj.w * poly6(S, len3(dij));
+                    take(ji, p);
+                    if (!go) break;
                 }
             }
+        } else {
+            while (next(j)) take(j, pos4[j]);
         }
         nq = 0;
     };
@@ -1280,7 +1315,8 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
                 c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4, cap);
         } else {
             const size_t hits = size_t(kHitChunks) * c.block[kPassDensity] * sizeof(uint2);
-            kDensity<<<grid(c, kPassDensity), c.block[kPassDensity], hits, c.stream>>>(
+            const auto kernel = c.slotBlocks <= kAheadSlots / kSlotAlign ? kDensity<true> : kDensity<false>;
+            kernel<<<grid(c, kPassDensity), c.block[kPassDensity], hits, c.stream>>>(
                 c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4);
         }
         break;
