@@ -85,6 +85,16 @@ struct SceneState {
     unsigned int list_need;  // largest neighbour count above 7/8 of the list capacity (0: none)
 };
 
+// Programmatic dependent launch: the passes of a substep are a chain of short
+// kernels, each launched while the one before drains (launchChained in
+// sf_kernels.h) and held here until it has finished. Returns i unchanged; what
+// a kernel reads is addressed through it, so that no load, not even one from
+// memory that the kernel itself never writes, can move ahead of the wait.
+__device__ __forceinline__ int afterPrevious(int i) {
+    asm volatile("griddepcontrol.wait;" : "+r"(i) : : "memory");
+    return i;
+}
+
 // ---------------------------------------------------------------- float3 math
 __device__ __forceinline__ float3 mk3(float x, float y, float z) { return make_float3(x, y, z); }
 __device__ __forceinline__ float3 xyz(float4 v) { return make_float3(v.x, v.y, v.z); }

@@ -38,7 +38,7 @@
 namespace sfg {
 
 #define SF_SLOT_PROLOGUE                                                   \
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;                \
+    const int slot = blockIdx.x * blockDim.x + afterPrevious(threadIdx.x); \
     const int sid = blockScene[(blockIdx.x * blockDim.x) / kSlotAlign];    \
     const SceneDev& S = scenes[sid];
 
@@ -1298,8 +1298,8 @@ void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, co
 }
 
 template <int G> void launchDensityLanes(const LaunchCtx& c, const PassBuffers& b) {
-    kDensityLanes<G><<<grid(c, kPassDensity) * G, c.block[kPassDensity], 0, c.stream>>>(
-        c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4);
+    launchChained(c.stream, grid(c, kPassDensity) * G, c.block[kPassDensity], 0, kDensityLanes<G>, c.scenes,
+                  c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4);
 }
 void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
     switch (c.lanes[kPassDensity]) {
@@ -1316,8 +1316,8 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
         } else {
             const size_t hits = size_t(kHitChunks) * c.block[kPassDensity] * sizeof(uint2);
             const auto kernel = c.slotBlocks <= kAheadSlots / kSlotAlign ? kDensity<true> : kDensity<false>;
-            kernel<<<grid(c, kPassDensity), c.block[kPassDensity], hits, c.stream>>>(
-                c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4);
+            launchChained(c.stream, grid(c, kPassDensity), c.block[kPassDensity], hits, kernel, c.scenes,
+                          c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4);
         }
         break;
     }
@@ -1326,11 +1326,11 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
 template <int G> void launchAvgFlowG(const LaunchCtx& c, const PassBuffers& b, bool summed) {
     const int blocks = grid(c, kPassAvgFlow) * G, threads = c.block[kPassAvgFlow];
     if (summed)
-        kAvgFlow<G, true><<<blocks, threads, 0, c.stream>>>(c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4,
-                                                            b.flow4, b.vrec2, b.grec4);
+        launchChained(c.stream, blocks, threads, 0, kAvgFlow<G, true>, c.scenes, c.blockScene, b.lists, b.pos4,
+                      b.vel4, b.aux4, b.flow4, b.vrec2, b.grec4);
     else
-        kAvgFlow<G, false><<<blocks, threads, 0, c.stream>>>(c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4,
-                                                             b.flow4, b.vrec2, b.grec4);
+        launchChained(c.stream, blocks, threads, 0, kAvgFlow<G, false>, c.scenes, c.blockScene, b.lists, b.pos4,
+                      b.vel4, b.aux4, b.flow4, b.vrec2, b.grec4);
 }
 void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b, bool chained) {
     // the staged form of the density pass does not sum the sand volume
@@ -1344,9 +1344,9 @@ void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b, bool chained) {
 }
 
 template <int G> void launchVoidageAdhesionG(const LaunchCtx& c, const PassBuffers& b) {
-    kVoidageAdhesion<G><<<grid(c, kPassVoidage) * G, c.block[kPassVoidage], 0, c.stream>>>(
-        c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4, b.flow4, b.adh4, b.avgadh4, b.col4, b.dp, b.vrec2,
-        b.grec4);
+    launchChained(c.stream, grid(c, kPassVoidage) * G, c.block[kPassVoidage], 0, kVoidageAdhesion<G>, c.scenes,
+                  c.blockScene, b.lists, b.pos4, b.vel4, b.aux4, b.flow4, b.adh4, b.avgadh4, b.col4, b.dp, b.vrec2,
+                  b.grec4);
 }
 void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b) {
     switch (c.lanes[kPassVoidage]) {
@@ -1358,10 +1358,9 @@ void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b) {
 }
 
 void launchIntegrate(const LaunchCtx& c, const PassBuffers& b, float timeArg, int adaptive, const float* timeArgDev) {
-    kIntegrate<<<grid(c, kPassIntegrate), c.block[kPassIntegrate], 0, c.stream>>>(c.scenes, c.blockScene, c.state,
-                                                          timeArg, timeArgDev, adaptive,
-                                                          b.lists.bcs, b.bpos4, b.pos4, b.vel4, b.acc4, b.adh4,
-                                                          b.avgadh4);
+    launchChained(c.stream, grid(c, kPassIntegrate), c.block[kPassIntegrate], 0, kIntegrate, c.scenes, c.blockScene,
+                  c.state, timeArg, timeArgDev, adaptive, b.lists.bcs, b.bpos4, b.pos4, b.vel4, b.acc4, b.adh4,
+                  b.avgadh4);
 }
 
 }  // namespace sfg

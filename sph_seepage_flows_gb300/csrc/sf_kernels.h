@@ -6,6 +6,28 @@
 
 namespace sfg {
 
+// Launches a kernel that starts with afterPrevious (sf_device.cuh), which lets
+// the GPU set it up while the kernel before it in the stream drains; captured
+// graphs keep the edge as such. A substep of ten kernels: 1,770 particles 52 ->
+// 50 us, 20k column 76 -> 74, 1M embankment 572 -> 565. The kernels do not
+// release their successors early (griddepcontrol.launch_dependents): the next
+// kernel's blocks then wait on the SMs for all of this one, and the substeps
+// became 2-3 us longer.
+template <typename... P, typename... A>
+inline void launchChained(cudaStream_t s, int blocks, int threads, size_t shared, void (*kernel)(P...), A... args) {
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(blocks));
+    cfg.blockDim = dim3(unsigned(threads));
+    cfg.dynamicSmemBytes = shared;
+    cfg.stream = s;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 struct SceneDev;
 struct SceneState;
 

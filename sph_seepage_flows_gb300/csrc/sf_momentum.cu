@@ -237,9 +237,9 @@ __global__ void __launch_bounds__(kSlotAlign, 4) kWaterMomentum(
 static inline int grid(const LaunchCtx& c, int pass) { return c.slotBlocks * (kSlotAlign / c.block[pass]); }
 
 template <int G> void launchSandMomentumG(const LaunchCtx& c, const PassBuffers& b) {
-    kSandMomentum<G><<<grid(c, kPassSand) * G, c.block[kPassSand], 0, c.stream>>>(
-        c.scenes, c.blockScene, b.lists, b.pos4, b.vel4, b.aux4, b.flow4, b.avgadh4, b.mat4, b.bpos4, b.dp, b.grec4,
-        b.drag4, b.acc4);
+    launchChained(c.stream, grid(c, kPassSand) * G, c.block[kPassSand], 0, kSandMomentum<G>, c.scenes, c.blockScene,
+                  b.lists, b.pos4, b.vel4, b.aux4, b.flow4, b.avgadh4, b.mat4, b.bpos4, b.dp, b.grec4, b.drag4,
+                  b.acc4);
 }
 void launchSandMomentum(const LaunchCtx& c, const PassBuffers& b) {
     switch (c.lanes[kPassSand]) {
@@ -251,9 +251,9 @@ void launchSandMomentum(const LaunchCtx& c, const PassBuffers& b) {
 }
 
 template <int G> void launchWaterMomentumG(const LaunchCtx& c, const PassBuffers& b) {
-    kWaterMomentum<G><<<grid(c, kPassWater) * G, c.block[kPassWater], 0, c.stream>>>(
-        c.scenes, c.blockScene, c.state, b.lists, b.pos4, b.vel4, b.aux4, b.drag4, b.adh4, b.bpos4, b.dp, b.grec4,
-        b.acc4, c.errWord);
+    launchChained(c.stream, grid(c, kPassWater) * G, c.block[kPassWater], 0, kWaterMomentum<G>, c.scenes,
+                  c.blockScene, c.state, b.lists, b.pos4, b.vel4, b.aux4, b.drag4, b.adh4, b.bpos4, b.dp, b.grec4,
+                  b.acc4, c.errWord);
 }
 void launchWaterMomentum(const LaunchCtx& c, const PassBuffers& b) {
     switch (c.lanes[kPassWater]) {

@@ -14,7 +14,7 @@ namespace sfg {
 // sums are already in a different order from the reference's, so the split
 // only moves FP32 rounding; small scenes get G times the threads in flight.
 #define SF_SLOT_PROLOGUE_G                                                      \
-    const int gid = blockIdx.x * blockDim.x + threadIdx.x;                      \
+    const int gid = blockIdx.x * blockDim.x + afterPrevious(threadIdx.x);       \
     const int slot = gid / G, part = gid % G;                                   \
     const int sid = blockScene[(blockIdx.x * (blockDim.x / G)) / kSlotAlign];   \
     const SceneDev& S = scenes[sid];

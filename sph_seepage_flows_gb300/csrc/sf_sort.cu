@@ -443,7 +443,7 @@ __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restr
     __shared__ unsigned int parked, parkedBase;
     if (threadIdx.x == 0) parked = 0u;
     __syncthreads();
-    const int slot = blockIdx.x * kSlotAlign + threadIdx.x;
+    const int slot = blockIdx.x * kSlotAlign + afterPrevious(threadIdx.x);
     const SceneDev& S = scenes[blockScene[blockIdx.x]];
     const float4 p = pos4[slot];
     const bool live = p.w != 0.f;
@@ -471,7 +471,7 @@ __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restr
 // place and writes its sum.
 __global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int nCells) {
     unsigned int carry = 0u, total;
-    const int tileBeg = int(blockIdx.x) << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
+    const int tileBeg = afterPrevious(int(blockIdx.x)) << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
     for (int base = tileBeg; base < tileEnd; base += kScanChunk) {
         const int c = base + int(threadIdx.x) * kScanItems;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -489,14 +489,15 @@ __global__ void __launch_bounds__(kSortThreads) kCountScatter(CountScratch cc, i
     // every block scans the (at most kMaxCountTiles) tile sums
     __shared__ unsigned int before[kMaxCountTiles];
     unsigned int carry = 0u, total;
+    const int tid = afterPrevious(threadIdx.x);
     for (int base = 0; base < tiles; base += kSortThreads) {
-        const int t = base + int(threadIdx.x);
+        const int t = base + tid;
         const unsigned int a = blockScan(t < tiles ? cc.tileCount[t] : 0u, total);
         if (t < tiles) before[t] = carry + a;
         carry += total;
     }
     __syncthreads();
-    const int first = blockIdx.x * kSortThreads + threadIdx.x, threads = gridDim.x * kSortThreads;
+    const int first = blockIdx.x * kSortThreads + tid, threads = gridDim.x * kSortThreads;
     for (int i = first; i < n; i += threads) {
         const uint2 kr = cc.keyRank[i];
         cc.arrived[cc.count[kr.x] + before[kr.x >> cc.tileShift] + kr.y] = unsigned(i);
@@ -512,7 +513,7 @@ __global__ void __launch_bounds__(kSortThreads)
                  float4* __restrict__ velOut, float4* __restrict__ colOut, float4* __restrict__ matOut,
                  float2* __restrict__ amcOut, int* __restrict__ pidOut, float* __restrict__ pairXY,
                  float* __restrict__ pairZ) {
-    const int i = blockIdx.x * kSortThreads + threadIdx.x;
+    const int i = blockIdx.x * kSortThreads + afterPrevious(threadIdx.x);
     for (int c = i; c < ((nCells + 3) & ~3); c += gridDim.x * kSortThreads) cc.count[c] = 0u;
     if (i >= n) return;
     const unsigned int o = cc.arrived[i];
@@ -544,13 +545,13 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
                        float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
                        unsigned int* cellStart, float4* pairXY, float2* pairZ) {
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
-    kCountKeys<<<blocks, kSlotAlign, 0, c.stream>>>(c.scenes, c.blockScene, pos, cc, c.errWord);
-    kCellScan<<<tiles, kSortThreads, 0, c.stream>>>(cc, nCells);
-    kCountScatter<<<std::min(blocks, kScatterBlocks), kSortThreads, 0, c.stream>>>(cc, n, nCells, tiles, cellStart);
-    kCellReorder<<<blocks, kSortThreads, 0, c.stream>>>(cc, n, nCells, cellStart, pos, vel, col, mat, amc, pid, posOut, velOut,
-                                                        colOut, matOut, amcOut, pidOut,
-                                                        reinterpret_cast<float*>(pairXY),
-                                                        reinterpret_cast<float*>(pairZ));
+    launchChained(c.stream, blocks, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc, c.errWord);
+    launchChained(c.stream, tiles, kSortThreads, 0, kCellScan, cc, nCells);
+    launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
+                  cellStart);
+    launchChained(c.stream, blocks, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
+                  pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
+                  reinterpret_cast<float*>(pairZ));
     return 4;
 }
 
