@@ -218,6 +218,10 @@ struct sf_handle {
     bool countingSort = false;  // by cell count and slot count (useCountingSort), else the radix sort
     unsigned int *cellCount = nullptr, *tileCount = nullptr;
     uint2* keyRank = nullptr;
+    // the keys and counts of the counting sort: none (counts zero), of the
+    // positions as they are (left by the integrator or the key kernel), or of
+    // positions that have changed since
+    enum { kCountsZero, kCountsReady, kCountsStale } counts = kCountsZero;
     float4* bpos = nullptr;
     int* blabel = nullptr;
     // staging for field access
@@ -340,6 +344,14 @@ struct sf_handle {
         b.grec4 = grec4;
         return b;
     }
+    // positions or buffers changed outside the substep's passes
+    void positionsChanged() {
+        pairsFresh = false;
+        if (counts == kCountsReady) counts = kCountsStale;
+    }
+    CountScratch countScratch() const {
+        return CountScratch{cellCount, tileCount, keyRank, sc.vals, keys, countTileShift(totalCells)};
+    }
     void setLanes(int all) { lanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
     void setAutomaticLanes(int smCount) {
         setLanes(lanesForSlots(totalSlots, smCount));
@@ -448,18 +460,36 @@ struct sf_handle {
 
 namespace {
 
+sf_status clearCounts(sf_handle* h) {
+    h->counts = sf_handle::kCountsZero;
+    return h->cuda(cudaMemsetAsync(h->cellCount, 0, sizeof(unsigned) * (size_t(h->totalCells) + 4), h->stream),
+                   "clear cell counts");
+}
+
+// The counting sort's keys and counts of the current positions.
+sf_status ensureCounts(sf_handle* h) {
+    if (!h->countingSort || h->counts == sf_handle::kCountsReady) return SF_OK;
+    if (h->counts == sf_handle::kCountsStale)
+        if (sf_status st = clearCounts(h)) return st;
+    launchCountKeys(h->ctx(), h->totalSlots, h->pos[h->cur], h->countScratch());
+    h->launches += 1;
+    h->counts = sf_handle::kCountsReady;
+    return h->cuda(cudaGetLastError(), "count keys launch");
+}
+
 // The sort stage: the counting sort by cell, or keys (with the first radix
 // pass's tile histograms), stable radix sort and reorder into the other buffer
 // set (with the cell table).
 sf_status runSort(sf_handle* h) {
     LaunchCtx c = h->ctx();
     if (h->countingSort) {
-        const CountScratch cc{h->cellCount, h->tileCount, h->keyRank, h->sc.vals, h->keys,
-                              countTileShift(h->totalCells)};
+        if (sf_status st = ensureCounts(h)) return st;
+        const CountScratch cc = h->countScratch();
         const int o = h->cur, t = 1 - h->cur;
         h->launches += launchCountingSort(c, h->totalSlots, h->totalCells, cc, h->pos[o], h->vel[o], h->col[o],
                                           h->mat[o], h->amc[o], h->pid[o], h->pos[t], h->vel[t], h->col[t], h->mat[t],
                                           h->amc[t], h->pid[t], h->cs, h->pairXY, h->pairZ);
+        h->counts = sf_handle::kCountsZero;
         h->sortedKeys = cc.sortedKeys;
         h->pairsFresh = true;
         h->cur = t;
@@ -499,8 +529,12 @@ sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive, bool ch
     case SF_STAGE_SAND_MOMENTUM: launchSandMomentum(c, b); break;
     case SF_STAGE_WATER_MOMENTUM: launchWaterMomentum(c, b); break;
     case SF_STAGE_INTEGRATE:
-        launchIntegrate(c, b, timeArg, adaptive, h->captureStep ? h->dTimeArg : nullptr);
+        if (h->countingSort && h->counts != sf_handle::kCountsZero)  // no sort since the last count
+            if (sf_status st = clearCounts(h)) return st;
+        launchIntegrate(c, b, timeArg, adaptive, h->captureStep ? h->dTimeArg : nullptr,
+                        h->countingSort ? h->countScratch() : CountScratch{});
         h->pairsFresh = false;
+        if (h->countingSort) h->counts = sf_handle::kCountsReady;
         break;
     default: return h->fail(SF_ERR_INVALID, "unknown stage");
     }
@@ -541,7 +575,7 @@ sf_status countNeighborsMax(sf_handle* h, unsigned* maxCount) {
     if (!sorted) {
         h->cur = cur;
         h->sorted = false;
-        h->pairsFresh = false;
+        h->positionsChanged();
     }
     return SF_OK;
 }
@@ -954,14 +988,21 @@ static sf_status ensureStepGraph(sf_handle* h, GraphCache& g) {
     if (g.exec) return SF_OK;
     const int curBefore = h->cur;
     const int64_t launchesBefore = h->launches;
+    // (graphs begin with the sort from counts: see ensureCounts before a replay)
+    const auto countsBefore = h->counts;
+    h->counts = sf_handle::kCountsReady;
     cudaGraph_t graph = nullptr;
     sf_status st = h->cuda(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
-    if (st) return st;
+    if (st) {
+        h->counts = countsBefore;
+        return st;
+    }
     h->captureStep = true;
     st = runSubstep(h, 0.f, 1);
     h->captureStep = false;
     const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
     h->cur = curBefore;
+    h->counts = countsBefore;
     g.nodes = int(h->launches - launchesBefore);
     h->launches = launchesBefore;
     if (st != SF_OK) {
@@ -994,13 +1035,14 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
         h->timeArg = t;
     }
     GraphCache& g = h->graphStep[h->cur];
-    sf_status st = ensureStepGraph(h, g);
-    if (st != SF_OK) return st;
+    sf_status st = ensureCounts(h);
+    if (st != SF_OK || (st = ensureStepGraph(h, g)) != SF_OK) return st;
     if (h->cuda(cudaGraphLaunch(g.exec, h->stream), "graph launch")) return SF_ERR_CUDA;
     h->launches += g.nodes;
     h->cur = 1 - h->cur;
     h->sorted = true;
     h->pairsFresh = false;
+    if (h->countingSort) h->counts = sf_handle::kCountsReady;
     const int copy = queueStateCopy(h);
     if (ms_out) {
         cudaEventRecord(e1, h->stream);
@@ -1052,12 +1094,15 @@ static sf_status ensureGraph(sf_handle* h, GraphCache& g, int nsub, float dt) {
     }
     const int curBefore = h->cur;
     const int64_t launchesBefore = h->launches;
+    const auto countsBefore = h->counts;
     cudaGraph_t graph = nullptr;
     sf_status st = h->cuda(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
     if (st) return st;
+    h->counts = sf_handle::kCountsReady;
     for (int k = 0; k < nsub && st == SF_OK; ++k) st = runSubstep(h, dt, 0);
     cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
     h->cur = curBefore;
+    h->counts = countsBefore;
     g.nodes = int(h->launches - launchesBefore);
     h->launches = launchesBefore;
     if (st != SF_OK) {
@@ -1076,7 +1121,8 @@ namespace {
 
 // n fixed-dt substeps replayed from the captured graphs.
 sf_status queueSubstepsFixed(sf_handle* h, float dt, int64_t n) {
-    sf_status st = SF_OK;
+    sf_status st = ensureCounts(h);
+    if (st) return st;
     if (n % 2 == 1) {  // the odd substep from a one-substep graph of this buffer set
         GraphCache& g1 = h->graph1[h->cur];
         if ((st = ensureGraph(h, g1, 1, dt))) return st;
@@ -1094,6 +1140,7 @@ sf_status queueSubstepsFixed(sf_handle* h, float dt, int64_t n) {
     }
     h->sorted = true;
     h->pairsFresh = false;
+    if (h->countingSort) h->counts = sf_handle::kCountsReady;
     return SF_OK;
 }
 
@@ -1519,9 +1566,14 @@ sf_status sf_get_fields(sf_handle* h, int32_t scene, int32_t n_fields, const int
 
 namespace {
 
+// Fields that a slot's cell or its parking depends on.
+bool movesParticles(int field) {
+    return field == SF_FIELD_POS || field == SF_FIELD_LABEL || field == SF_FIELD_MASS;
+}
+
 sf_status launchSetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
     for (int k = 0; k < list.n; ++k)
-        if (list.field[k] == SF_FIELD_POS) h->pairsFresh = false;
+        if (movesParticles(list.field[k])) h->positionsChanged();
     kSetFields<<<int((n + 255) / 256), 256, 0, h->stream>>>(list, int(n), h->hScenes[scene].slot_off, order,
                                                            fieldArrays(h), h->dScenes + scene);
     return h->cuda(cudaGetLastError(), "set_field launch");
@@ -1549,7 +1601,7 @@ sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
     float4* vec = order == SF_ORDER_SORTED ? vec3Array(h, field) : nullptr;
     if (!vec || (reinterpret_cast<uintptr_t>(from) & 15u) != 0)
         return launchSetFields(h, scene, oneField(field, from), order, n);
-    if (field == SF_FIELD_POS) h->pairsFresh = false;
+    if (movesParticles(field)) h->positionsChanged();
     kSetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
         int(n), h->hScenes[scene].slot_off, vec, static_cast<const float4*>(from),
         field == SF_FIELD_VEL ? h->grec4 : nullptr);
@@ -1691,7 +1743,7 @@ sf_status sf_add_sph_particles(sf_handle* h, int32_t scene, const float* pos3, i
         return SF_ERR_CUDA;
     h->n[scene] += n;
     h->nextId[scene] += n;
-    h->pairsFresh = false;
+    h->positionsChanged();
     return SF_OK;
 }
 
@@ -1704,8 +1756,11 @@ __global__ void __launch_bounds__(kSlotAlign) kResetOrder(const SceneDev* __rest
                                                           const int* __restrict__ blockScene, FieldArrays from,
                                                           float4* __restrict__ pos2, float4* __restrict__ vel2,
                                                           float4* __restrict__ col2, float4* __restrict__ mat2,
-                                                          float2* __restrict__ amc2, int* __restrict__ pid2) {
+                                                          float2* __restrict__ amc2, int* __restrict__ pid2,
+                                                          unsigned int* __restrict__ cellCount, int nCells) {
     const int s = blockIdx.x * kSlotAlign + threadIdx.x;
+    if (cellCount)  // the counts were those of the old order
+        for (int c = s; c < nCells; c += gridDim.x * kSlotAlign) cellCount[c] = 0u;
     const int id = from.pid[s];
     const int d = id >= 0 ? scenes[blockScene[blockIdx.x]].slot_off + id : s;
     pos2[d] = from.pos[s];
@@ -1722,11 +1777,14 @@ sf_status sf_reset_order(sf_handle* h) {
     if (!h) return SF_ERR_INVALID;
     const int t = 1 - h->cur;
     kResetOrder<<<h->slotBlocks, kSlotAlign, 0, h->stream>>>(h->dScenes, h->dBlockScene, fieldArrays(h), h->pos[t],
-                                                             h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t]);
+                                                             h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t],
+                                                             h->counts != sf_handle::kCountsZero ? h->cellCount : nullptr,
+                                                             h->totalCells + 4);
     h->launches += 1;
     h->cur = t;
     h->sorted = false;
     h->pairsFresh = false;
+    h->counts = sf_handle::kCountsZero;
     return h->cuda(cudaGetLastError(), "reset order launch");
 }
 
@@ -1946,7 +2004,7 @@ size_t snapStride(const sf_handle* h) {
 }
 
 sf_status snapCopy(sf_handle* h, char* snap, bool save) {
-    if (!save) h->pairsFresh = false;
+    if (!save) h->positionsChanged();
     const size_t M = size_t(h->totalSlots);
     const int c = h->cur;
     void* arrays[6] = {h->pos[c], h->vel[c], h->col[c], h->mat[c], h->amc[c], h->pid[c]};
@@ -2088,12 +2146,15 @@ sf_status runSubstepStoreGraphed(sf_handle* h, float dt, int64_t t) {
         }
         const int curBefore = h->cur;
         const int64_t launchesBefore = h->launches;
+        const auto countsBefore = h->counts;
         cudaGraph_t graph = nullptr;
         sf_status st = h->cuda(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         if (st) return st;
+        h->counts = sf_handle::kCountsReady;
         st = runSubstepStore(h, dt, slabAt(h, h->slab + size_t(t) * slabStride(h)));
         cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
         h->cur = curBefore;
+        h->counts = countsBefore;
         g.nodes = int(h->launches - launchesBefore);
         h->launches = launchesBefore;
         if (st != SF_OK) {
@@ -2106,11 +2167,13 @@ sf_status runSubstepStoreGraphed(sf_handle* h, float dt, int64_t t) {
         if (st) return st;
         g.dt = dt;
     }
+    if (sf_status st = ensureCounts(h)) return st;
     if (h->cuda(cudaGraphLaunch(g.exec, h->stream), "graph launch")) return SF_ERR_CUDA;
     h->launches += g.nodes;
     h->cur = 1 - h->cur;
     h->sorted = true;
     h->pairsFresh = false;
+    if (h->countingSort) h->counts = sf_handle::kCountsReady;
     return SF_OK;
 }
 

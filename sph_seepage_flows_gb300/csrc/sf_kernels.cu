@@ -31,6 +31,7 @@
 // magnitudes).
 #include <algorithm>
 
+#include "sf_count.cuh"
 #include "sf_device.cuh"
 #include "sf_kernels.h"
 #include "sf_neighbors.cuh"
@@ -1164,7 +1165,10 @@ __global__ void __launch_bounds__(kSlotAlign, 4) kVoidageAdhesion(
 // then CudaSFParticles::Advect with AccDampingForSand (cuda_sf_particles.cu:
 // 18-48, cuda_sf_particles.cuh:19-40) and SFWaterBoundaryConstrain_CUDA
 // (cuda_sph_sf_solver_gpu.cuh:979-1074). adaptive: timeArg is the render
-// interval and dt = timeArg / N_sub; otherwise dt = timeArg.
+// interval and dt = timeArg / N_sub; otherwise dt = timeArg. The new positions
+// are counted into their cells for the next sort (countSlot), which then needs
+// no pass over them of its own: 8 adaptive steps of 40k particles 817 -> 764
+// us, 16 substeps of the 20k column 1223 -> 1178, 8 at 1M 4696 -> 4665.
 __device__ __forceinline__ long long cflSubsteps(const SceneDev& S, float amax, float T) {
     if (!S.wcsph) {
         const float q = T / S.params_dt;
@@ -1184,7 +1188,8 @@ __global__ void kIntegrate(const SceneDev* __restrict__ scenes, const int* __res
                            int adaptive,
                            const unsigned int* __restrict__ bcs, const float4* __restrict__ bpos4,
                            float4* __restrict__ pos4, float4* __restrict__ vel4, float4* __restrict__ acc4,
-                           float4* __restrict__ adh4, float4* __restrict__ avgadh4) {
+                           float4* __restrict__ adh4, float4* __restrict__ avgadh4, CountScratch cc,
+                           unsigned int* errWord) {
     SF_SLOT_PROLOGUE
     if (timeArgDev) timeArg = *timeArgDev;  // a graph-replayed step reads the time from the device
     float dt = timeArg;
@@ -1202,50 +1207,54 @@ __global__ void kIntegrate(const SceneDev* __restrict__ scenes, const int* __res
         state[sid].dt = dt;
     }
     float4 p4 = pos4[slot];
-    if (p4.w == 0.f) return;
-    float4 v4 = vel4[slot];
-    float3 a = xyz(acc4[slot]);
-    float3 v = xyz(v4);
-    if (p4.w < 0.f) {
-        const float3 q = a * (v + 0.5f * dt * a);
-        const float3 s = mk3(float(sgn1(q.x)), float(sgn1(q.y)), float(sgn1(q.z)));
-        a = a * (mk3(1.f, 1.f, 1.f) - S.damping * s);
-        acc4[slot] = make_float4(a.x, a.y, a.z, 0.f);
-    }
-    v = v + dt * a;
-    float3 p = xyz(p4) + dt * v;
-    if (p4.w > 0.f) {
-        const float r2 = 2.f * S.sph_radius;
-        float3 tp = p, tv = v;
-        if (tp.x > S.hpx - r2) { tp.x = S.hpx - r2; tv.x = fminf(tv.x, 0.f); }
-        if (tp.x < S.lpx + r2) { tp.x = S.lpx + r2; tv.x = fmaxf(tv.x, 0.f); }
-        if (tp.y > S.hpy - r2) { tp.y = S.hpy - r2; tv.y = fminf(tv.y, 0.f); }
-        if (tp.y < S.lpy + r2) { tp.y = S.lpy + r2; tv.y = fmaxf(tv.y, 0.f); }
-        if (tp.z > S.hpz - r2) { tp.z = S.hpz - r2; tv.z = fminf(tv.z, 0.f); }
-        if (tp.z < S.lpz + r2) { tp.z = S.lpz + r2; tv.z = fmaxf(tv.z, 0.f); }
-        if (S.shape_boundary) {  // only boundary particles with label 1 push water out
-            forEachCell(S, cellOf(S, p), [&](int cell) {
-                for (unsigned j = bcs[cell]; j < bcs[cell + 1]; ++j) {
-                    const float4 bj = bpos4[j];
-                    if (!(bj.w < 0.f)) continue;
-                    const float dpij = len3(p - xyz(bj));
-                    const float overlap = dpij - r2;
-                    if (overlap < 0.f) {
-                        const float3 nn = (p - xyz(bj)) / dpij;
-                        tv = tv * 0.f;
-                        tp += nn * -overlap;
-                    }
-                }
-            });
+    if (p4.w != 0.f) {
+        float4 v4 = vel4[slot];
+        float3 a = xyz(acc4[slot]);
+        float3 v = xyz(v4);
+        if (p4.w < 0.f) {
+            const float3 q = a * (v + 0.5f * dt * a);
+            const float3 s = mk3(float(sgn1(q.x)), float(sgn1(q.y)), float(sgn1(q.z)));
+            a = a * (mk3(1.f, 1.f, 1.f) - S.damping * s);
+            acc4[slot] = make_float4(a.x, a.y, a.z, 0.f);
         }
-        p = tp;
-        v = tv;
+        v = v + dt * a;
+        float3 p = xyz(p4) + dt * v;
+        if (p4.w > 0.f) {
+            const float r2 = 2.f * S.sph_radius;
+            float3 tp = p, tv = v;
+            if (tp.x > S.hpx - r2) { tp.x = S.hpx - r2; tv.x = fminf(tv.x, 0.f); }
+            if (tp.x < S.lpx + r2) { tp.x = S.lpx + r2; tv.x = fmaxf(tv.x, 0.f); }
+            if (tp.y > S.hpy - r2) { tp.y = S.hpy - r2; tv.y = fminf(tv.y, 0.f); }
+            if (tp.y < S.lpy + r2) { tp.y = S.lpy + r2; tv.y = fmaxf(tv.y, 0.f); }
+            if (tp.z > S.hpz - r2) { tp.z = S.hpz - r2; tv.z = fminf(tv.z, 0.f); }
+            if (tp.z < S.lpz + r2) { tp.z = S.lpz + r2; tv.z = fmaxf(tv.z, 0.f); }
+            if (S.shape_boundary) {  // only boundary particles with label 1 push water out
+                forEachCell(S, cellOf(S, p), [&](int cell) {
+                    for (unsigned j = bcs[cell]; j < bcs[cell + 1]; ++j) {
+                        const float4 bj = bpos4[j];
+                        if (!(bj.w < 0.f)) continue;
+                        const float dpij = len3(p - xyz(bj));
+                        const float overlap = dpij - r2;
+                        if (overlap < 0.f) {
+                            const float3 nn = (p - xyz(bj)) / dpij;
+                            tv = tv * 0.f;
+                            tp += nn * -overlap;
+                        }
+                    }
+                });
+            }
+            p = tp;
+            v = tv;
+        }
+        p4 = make_float4(p.x, p.y, p.z, p4.w);
+        pos4[slot] = p4;
+        vel4[slot] = make_float4(v.x, v.y, v.z, v4.w);
+        // the two thrust::fill clears of cuda_sph_sf_solver.cu:384-385
+        adh4[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+        avgadh4[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
-    pos4[slot] = make_float4(p.x, p.y, p.z, p4.w);
-    vel4[slot] = make_float4(v.x, v.y, v.z, v4.w);
-    // the two thrust::fill clears of cuda_sph_sf_solver.cu:384-385
-    adh4[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
-    avgadh4[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
+    // the next sort's keys and counts
+    if (cc.keyRank) countSlot(S, slot, p4, cc, errWord);
 }
 
 // ------------------------------------------------- neighbour-count probe
@@ -1357,10 +1366,11 @@ void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b) {
     }
 }
 
-void launchIntegrate(const LaunchCtx& c, const PassBuffers& b, float timeArg, int adaptive, const float* timeArgDev) {
+void launchIntegrate(const LaunchCtx& c, const PassBuffers& b, float timeArg, int adaptive, const float* timeArgDev,
+                     const CountScratch& cc) {
     launchChained(c.stream, grid(c, kPassIntegrate), c.block[kPassIntegrate], 0, kIntegrate, c.scenes, c.blockScene,
                   c.state, timeArg, timeArgDev, adaptive, b.lists.bcs, b.bpos4, b.pos4, b.vel4, b.acc4, b.adh4,
-                  b.avgadh4);
+                  b.avgadh4, cc, c.errWord);
 }
 
 }  // namespace sfg

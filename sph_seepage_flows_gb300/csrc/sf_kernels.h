@@ -158,10 +158,20 @@ void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b, bool chained);
 void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b);
 void launchSandMomentum(const LaunchCtx& c, const PassBuffers& b);
 void launchWaterMomentum(const LaunchCtx& c, const PassBuffers& b);
+// Scratch of the counting sort (sf_sort.cu); n: slots, a multiple of 256.
+struct CountScratch {
+    unsigned int* count;       // nCells rounded up to a multiple of 4
+    unsigned int* tileCount;   // kMaxCountTiles: slots per table tile
+    uint2* keyRank;            // n: key of each slot before the sort, place among the slots counted into its cell
+    unsigned int* arrived;     // n: slots of each cell, in arrival order
+    unsigned int* sortedKeys;  // n: keys after the sort
+    int tileShift;             // log2 of the cells per table tile (countTileShift)
+};
 // timeArgDev: when not null, the kernel reads timeArg from this device scalar
 // (graph-replayed steps whose render interval changes from call to call).
-void launchIntegrate(const LaunchCtx& c, const PassBuffers& b, float timeArg, int adaptive,
-                     const float* timeArgDev = nullptr);
+// cc: where the next sort's keys and counts go (keyRank null: nowhere).
+void launchIntegrate(const LaunchCtx& c, const PassBuffers& b, float timeArg, int adaptive, const float* timeArgDev,
+                     const CountScratch& cc);
 // Largest number of particles within the interaction reach of any particle
 // (itself included), atomically maxed into *maxCount; needs the cell table.
 void launchNeighborCountMax(const LaunchCtx& c, const float4* pos4, const unsigned int* cs, unsigned int* maxCount);
@@ -208,15 +218,6 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
                    const unsigned int* sortedKeys, int nCells, unsigned int* cellStart, float4* pairXY,
                    float2* pairZ);
 // ---- counting sort by cell (sf_sort.cu) ----
-// Scratch of the counting sort; n: slots, a multiple of 256.
-struct CountScratch {
-    unsigned int* count;       // nCells rounded up to a multiple of 4, zero between sorts
-    unsigned int* tileCount;   // kMaxCountTiles: slots per table tile
-    uint2* keyRank;            // n: key of each slot before the sort, place among the slots counted into its cell
-    unsigned int* arrived;     // n: slots of each cell, in arrival order
-    unsigned int* sortedKeys;  // n: keys after the sort
-    int tileShift;             // log2 of the cells per table tile (countTileShift)
-};
 constexpr int kMaxCountTiles = 1024;
 // Whether the counting sort is used: its table passes cost 12 B per cell, which
 // stays behind the radix sort's cost while there are at most 8 cells per slot
@@ -225,8 +226,11 @@ bool useCountingSort(int slots, int cells);
 // log2 of the cells per table tile: 1024 cells, doubled until at most
 // kMaxCountTiles tiles are left (every block of the scatter scans the tile sums).
 int countTileShift(int cells);
-// The sort stage in four launches: keys, cell table, stable order and gather of
-// the persistent arrays (with the slot-pair positions). Returns kernels launched.
+// Keys and counts of n slots at pos, into zero counts.
+void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc);
+// The sort stage from the keys and counts: cell table, stable order and gather
+// of the persistent arrays (with the slot-pair positions); the counts are zero
+// afterwards. Returns kernels launched.
 int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch& cc, const float4* pos,
                        const float4* vel, const float4* col, const float4* mat, const float2* amc, const int* pid,
                        float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,

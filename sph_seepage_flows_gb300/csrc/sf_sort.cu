@@ -20,6 +20,7 @@
 // digit passes is six launches.
 #include <algorithm>
 
+#include "sf_count.cuh"
 #include "sf_device.cuh"
 #include "sf_kernels.h"
 
@@ -407,9 +408,11 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 
 // ------------------------------------------------- counting sort by cell
 // The sort stage where the cell table is not much larger than the particle
-// arrays (useCountingSort): four launches instead of seven or eight.
+// arrays (useCountingSort): three or four launches instead of seven or eight.
 //   kCountKeys     the key of every slot and its place among the slots counted
-//                  into its cell (in arrival order)
+//                  into its cell (in arrival order); the integrator leaves the
+//                  same for the positions it writes, so this runs only after
+//                  positions came from elsewhere
 //   kCellScan      exclusive scan of the counts within each table tile
 //   kCountScatter  adds the slots of the tiles before (the cell table), and
 //                  lists the slots of each cell in arrival order
@@ -440,31 +443,8 @@ __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restr
                                                          const int* __restrict__ blockScene,
                                                          const float4* __restrict__ pos4, CountScratch cc,
                                                          unsigned int* errWord) {
-    __shared__ unsigned int parked, parkedBase;
-    if (threadIdx.x == 0) parked = 0u;
-    __syncthreads();
     const int slot = blockIdx.x * kSlotAlign + afterPrevious(threadIdx.x);
-    const SceneDev& S = scenes[blockScene[blockIdx.x]];
-    const float4 p = pos4[slot];
-    const bool live = p.w != 0.f;
-    const unsigned int key = slotKey(S, p, errWord);
-    // runs of equal keys in the warp: one atomic each
-    const unsigned int lane = threadIdx.x & 31u;
-    const unsigned int prev = __shfl_up_sync(0xffffffffu, key, 1);
-    const unsigned int heads = __ballot_sync(0xffffffffu, lane == 0u || prev != key);
-    unsigned int at = 0u;
-    if ((heads >> lane) & 1u) {
-        const unsigned int behind = lane == 31u ? 0u : heads >> (lane + 1u);
-        const unsigned int len = behind ? unsigned(__ffs(behind)) : 32u - lane;
-        // the parking cell may hold most slots of a handle: one atomic per block
-        at = live ? atomicAdd(&cc.count[key], len) : atomicAdd(&parked, len);
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) parkedBase = parked ? atomicAdd(&cc.count[S.cell_off + S.ncell], parked) : 0u;
-    __syncthreads();
-    const int leader = 31 - __clz(heads & (0xffffffffu >> (31u - lane)));
-    at = __shfl_sync(0xffffffffu, at, leader) + (lane - unsigned(leader));
-    cc.keyRank[slot] = make_uint2(key, live ? at : parkedBase + at);
+    countSlot(scenes[blockScene[blockIdx.x]], slot, pos4[slot], cc, errWord);
 }
 
 // Block b scans table tile b (2^tileShift cells, a multiple of kScanChunk) in
@@ -540,19 +520,22 @@ __global__ void __launch_bounds__(kSortThreads)
     pairZ[d] = p.z;
 }
 
+void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc) {
+    launchChained(c.stream, n / kSlotAlign, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc, c.errWord);
+}
+
 int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch& cc, const float4* pos,
                        const float4* vel, const float4* col, const float4* mat, const float2* amc, const int* pid,
                        float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
                        unsigned int* cellStart, float4* pairXY, float2* pairZ) {
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
-    launchChained(c.stream, blocks, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc, c.errWord);
     launchChained(c.stream, tiles, kSortThreads, 0, kCellScan, cc, nCells);
     launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
                   cellStart);
     launchChained(c.stream, blocks, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
                   pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
                   reinterpret_cast<float*>(pairZ));
-    return 4;
+    return 3;
 }
 
 }  // namespace sfg

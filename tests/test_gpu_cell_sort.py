@@ -94,3 +94,56 @@ def test_noalloc_sort_is_the_stable_key_order(cuda_lib, n, grid, crowd):
         assert np.array_equal(perm.cpu().numpy(), want)
         assert np.array_equal(table.cpu().numpy(), np.searchsorted(keys[want], np.arange(cells + 1)))
         assert int(room[0]) == int(room[-1]) == -7
+
+
+def test_counts_of_the_integrator_follow_what_happens_between_substeps(cuda_lib):
+    """The integrator counts the positions it writes for the next sort. Whatever comes between (fields set, particles
+    added, the order reset, stages by hand, an adjoint run), a run equals one whose every substep sorts from scratch."""
+    from sph_seepage_flows_gb300.capi import Simulation
+    dt = 1e-4
+
+    def scenario(sim, n, substep):
+        rng = np.random.default_rng(3)
+        substep(2)
+        pos = sim.field("pos", order="id")
+        sim.set_field("pos", (pos + rng.uniform(-1e-3, 1e-3, pos.shape)).astype(np.float32), order="id")
+        substep(3)
+        sim.set_field("vel", sim.field("vel") * np.float32(0.5))
+        substep(1)
+        sim.add_sph_particles(rng.uniform(0.1, 0.3, (40, 3)), [0, 0, 1], [0, 0, 0], float(sim.scenes[0].params.sph_mass), 0.01)
+        substep(2)
+        sim.stage("sort")
+        sim.stage("sort")
+        substep(1)
+        sim.stage("integrate", 1e-6)
+        sim.stage("integrate", 1e-6)
+        substep(1)
+        sim.adjoint(dt, 3, sim.field("pos", order="id"), checkpoint_every=2)
+        substep(2)
+        sim.reset_order()
+        substep(1)
+        sim.step(1.0 / 30.0)
+        sim.step(1.0 / 30.0)
+        return {k: sim.field(k) for k in ("id", "key", "pos", "vel", "density", "acc")}, sim.cell_table(0)
+
+    outs = []
+    for by_hand in (False, True):
+        sc = scenes.tiny(seed=5)
+        sim = Simulation(sc, capacity=sc.n + 100)
+
+        def substep(k):
+            if not by_hand:
+                sim.substeps_fixed(dt, k)
+                return
+            for _ in range(k):
+                # a write of the positions as they are: the next sort counts anew
+                sim.set_field("pos", sim.field("pos"))
+                for st in ("sort", "density", "avgflow", "voidage_adhesion", "sand_momentum", "water_momentum"):
+                    sim.stage(st, dt)
+                sim.stage("integrate", dt)
+
+        outs.append(scenario(sim, sc.n, substep))
+        assert sim.check_error() == 0
+    for k, v in outs[0][0].items():
+        assert np.array_equal(v, outs[1][0][k]), k
+    assert np.array_equal(outs[0][1], outs[1][1])
