@@ -322,8 +322,8 @@ sf_status sf_set_tuning(sf_handle* h, int32_t block_size, int32_t items_per_thre
 /* Threads per particle of the neighbour passes and of the adjoint pair
  * kernels (no reference counterpart): 1, 2, 4 or 8, or 0 for the automatic
  * choice (doubled up to 8 while fewer than 2048 threads per SM would run,
- * i.e. 1 for large scenes; the density and average-flow passes use 8 or 4
- * only while no more than 1152 threads per SM run, else 1). The density, average-flow and voidage/adhesion
+ * i.e. 1 for large scenes; the density pass uses 8 while no more than 1152
+ * threads per SM run, else 1, the average-flow pass 8, 2 or 1). The density, average-flow and voidage/adhesion
  * results and the neighbour lists are the same for every value; the
  * momentum sums are grouped differently (FP32 rounding only). Takes effect
  * at the next substep (captured graphs are dropped). */

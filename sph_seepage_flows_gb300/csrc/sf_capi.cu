@@ -355,7 +355,8 @@ struct sf_handle {
     void setLanes(int all) { lanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
     void setAutomaticLanes(int smCount) {
         setLanes(lanesForSlots(totalSlots, smCount));
-        listLanes[0] = listLanes[1] = listLanesForSlots(totalSlots, smCount);
+        listLanes[0] = densityLanesForSlots(totalSlots, smCount);
+        listLanes[1] = flowLanesForSlots(totalSlots, smCount);
     }
     // Drop the captured substep graphs (after a change of buffers or launch shapes).
     void dropGraphs() {

@@ -1287,10 +1287,11 @@ int lanesForSlots(long long totalSlots, int smCount) {
     return g;
 }
 
-int listLanesForSlots(long long totalSlots, int smCount) {
-    for (int g = 8; g > 2; g /= 2)
-        if (totalSlots * g <= 1152LL * smCount) return g;
-    return 1;
+int densityLanesForSlots(long long totalSlots, int smCount) { return totalSlots * 8 <= 1152LL * smCount ? 8 : 1; }
+
+int flowLanesForSlots(long long totalSlots, int smCount) {
+    if (totalSlots * 8 <= 1152LL * smCount) return 8;
+    return totalSlots <= 4096LL * smCount ? 2 : 1;
 }
 
 // Blocks of a tuned pass over all slots.

@@ -143,12 +143,16 @@ struct PassBuffers {
 // adjoint pair kernels for totalSlots slots on a GPU with smCount SMs:
 // doubled, up to 8, while fewer than 2048 threads per SM would run.
 int lanesForSlots(long long totalSlots, int smCount);
-// Threads per slot of the density and average-flow passes, whose one-lane
-// forms do the least work in all: 8 or 4 as long as no more than 1152 threads
-// per SM run, else 1. Density / average flow in us with 1, 4 and 8 lanes:
-// 20k column 64, 33, 33 / 25, 18, 14; 40k 45, 43, 49 / 18, 12, 13; 120k 65,
-// 92, 117 / 23, 29, 33; 252k 82, 223, 272 / 26, 47, 60 (2 lanes 226 / 47).
-int listLanesForSlots(long long totalSlots, int smCount);
+// Threads per slot of the density pass, whose one-lane form does a third of the
+// work in all: 8 while no more than 1152 threads per SM run, else 1. Density in
+// us with 1 and 8 lanes: 7k 54 and 21, 20k column 64 and 33, 40k 43 and 49 (4
+// lanes 43, but a substep 79 -> 77 with 1), 120k 63 and 117, 252k 85 and 272.
+int densityLanesForSlots(long long totalSlots, int smCount);
+// Threads per slot of the average-flow pass: 8 for the same scenes, 2 up to 4096
+// slots per SM, else 1. A substep in us with 1, 2, 4 and 8 lanes: 20k column 87,
+// 81, 76, 74; 120k 129.5, 126.4, 126.5, 129.4; 252k 190, 187, 189, 198; 791k
+// 547, 545, 560, 594.
+int flowLanesForSlots(long long totalSlots, int smCount);
 
 void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, const int* blabel,
                           const unsigned int* bcs);
