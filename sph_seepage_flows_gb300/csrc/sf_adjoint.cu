@@ -335,6 +335,53 @@ __device__ __forceinline__ void adhesionVjp(const SceneDev& S, float3 d, float s
     gsat = bezierDeriv(S.adhG, satJ) * m * g * du;
 }
 
+// The per-particle parts between two pair levels. Each uses only what its own
+// slot holds, so the pair kernel before it ends with it (in lane 0) instead of
+// a launch of its own, as does the density level with the scatter by id: of 11
+// launches a reverse substep keeps 8, each a few us long for a scene of 20k
+// particles (its gradient call 3.92 -> 3.83 ms, 12 calibrations 9.21 -> 8.99
+// ms, gradients bit for bit the same). kAdjFlowSelf stays a launch: as the end
+// of kAdjVoidPairs it changes how that kernel is compiled, and through the
+// steep ends of the adhesion spline gradients then moved by up to 1e-2.
+
+// A4a: sand: voidage = num / den -> (num-bar, den-bar); water: adhesion
+// cotangent total (F_adh-bar + avg-bar / v_s) and v_s-bar.
+__device__ __forceinline__ void voidSelf(const AdjBuffers& A, const PassBuffers& b, int slot, bool sand) {
+    if (sand) {
+        // voidage = num / den, with den and the quotient stored by the forward
+        const float den = b.dp[slot].x;
+        // quotient rule without squaring den (a small den would underflow)
+        const float eb = A.s[slot].z;
+        A.r[slot] = den != 0.f ? make_float4(eb / den, -(eb / den) * b.aux4[slot].w, 0.f, 0.f)
+                               : make_float4(0.f, 0.f, 0.f, 0.f);
+    } else {
+        const float vs = b.adh4[slot].w;  // stored by the forward
+        const float3 avgB = xyz(A.avgadh[slot]);
+        float3 tot = xyz(A.adh[slot]);
+        float vsb = 0.f;
+        if (vs != 0.f) {  // avg = F / v_s: d/dv_s = -avg / v_s
+            tot = tot + avgB / vs;
+            vsb = -dot3(avgB, xyz(b.avgadh4[slot])) / vs;
+        }
+        A.r[slot] = f4(tot, vsb);
+    }
+}
+
+// A6a: water: density cotangent including the pressure path.
+__device__ __forceinline__ void densitySelf(const SceneDev& S, const AdjBuffers& A, const PassBuffers& b, int slot) {
+    const float rho = b.vel4[slot].w;
+    float dp;
+    if (S.tait) {  // ComputeSFPressureByTait_CUDA
+        const float x = rho / S.rho0;
+        const float p = S.stiff * (powf(x, 7.f) - 1.f);
+        dp = S.stiff * 7.f * powf(x, 6.f) / S.rho0 * (p < 0.f ? S.neg_scale : 1.f);
+    } else {
+        dp = S.stiff;
+    }
+    const float4 s = A.s[slot];
+    A.r[slot] = make_float4(s.x + s.y * dp, 0.f, 0.f, 0.f);
+}
+
 // ------------------------------------------------------------- kernels
 __global__ void kAdjSeed(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene,
                          const float4* __restrict__ pos4, const int* __restrict__ pid,
@@ -732,39 +779,13 @@ __global__ void __launch_bounds__(kSlotAlign, 3) kAdjSandPairs(const SceneDev* _
         if (part == 0) {
             add3(A.x[slot], gx);
             add3(A.v[slot], gv);
+            voidSelf(A, b, slot, pk4.w < 0.f);
         }
     }
     const float2 t = blockSum2(gTan, gCap);
     if (threadIdx.x == 0) {
         paramPartial[3 * blockIdx.x] += t.x;
         paramPartial[3 * blockIdx.x + 1] += t.y;
-    }
-}
-
-// A4a: sand: voidage = num / den -> (num-bar, den-bar); water: adhesion
-// cotangent total (F_adh-bar + avg-bar / v_s) and v_s-bar.
-__global__ void __launch_bounds__(kSlotAlign) kAdjVoidSelf(AdjBuffers A, PassBuffers b) {
-    const int slot = blockIdx.x * blockDim.x + threadIdx.x;
-    const float4 pk4 = b.pos4[slot];
-    if (pk4.w == 0.f) return;
-    const float3 xk = xyz(pk4);
-    if (pk4.w < 0.f) {
-        // voidage = num / den, with den and the quotient stored by the forward
-        const float den = b.dp[slot].x;
-        // quotient rule without squaring den (a small den would underflow)
-        const float eb = A.s[slot].z;
-        A.r[slot] = den != 0.f ? make_float4(eb / den, -(eb / den) * b.aux4[slot].w, 0.f, 0.f)
-                               : make_float4(0.f, 0.f, 0.f, 0.f);
-    } else {
-        const float vs = b.adh4[slot].w;  // stored by the forward
-        const float3 avgB = xyz(A.avgadh[slot]);
-        float3 tot = xyz(A.adh[slot]);
-        float vsb = 0.f;
-        if (vs != 0.f) {  // avg = F / v_s: d/dv_s = -avg / v_s
-            tot = tot + avgB / vs;
-            vsb = -dot3(avgB, xyz(b.avgadh4[slot])) / vs;
-        }
-        A.r[slot] = f4(tot, vsb);
     }
 }
 
@@ -929,25 +950,7 @@ __global__ void __launch_bounds__(kSlotAlign, 3) kAdjFlowPairs(const SceneDev* _
     if (part != 0) return;
     add3(A.x[slot], gx);
     add3(A.v[slot], gv);
-}
-
-// A6a: water: density cotangent including the pressure path.
-__global__ void kAdjDensitySelf(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene,
-                                AdjBuffers A, PassBuffers b) {
-    SF_ADJ_PROLOGUE
-    const float4 pk4 = b.pos4[slot];
-    if (!(pk4.w > 0.f)) return;
-    const float rho = b.vel4[slot].w;
-    float dp;
-    if (S.tait) {  // ComputeSFPressureByTait_CUDA
-        const float x = rho / S.rho0;
-        const float p = S.stiff * (powf(x, 7.f) - 1.f);
-        dp = S.stiff * 7.f * powf(x, 6.f) / S.rho0 * (p < 0.f ? S.neg_scale : 1.f);
-    } else {
-        dp = S.stiff;
-    }
-    const float4 s = A.s[slot];
-    A.r[slot] = make_float4(s.x + s.y * dp, 0.f, 0.f, 0.f);
+    if (pk4.w > 0.f) densitySelf(S, A, b, slot);
 }
 
 // A6b: density pair terms: own m_j W(x_k - x_j) and water j's m_k W(x_j - x_k),
@@ -955,10 +958,22 @@ __global__ void kAdjDensitySelf(const SceneDev* __restrict__ scenes, const int* 
 template <int G>
 __global__ void __launch_bounds__(kSlotAlign, 3) kAdjDensityPairs(const SceneDev* __restrict__ scenes,
                                                                const int* __restrict__ blockScene, AdjBuffers A,
-                                                               PassBuffers b) {
+                                                               PassBuffers b, const int* __restrict__ pid) {
     SF_ADJ_PROLOGUE_G
     const float4 pk4 = b.pos4[slot];
-    if (!(pk4.w > 0.f)) return;
+    if (pk4.w == 0.f) return;
+    // cotangents of the substep's input position and velocity, by id
+    auto finish = [&](float3 gx) {
+        const int id = S.slot_off + pid[slot];
+        float4 x = A.x[slot];
+        add3(x, gx);
+        A.adjX[id] = x;
+        A.adjV[id] = A.v[slot];
+    };
+    if (pk4.w < 0.f) {
+        if (part == 0) finish(mk3(0.f, 0.f, 0.f));
+        return;
+    }
     const float3 xk = xyz(pk4);
     const float mk = pk4.w;
     const float rk = A.r[slot].x;
@@ -979,17 +994,7 @@ __global__ void __launch_bounds__(kSlotAlign, 3) kAdjDensityPairs(const SceneDev
         gx += (rk * S.rho0 * fabsf(bj.w)) * poly6Grad(S, xk - xyz(bj));
     }
     gx = groupSum3<G>(gx);
-    if (part == 0) add3(A.x[slot], gx);
-}
-
-// Cotangents of the substep's input positions and velocities, by id.
-__global__ void kAdjFinish(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, AdjBuffers A,
-                           const float4* __restrict__ pos4, const int* __restrict__ pid) {
-    SF_ADJ_PROLOGUE
-    if (pos4[slot].w == 0.f) return;
-    const int id = S.slot_off + pid[slot];
-    A.adjX[id] = A.x[slot];
-    A.adjV[id] = A.v[slot];
+    if (part == 0) finish(gx);
 }
 
 __global__ void kAdjStore(PassBuffers b, const int* __restrict__ pid, AdjSlab s) {
@@ -1015,7 +1020,8 @@ void launchAdjSeed(const LaunchCtx& c, const float4* pos4, const int* pid, const
 }
 
 template <int G>
-void launchAdjPairs(const LaunchCtx& c, const AdjBuffers& A, const PassBuffers& b, float* paramPartial, int level) {
+void launchAdjPairs(const LaunchCtx& c, const AdjBuffers& A, const PassBuffers& b, const int* pid, float* paramPartial,
+                    int level) {
     const dim3 g(c.slotBlocks * G), t(kSlotAlign);
     const cudaStream_t s = c.stream;
     switch (level) {
@@ -1023,17 +1029,17 @@ void launchAdjPairs(const LaunchCtx& c, const AdjBuffers& A, const PassBuffers& 
     case 1: kAdjSandPairs<G><<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b, paramPartial); break;
     case 2: kAdjVoidPairs<G><<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b); break;
     case 3: kAdjFlowPairs<G><<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b); break;
-    default: kAdjDensityPairs<G><<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b); break;
+    default: kAdjDensityPairs<G><<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b, pid); break;
     }
 }
 
-void launchPairs(const LaunchCtx& c, const AdjBuffers& A, const PassBuffers& b, float* paramPartial, int lanes,
-                 int level) {
+void launchPairs(const LaunchCtx& c, const AdjBuffers& A, const PassBuffers& b, const int* pid, float* paramPartial,
+                 int lanes, int level) {
     switch (lanes) {
-    case 2: launchAdjPairs<2>(c, A, b, paramPartial, level); break;
-    case 4: launchAdjPairs<4>(c, A, b, paramPartial, level); break;
-    case 8: launchAdjPairs<8>(c, A, b, paramPartial, level); break;
-    default: launchAdjPairs<1>(c, A, b, paramPartial, level); break;
+    case 2: launchAdjPairs<2>(c, A, b, pid, paramPartial, level); break;
+    case 4: launchAdjPairs<4>(c, A, b, pid, paramPartial, level); break;
+    case 8: launchAdjPairs<8>(c, A, b, pid, paramPartial, level); break;
+    default: launchAdjPairs<1>(c, A, b, pid, paramPartial, level); break;
     }
 }
 
@@ -1042,17 +1048,14 @@ int launchAdjSubstep(const LaunchCtx& c, const AdjBuffers& A, const PassBuffers&
     const dim3 g(c.slotBlocks), t(kSlotAlign);
     const cudaStream_t s = c.stream;
     kAdjIntegrate<<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b, pid, dt);
-    launchPairs(c, A, b, paramPartial, lanes, 0);
+    launchPairs(c, A, b, pid, paramPartial, lanes, 0);
     kAdjSandSelf<<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b, paramPartial, lanes);
-    launchPairs(c, A, b, paramPartial, lanes, 1);
-    kAdjVoidSelf<<<g, t, 0, s>>>(A, b);
-    launchPairs(c, A, b, paramPartial, lanes, 2);
+    launchPairs(c, A, b, pid, paramPartial, lanes, 1);
+    launchPairs(c, A, b, pid, paramPartial, lanes, 2);
     kAdjFlowSelf<<<g, t, 0, s>>>(A, b);
-    launchPairs(c, A, b, paramPartial, lanes, 3);
-    kAdjDensitySelf<<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b);
-    launchPairs(c, A, b, paramPartial, lanes, 4);
-    kAdjFinish<<<g, t, 0, s>>>(c.scenes, c.blockScene, A, b.pos4, pid);
-    return 11;
+    launchPairs(c, A, b, pid, paramPartial, lanes, 3);
+    launchPairs(c, A, b, pid, paramPartial, lanes, 4);
+    return 8;
 }
 
 }  // namespace sfg
