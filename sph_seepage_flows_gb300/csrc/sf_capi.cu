@@ -251,7 +251,8 @@ struct sf_handle {
     // blocks even out the lengths of their walks (1M embankment with 128 / 256:
     // density 256 / 275 us, average flow 82 / 94, water momentum 115 / 119)
     int block[kTunedPasses] = {128, 128, 128, 128, 128, kSlotAlign};
-    int lanes = 1;  // threads per slot of the momentum passes and the adjoint pair kernels
+    int lanes = 1;     // threads per slot of the momentum passes
+    int adjLanes = 1;  // and of the adjoint pair kernels
     // threads per slot of the passes before them, whose results do not depend on it
     int listLanes[3] = {1, 1, 1};  // density, average flow, voidage / adhesion
     int densityStaged = 0;  // the one-lane density pass stages its candidates in shared memory (tuned)
@@ -282,7 +283,7 @@ struct sf_handle {
         err = std::string(what) + ": " + cudaGetErrorString(e);
         return SF_ERR_CUDA;
     }
-    int adjBlocks() const { return slotBlocks * lanes; }
+    int adjBlocks() const { return slotBlocks * adjLanes; }
     static constexpr int kMaxLanes = 8;
     LaunchCtx ctx() const {
         LaunchCtx c;
@@ -352,11 +353,12 @@ struct sf_handle {
     CountScratch countScratch() const {
         return CountScratch{cellCount, tileCount, keyRank, sc.vals, keys, countTileShift(totalCells)};
     }
-    void setLanes(int all) { lanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
+    void setLanes(int all) { lanes = adjLanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
     void setAutomaticLanes(int smCount) {
         setLanes(lanesForSlots(totalSlots, smCount));
         listLanes[0] = densityLanesForSlots(totalSlots, smCount);
         listLanes[1] = flowLanesForSlots(totalSlots, smCount);
+        adjLanes = adjointLanesForSlots(totalSlots, smCount);
     }
     // Drop the captured substep graphs (after a change of buffers or launch shapes).
     void dropGraphs() {
@@ -1925,6 +1927,7 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
     // the two momentum passes share the one of their smaller sum.
     constexpr int kFirstMomentum = kPassSand;
     float bestMomentum = 0.f, bestList[kFirstMomentum] = {};
+    const int adjLanes = h->adjLanes;  // not timed here: stays as it is
     int bestLanes = h->lanes, bestListLanes[kFirstMomentum], bestBlock[kTunedPasses - 1], bestStaged = 0;
     for (int p = 0; p < kTunedPasses - 1; ++p) bestBlock[p] = h->block[p];
     for (int p = 0; p < kFirstMomentum; ++p) bestListLanes[p] = h->listLanes[p];
@@ -1968,6 +1971,7 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
         }
     }
     h->lanes = bestLanes;
+    h->adjLanes = adjLanes;
     for (int p = 0; p < kFirstMomentum; ++p) h->listLanes[p] = bestListLanes[p];
     h->densityStaged = bestStaged;
     for (int p = 0; p < kTunedPasses - 1; ++p) h->block[p] = bestBlock[p];
@@ -2196,7 +2200,7 @@ sf_status runAdjSubstepGraphed(sf_handle* h, float dt, int64_t t) {
         sf_status st = h->cuda(cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal), "begin capture");
         if (st) return st;
         const AdjSlab sl = slabAt(h, h->slab + size_t(t) * slabStride(h));
-        g.nodes = launchAdjSubstep(h->ctx(), h->adj, slabBuffers(h, sl), sl.pid, dt, h->adjParam, h->lanes);
+        g.nodes = launchAdjSubstep(h->ctx(), h->adj, slabBuffers(h, sl), sl.pid, dt, h->adjParam, h->adjLanes);
         const cudaError_t le = cudaGetLastError();
         const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
         if (h->cuda(le, "adjoint launch") || h->cuda(ce, "end capture")) {
@@ -2343,7 +2347,8 @@ sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t che
             l += lossPart[size_t(b)].x;
             ns += lossPart[size_t(b)].y;
         }
-        for (int b = S.slot_off / kSlotAlign * h->lanes; b < (S.slot_off + S.slot_cap) / kSlotAlign * h->lanes; ++b)
+        for (int b = S.slot_off / kSlotAlign * h->adjLanes; b < (S.slot_off + S.slot_cap) / kSlotAlign * h->adjLanes;
+             ++b)
             for (int k = 0; k < 3; ++k) g[k] += paramPart[3 * size_t(b) + size_t(k)];
         const double inv = ns > 0.0 ? 1.0 / ns : 0.0;
         loss_out[s] = float(l * inv);

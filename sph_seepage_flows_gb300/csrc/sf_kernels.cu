@@ -1287,6 +1287,11 @@ int lanesForSlots(long long totalSlots, int smCount) {
     return g;
 }
 
+int adjointLanesForSlots(long long totalSlots, int smCount) {
+    const int g = lanesForSlots(totalSlots, smCount);
+    return g == 1 && totalSlots <= 4096LL * smCount ? 2 : g;
+}
+
 int densityLanesForSlots(long long totalSlots, int smCount) { return totalSlots * 8 <= 1152LL * smCount ? 8 : 1; }
 
 int flowLanesForSlots(long long totalSlots, int smCount) {

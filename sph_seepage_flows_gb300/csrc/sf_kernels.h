@@ -139,10 +139,16 @@ struct PassBuffers {
     float4* grec4;
 };
 
-// Threads per slot of the voidage / adhesion and momentum passes and of the
-// adjoint pair kernels for totalSlots slots on a GPU with smCount SMs:
-// doubled, up to 8, while fewer than 2048 threads per SM would run.
+// Threads per slot of the voidage / adhesion and momentum passes for
+// totalSlots slots on a GPU with smCount SMs: doubled, up to 8, while fewer
+// than 2048 threads per SM would run.
 int lanesForSlots(long long totalSlots, int smCount);
+// The same for the adjoint pair kernels, but 2 up to 4096 threads per SM: with
+// 24 warps per SM at most, one lane per particle leaves their last wave short
+// until there are more. A reverse substep in us with 1, 2, 4 and 8 lanes: 20k
+// 136 89 65 55, 40k 158 101 76 75, 80k 182 125 109 116, 160k 193 158 158 200,
+// 320k 285 255 286 394, 640k 439 446 575 856, 1M 633 689 936 1401.
+int adjointLanesForSlots(long long totalSlots, int smCount);
 // Threads per slot of the density pass, whose one-lane form does a third of the
 // work in all: 8 while no more than 1152 threads per SM run, else 1. Density in
 // us with 1 and 8 lanes: 7k 54 and 21, 20k column 64 and 33, 40k 43 and 49 (4
