@@ -791,7 +791,7 @@ __global__ void __launch_bounds__(kSlotAlign, 3) kAdjSandPairs(const SceneDev* _
 
 // A4b: voidage / adhesion pair terms from both ends.
 template <int G>
-__global__ void __launch_bounds__(kSlotAlign, 3) kAdjVoidPairs(const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kSlotAlign, 4) kAdjVoidPairs(const SceneDev* __restrict__ scenes,
                                                             const int* __restrict__ blockScene, AdjBuffers A,
                                                             PassBuffers b) {
     SF_ADJ_PROLOGUE_G
@@ -893,7 +893,7 @@ __global__ void kAdjFlowSelf(AdjBuffers A, PassBuffers b) {
 
 // A5b: average flow / saturation / fluid voidage pair terms from both ends.
 template <int G>
-__global__ void __launch_bounds__(kSlotAlign, 3) kAdjFlowPairs(const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kSlotAlign, 4) kAdjFlowPairs(const SceneDev* __restrict__ scenes,
                                                             const int* __restrict__ blockScene, AdjBuffers A,
                                                             PassBuffers b) {
     SF_ADJ_PROLOGUE_G
