@@ -2291,6 +2291,26 @@ sf_status ensureAdjoint(sf_handle* h, size_t snapshots, size_t slabs) {
 
 }  // namespace
 
+namespace {
+
+// A scene's cotangents by id as the caller's packed gradients, scaled in
+// double. On the host this took a copy with a wait and a loop per scene and
+// array (@@).
+__global__ void kAdjOutput(int n, const float4* __restrict__ x, const float4* __restrict__ v, double scale,
+                           float* __restrict__ outX, float* __restrict__ outV) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    auto put = [&](float* out, float4 g) {
+        out[3 * size_t(i)] = float(double(g.x) * scale);
+        out[3 * size_t(i) + 1] = float(double(g.y) * scale);
+        out[3 * size_t(i) + 2] = float(double(g.z) * scale);
+    };
+    if (outX) put(outX, x[i]);
+    if (outV) put(outV, v[i]);
+}
+
+}  // namespace
+
 sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t checkpoint_every,
                          const float* target_pos, float* loss_out, float* grad_params_out, float* grad_pos0_out,
                          float* grad_vel0_out, float* ms_out) {
@@ -2367,7 +2387,6 @@ sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t che
     // per-scene reductions in block order, and the id-ordered gradients
     std::vector<float2> lossPart(size_t(h->slotBlocks));
     std::vector<float> paramPart(3 * size_t(h->adjBlocks()));
-    std::vector<float4> gx, gv;
     if (h->cuda(cudaMemcpyAsync(lossPart.data(), h->adjLoss, sizeof(float2) * lossPart.size(), cudaMemcpyDeviceToHost,
                                 h->stream),
                 "loss D2H") ||
@@ -2376,6 +2395,14 @@ sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t che
                 "parameter gradient D2H") ||
         h->cuda(cudaStreamSynchronize(h->stream), "adjoint sync"))
         return SF_ERR_CUDA;
+    // packed gradients: positions, then velocities
+    const size_t gradBytes = sizeof(float) * 3 * size_t(off);
+    float *gx = nullptr, *gv = nullptr;
+    if (off > 0 && (grad_pos0_out || grad_vel0_out)) {
+        if (ensureStage(h, 2 * gradBytes)) return SF_ERR_CUDA;
+        if (grad_pos0_out) gx = static_cast<float*>(h->stage);
+        if (grad_vel0_out) gv = static_cast<float*>(h->stage) + 3 * size_t(off);
+    }
     off = 0;
     for (int s = 0; s < h->nScenes; ++s) {
         const SceneDev& S = h->hScenes[s];
@@ -2394,24 +2421,21 @@ sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t che
         if (grad_params_out)
             for (int k = 0; k < 3; ++k) grad_params_out[3 * s + k] = float(g[k] * ginv);
         const int64_t n = h->n[s];
-        for (int which = 0; which < 2; ++which) {
-            float* out = which ? grad_vel0_out : grad_pos0_out;
-            if (!out || n == 0) continue;
-            std::vector<float4>& buf = which ? gv : gx;
-            buf.resize(size_t(n));
-            if (h->cuda(cudaMemcpyAsync(buf.data(), (which ? h->adj.adjV : h->adj.adjX) + S.slot_off,
-                                        sizeof(float4) * size_t(n), cudaMemcpyDeviceToHost, h->stream),
-                        "gradient D2H") ||
-                h->cuda(cudaStreamSynchronize(h->stream), "gradient sync"))
-                return SF_ERR_CUDA;
-            for (int64_t i = 0; i < n; ++i) {
-                out[3 * (off + i)] = float(double(buf[size_t(i)].x) * ginv);
-                out[3 * (off + i) + 1] = float(double(buf[size_t(i)].y) * ginv);
-                out[3 * (off + i) + 2] = float(double(buf[size_t(i)].z) * ginv);
-            }
+        if (n > 0 && (gx || gv)) {
+            kAdjOutput<<<int((n + 255) / 256), 256, 0, h->stream>>>(int(n), h->adj.adjX + S.slot_off,
+                                                                    h->adj.adjV + S.slot_off, ginv,
+                                                                    gx ? gx + 3 * off : nullptr,
+                                                                    gv ? gv + 3 * off : nullptr);
+            h->launches += 1;
         }
         off += n;
     }
+    if ((gx && h->cuda(cudaMemcpyAsync(grad_pos0_out, gx, gradBytes, cudaMemcpyDeviceToHost, h->stream),
+                       "gradient D2H")) ||
+        (gv && h->cuda(cudaMemcpyAsync(grad_vel0_out, gv, gradBytes, cudaMemcpyDeviceToHost, h->stream),
+                       "gradient D2H")) ||
+        ((gx || gv) && h->cuda(cudaStreamSynchronize(h->stream), "gradient sync")))
+        return SF_ERR_CUDA;
     if (ms_out) {
         cudaEventElapsedTime(&ms_out[0], ev[0], ev[1]);
         cudaEventElapsedTime(&ms_out[1], ev[1], ev[2]);
