@@ -35,7 +35,10 @@
 // pairs 137 -> 95, voidage 101 -> 62, average flow 74 -> 46, density 43 -> 34;
 // with 48 registers the reverse sweep takes 6.1 ms of 10 substeps instead of
 // 5.2, with 128 5.4. The contacts keep a cursor with one body: their dual
-// numbers would not fit twice.
+// numbers would not fit twice. The sand pairs have 128 registers all the same:
+// at 80 the compiler contracts the contact terms in another way, and where the
+// friction angle's gradient is a small rest of large terms it then moved by up
+// to 1e-5 (12 calibrations take 8.70 ms instead of 8.66).
 //
 // Cotangents of positions and velocities between substeps are kept by
 // particle id (scene slot_off + id), so the sort needs no bookkeeping.
@@ -650,7 +653,7 @@ __global__ void __launch_bounds__(kSlotAlign) kAdjSandSelf(const SceneDev* __res
 //   f_i += [0 < e_j <= 1] (-m_i m_j p_j / max(eps, rho_i D_j)) G(x_i - x_j) + W vol_i avgadh_j,
 //   v_w,i += [0 < e_j <= 1] (m_j / D_j) W(x_i - x_j).
 template <int G>
-__global__ void __launch_bounds__(kSlotAlign, 3) kAdjSandPairs(const SceneDev* __restrict__ scenes,
+__global__ void __launch_bounds__(kSlotAlign, 2) kAdjSandPairs(const SceneDev* __restrict__ scenes,
                                                             const int* __restrict__ blockScene, AdjBuffers A,
                                                             PassBuffers b, float* __restrict__ paramPartial) {
     SF_ADJ_PROLOGUE_G
