@@ -358,6 +358,7 @@ __global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
     extern __shared__ uint2 sHits[];
     if (slot == S.slot_off) state[sid].amax_bits = 0u;
     const float4 pi4 = pos4[slot];
+    const unsigned live = __ballot_sync(0xffffffffu, pi4.w != 0.f);
     if (pi4.w == 0.f) return;
     const float3 pi = xyz(pi4);
     const int3 c = cellOf(S, pi);
@@ -522,12 +523,16 @@ __global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
             if (n < 32) hit &= (1u << n) - 1u;
             if (j0 < jBeg) hit &= ~1u;
             if (hit) {
+                if (nq == kHitChunks) drain();
                 mine[nq * stride] = make_uint2(j0, hit);
-                if (++nq == kHitChunks) drain();
+                ++nq;
             }
         }
+        // the warp drains together, before a column that could fill a lane's
+        // chunks: lanes draining one by one, each where it is full, take turns
+        const int chunks = nextBeg < nextEnd ? int(nextEnd - (nextBeg & ~1u) + 31u) >> 5 : 0;
+        if (__any_sync(live, m == 8 || nq + chunks > kHitChunks)) drain();
     }
-    drain();
     if (water)
         while (kb < bc && kb < kMaxBNbr) boundaryTerm();
     L.cnt[slot] = unsigned(min(cS, 0xFFFF)) | (unsigned(min(cW, 0xFFFF)) << 16);
