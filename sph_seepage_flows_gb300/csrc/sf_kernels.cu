@@ -1297,11 +1297,14 @@ int adjointLanesForSlots(long long totalSlots, int smCount) {
     return g == 1 && totalSlots <= 4096LL * smCount ? 2 : g;
 }
 
-int densityLanesForSlots(long long totalSlots, int smCount) { return totalSlots * 8 <= 1152LL * smCount ? 8 : 1; }
+int densityLanesForSlots(long long totalSlots, int smCount) {
+    if (totalSlots * 8 <= 1152LL * smCount) return 8;
+    return totalSlots * 4 <= 2304LL * smCount ? 4 : 1;
+}
 
 int flowLanesForSlots(long long totalSlots, int smCount) {
-    if (totalSlots * 8 <= 1152LL * smCount) return 8;
-    return totalSlots <= 4096LL * smCount ? 2 : 1;
+    const int g = densityLanesForSlots(totalSlots, smCount);
+    return g == 1 && totalSlots <= 4096LL * smCount ? 2 : g;
 }
 
 // Blocks of a tuned pass over all slots.

@@ -150,14 +150,21 @@ int lanesForSlots(long long totalSlots, int smCount);
 // 320k 285 255 286 394, 640k 439 446 575 856, 1M 633 689 936 1401.
 int adjointLanesForSlots(long long totalSlots, int smCount);
 // Threads per slot of the density pass, whose one-lane form does a third of the
-// work in all: 8 while no more than 1152 threads per SM run, else 1. Density in
-// us with 1 and 8 lanes: 7k 54 and 21, 20k column 64 and 33, 40k 43 and 49 (4
-// lanes 43, but a substep 79 -> 77 with 1), 120k 63 and 117, 252k 85 and 272.
+// work in all but is one long chain per particle: 8 while no more than 1152
+// threads per SM run, 4 while no more than 2304, else 1. Density in us with 1,
+// 4 and 8 lanes at the start / after 1200 substeps, when lists are longer:
+// columns of 30k 69 37 42 / 86 42 44, 60k 76 59 69 / 95 63 73, 80k 84 71 86 / 91
+// 77 92; flat 40k scene 48 43 48 / 93 53 61; embankments of 80k 65 64 80 / 92 70
+// 93, 120k 65 88 116 / 95 101 134.
 int densityLanesForSlots(long long totalSlots, int smCount);
-// Threads per slot of the average-flow pass: 8 for the same scenes, 2 up to 4096
-// slots per SM, else 1. A substep in us with 1, 2, 4 and 8 lanes: 20k column 87,
-// 81, 76, 74; 120k 129.5, 126.4, 126.5, 129.4; 252k 190, 187, 189, 198; 791k
-// 547, 545, 560, 594.
+// Threads per slot of the average-flow pass: as the density pass, but 2 for 1 up
+// to 4096 slots per SM. A substep in us with 1, 2, 4 and 8 lanes (/ after 1200
+// substeps): flat 40k scene 80.9 81.0 79.8 79.8 / 127.8 118.9 110.6 108.7 (8
+// adaptive substeps of another 40k state: 751 us with 2, 761 with 4, 794 with 8),
+// columns of 30k 95.0 88.4 83.2 81.9 and 60k 130.6 123.7 119.4 118.9, embankments
+// of 80k 124.7 121.7 121.5 122.3 / 159.4 151.3 150.2 150.7, 120k 134.6 131.5
+// 131.1 134.3 / 195.3 186.7 186.7 188.6, 300k 223.3 220.3 223.6 235.3; 791k
+// column 547 545 560 594.
 int flowLanesForSlots(long long totalSlots, int smCount);
 
 void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, const int* blabel,
