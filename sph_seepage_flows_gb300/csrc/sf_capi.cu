@@ -249,7 +249,7 @@ struct sf_handle {
     int64_t listGrowths = 0;
     // the neighbour passes run fastest with 64-128 threads per block: smaller
     // blocks even out the lengths of their walks (1M embankment with 128 / 256:
-    // density 256 / 275 us, average flow 82 / 94, water momentum 115 / 119)
+    // density 278 / 290 us, average flow 96 / 97, water momentum 102 / 109)
     int block[kTunedPasses] = {128, 128, 128, 128, 128, kSlotAlign};
     int lanes = 1;     // threads per slot of the momentum passes
     int adjLanes = 1;  // and of the adjoint pair kernels

@@ -334,14 +334,21 @@ constexpr int kAheadSlots = 600000;
 // candidate, whether or not its neighbour lanes read the same one; the float4
 // positions would be 16), the hit phase by issue. One pass per column that
 // appended from each chunk's mask and walked its lists again for contacts and
-// density: 312 / 295 / 111 us; this form 256 / 232 / 82. Of that, the density
-// terms in the hit phase with the boundary terms merged by the end slot of
+// density: 312 / 295 / 111 us; this form 256 / 232 / 82, and 278 / 245 / 82 now
+// that it also sums the sand's volume (26 us) and drains by warps. Of that, the
+// density terms in the hit phase with the boundary terms merged by the end slot of
 // their cell (instead of 27 cell-table steps over both lists) gave 36 us at
 // 791k, where every water particle is near the floor, and list addresses from
 // 32-bit strides 20 us everywhere. 12 waiting chunks: with 16 the larger shared
 // memory costs L1 (286 us at 1M), with 10 the disturbed column drains in the
 // middle of the walk (304 us). 48 registers: with 40 the spills cost 281 us,
 // with 64 the occupancy 268 us at 1M.
+//
+// Cells of more than ten particles have two chunks per column, more than the 12
+// that wait. Before a column that could fill any lane of the warp all its lanes
+// drain together: when each drained where it was full, they took turns, and the
+// 1M embankment took 587 us after 600 substeps instead of 359 (one pass per
+// column 388).
 //
 // kAhead: the hit phase loads the position of the next hit before it uses this
 // one's, with 64 registers (4 blocks of kSlotAlign threads per SM). That pays

@@ -425,8 +425,9 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 // per table tile beside the cells' (a few hundred addresses) made the 1M sort
 // 115 us with one per run, 66 with one per warp.
 // Sort stage against the radix sort: 1M embankment 77.5 -> 51.6 us (keys 10,
-// scan 3, scatter 8, reorder 27 of 190 MB through L2), 252k 40.9 -> 21, 64-scene
-// ensemble 86 -> 58; on small scenes its launches count: 40k 28.8 -> 16.5.
+// scan 3, scatter 8, reorder 27 of 190 MB through L2), and 42 behind an integrator
+// that counted; 252k 40.9 -> 13.6, 64-scene ensemble 86 -> 49; on small scenes
+// its launches count: 40k 28.8 -> 8.3.
 constexpr int kScanItems = 4;
 constexpr int kScanChunk = kSortThreads * kScanItems;
 constexpr int kScatterBlocks = 1216;  // 8 per SM: each scans the tile sums once
