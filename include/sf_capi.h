@@ -159,7 +159,7 @@ enum {
 
 /* Passes that sf_run_stage runs, in substep order. */
 enum {
-    SF_STAGE_SORT = 0,              /* hash, stable radix sort by cell, reorder, cell tables */
+    SF_STAGE_SORT = 0,              /* hash, stable sort by cell, reorder, cell tables */
     SF_STAGE_DENSITY = 1,           /* density + Tait/linear pressure */
     SF_STAGE_AVGFLOW = 2,           /* average flow, fluid voidage, saturation */
     SF_STAGE_VOIDAGE_ADHESION = 3,  /* sand voidage, water adhesion, wet-sand colour; also each
@@ -415,7 +415,7 @@ sf_status sf_set_adjoint_seed_scale(sf_handle* h, int32_t scene, float scale);
  *
  * The sort stage of a single-scene handle without a handle and without any
  * device allocation: cell keys of n positions (Pos2GridHash on `grid`), a
- * stable radix sort and the cell-start table. Scratch lives in a static
+ * stable sort and the cell-start table. Scratch lives in a static
  * device array sized for at most SF_NOALLOC_MAX_PARTICLES particles
  * (about 4.5 MB per device); larger n is rejected with SF_ERR_INVALID.
  *   pos_dev             in:  n * 3 floats, device memory
