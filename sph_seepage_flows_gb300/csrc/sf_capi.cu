@@ -216,8 +216,9 @@ struct sf_handle {
     unsigned int* sortedKeys = nullptr;  // points into keys/scratch after a sort
     SortScratch sc{};
     bool countingSort = false;  // by cell count and slot count (useCountingSort), else the radix sort
-    unsigned int *cellCount = nullptr, *tileCount = nullptr;
+    unsigned int *cellCount = nullptr, *tileCount = nullptr, *parkedBefore = nullptr;
     uint2* keyRank = nullptr;
+    unsigned char* parkedInWarp = nullptr;
     // the keys and counts of the counting sort: none (counts zero), of the
     // positions as they are (left by the integrator or the key kernel), or of
     // positions that have changed since
@@ -351,7 +352,8 @@ struct sf_handle {
         if (counts == kCountsReady) counts = kCountsStale;
     }
     CountScratch countScratch() const {
-        return CountScratch{cellCount, tileCount, keyRank, sc.vals, keys, countTileShift(totalCells)};
+        return CountScratch{cellCount, tileCount, keyRank, parkedInWarp, parkedBefore, sc.vals, keys,
+                            countTileShift(totalCells)};
     }
     void setLanes(int all) { lanes = adjLanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
     void setAutomaticLanes(int smCount) {
@@ -441,6 +443,8 @@ struct sf_handle {
         devFree(cellCount);
         devFree(keyRank);
         devFree(tileCount);
+        devFree(parkedInWarp);
+        devFree(parkedBefore);
         devFree(bpos);
         devFree(blabel);
         devFree(dScenes);
@@ -814,6 +818,8 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
         SF_ALLOC(h->cellCount, sizeof(unsigned) * (size_t(h->totalCells) + 4));
         SF_ALLOC(h->tileCount, sizeof(unsigned) * kMaxCountTiles);
         SF_ALLOC(h->keyRank, sizeof(uint2) * M);
+        SF_ALLOC(h->parkedInWarp, M / 32);
+        SF_ALLOC(h->parkedBefore, sizeof(unsigned) * M / kSlotAlign);
     } else {
         SF_ALLOC(h->sc.keysAlt, sizeof(unsigned) * M);
         SF_ALLOC(h->sc.valsAlt, sizeof(unsigned) * M);

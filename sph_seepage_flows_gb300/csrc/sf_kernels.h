@@ -180,6 +180,8 @@ struct CountScratch {
     unsigned int* count;       // nCells rounded up to a multiple of 4
     unsigned int* tileCount;   // kMaxCountTiles: slots per table tile
     uint2* keyRank;            // n: key of each slot before the sort, place among the slots counted into its cell
+    unsigned char* parkedInWarp;  // n / 32: parked slots of each 32
+    unsigned int* parkedBefore;   // n / 256: parked slots before each block of 256
     unsigned int* arrived;     // n: slots of each cell, in arrival order
     unsigned int* sortedKeys;  // n: keys after the sort
     int tileShift;             // log2 of the cells per table tile (countTileShift)

@@ -413,9 +413,11 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 //                  into its cell (in arrival order); the integrator leaves the
 //                  same for the positions it writes, so this runs only after
 //                  positions came from elsewhere
-//   kCellScan      exclusive scan of the counts within each table tile
+//   kCellScan      exclusive scan of the counts within each table tile, and of
+//                  the parked slots over the blocks of slots
 //   kCountScatter  adds the slots of the tiles before (the cell table), and
-//                  lists the slots of each cell in arrival order
+//                  lists the slots of each cell in arrival order (the parked
+//                  slots in slot order)
 //   kCellReorder   the place of each slot within its cell by slot number (the
 //                  stable order), the gather of the persistent arrays, and the
 //                  counts cleared for the next sort
@@ -448,11 +450,33 @@ __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restr
     countSlot(scenes[blockScene[blockIdx.x]], slot, pos4[slot], cc, errWord);
 }
 
-// Block b scans table tile b (2^tileShift cells, a multiple of kScanChunk) in
-// place and writes its sum.
-__global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int nCells) {
+// Exclusive prefix of the parked slots over the blocks of kSlotAlign slots, by
+// one block of threads, 4096 blocks a turn (a million slots).
+__device__ __forceinline__ void scanParked(const CountScratch& cc, int blocks) {
+    constexpr int kItems = 16;
     unsigned int carry = 0u, total;
-    const int tileBeg = afterPrevious(int(blockIdx.x)) << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
+    for (int base = 0; base < blocks; base += kSortThreads * kItems) {
+        const int first = base + int(threadIdx.x) * kItems;
+        unsigned int v[kItems], sum = 0u;
+#pragma unroll
+        for (int u = 0; u < kItems; ++u) sum += v[u] = first + u < blocks ? parkedInWarps(cc, first + u, 8) : 0u;
+        unsigned int a = carry + blockScan(sum, total);
+#pragma unroll
+        for (int u = 0; u < kItems; ++u) {
+            if (first + u < blocks) cc.parkedBefore[first + u] = a;
+            a += v[u];
+        }
+        carry += total;
+    }
+}
+
+// Block b scans table tile b (2^tileShift cells, a multiple of kScanChunk) in
+// place and writes its sum; the block behind the tiles scans the parked slots.
+__global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int n, int nCells) {
+    unsigned int carry = 0u, total;
+    const int tile = afterPrevious(int(blockIdx.x));
+    if (tile == int(gridDim.x) - 1) return scanParked(cc, n / kSlotAlign);
+    const int tileBeg = tile << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
     for (int base = tileBeg; base < tileEnd; base += kScanChunk) {
         const int c = base + int(threadIdx.x) * kScanItems;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -465,7 +489,9 @@ __global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int n
     if (threadIdx.x == 0) cc.tileCount[blockIdx.x] = carry;
 }
 
-__global__ void __launch_bounds__(kSortThreads) kCountScatter(CountScratch cc, int n, int nCells, int tiles,
+__global__ void __launch_bounds__(kSortThreads) kCountScatter(const SceneDev* __restrict__ scenes,
+                                                              const int* __restrict__ blockScene, CountScratch cc,
+                                                              int n, int nCells, int tiles,
                                                               unsigned int* __restrict__ cs) {
     // every block scans the (at most kMaxCountTiles) tile sums
     __shared__ unsigned int before[kMaxCountTiles];
@@ -480,7 +506,8 @@ __global__ void __launch_bounds__(kSortThreads) kCountScatter(CountScratch cc, i
     __syncthreads();
     const int first = blockIdx.x * kSortThreads + tid, threads = gridDim.x * kSortThreads;
     for (int i = first; i < n; i += threads) {
-        const uint2 kr = cc.keyRank[i];
+        uint2 kr = cc.keyRank[i];
+        if (kr.y & kParkedBit) kr.y = parkedPlace(cc, scenes[blockScene[i / kSlotAlign]], i, kr.y);
         cc.arrived[cc.count[kr.x] + before[kr.x >> cc.tileShift] + kr.y] = unsigned(i);
     }
     for (int c = first; c < nCells; c += threads) cs[c] = cc.count[c] + before[c >> cc.tileShift];
@@ -503,7 +530,7 @@ __global__ void __launch_bounds__(kSortThreads)
     const int id = pid[o];
     const unsigned int key = cc.keyRank[o].x;
     unsigned int d = unsigned(i);
-    if (p.w != 0.f) {  // parking slots are all alike and keep the place they have
+    if (p.w != 0.f) {  // the parked slots are listed in slot order
         const unsigned int beg = cs[key], end = cs[key + 1];
         d = beg;
         for (unsigned int q = beg; q < end; ++q) d += cc.arrived[q] < o ? 1u : 0u;
@@ -530,9 +557,9 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
                        float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
                        unsigned int* cellStart, float4* pairXY, float2* pairZ) {
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
-    launchChained(c.stream, tiles, kSortThreads, 0, kCellScan, cc, nCells);
-    launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
-                  cellStart);
+    launchChained(c.stream, tiles + 1, kSortThreads, 0, kCellScan, cc, n, nCells);
+    launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, c.scenes, c.blockScene,
+                  cc, n, nCells, tiles, cellStart);
     launchChained(c.stream, blocks, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
                   pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
                   reinterpret_cast<float*>(pairZ));
