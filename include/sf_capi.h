@@ -426,14 +426,14 @@ sf_status sf_set_adjoint_seed_scale(sf_handle* h, int32_t scene, float scale);
  *   stream              the CUDA stream to use (NULL = the legacy default stream)
  * Every call waits for its stream before returning, and returns
  * SF_ERR_DEVICE when a position is not finite (its kernels report that
- * through pinned host memory); the output buffers then hold unspecified
- * values. The first call on a device looks up the scratch address
- * (cudaGetSymbolAddress), which may load the module, and takes the pinned
- * words: make the first call before any stream capture. The lookup is
- * repeated when the cached address no longer belongs to the device (after
- * cudaDeviceReset). Calls that overlap on the GPU (two streams or host
- * threads) share the scratch and race: serialise them. Errors are reported
- * by sf_last_error_string(NULL). */
+ * through a page of registered host memory); the output buffers then hold
+ * unspecified values. The first call on a device looks up the scratch
+ * address (cudaGetSymbolAddress), which may load the module, and takes and
+ * registers that host page, which is kept: make the first call before any
+ * stream capture. The lookup is repeated after the device's context was
+ * reset (cudaDeviceReset), which the page's lost registration tells. Calls
+ * that overlap on the GPU (two streams or host threads) share the scratch and
+ * race: serialise them. Errors are reported by sf_last_error_string(NULL). */
 #define SF_NOALLOC_MAX_PARTICLES 262144
 sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const float* pos_dev, int64_t n,
                                int32_t* perm_out_dev, int32_t* cell_start_out_dev, void* stream);

@@ -12,16 +12,16 @@
 // The call is a chain of short launches and a wait: 200k particles 84 -> 33 us.
 //
 // The scratch (g_noallocScratch) holds the keys and the arrays of either form.
-// Its device address is looked up once per device with cudaGetSymbolAddress
-// (the first call on a device does it, and the first call after that device's
-// context was reset, which is detected by asking the runtime whether the
-// cached address is still a device address); the same lookup takes one page
-// of pinned host memory for the words that a call reports through, which its
-// kernels write directly. Every scratch word is written before it is read.
+// A call reports through one page of registered host memory, which its kernels
+// write directly. Both are looked up once per device (scratchOf). Every scratch
+// word is written before it is read.
 // Calls that overlap on the GPU share the scratch and race.
 #include "../../include/sf_capi.h"
 #include "sf_device.cuh"
 #include "sf_kernels.h"
+
+#include <stdlib.h>
+#include <unistd.h>
 
 #include <mutex>
 #include <string>
@@ -42,7 +42,7 @@ constexpr int kMaxDevices = 64;
 
 __device__ __align__(256) unsigned int g_noallocScratch[kWords];
 
-// What a call's kernels report, in pinned host memory: cleared by the host
+// What a call's kernels report, in registered host memory: cleared by the host
 // before the launches, set to 1 by any thread that finds the condition.
 struct Report {
     unsigned int nonFinite, crowded;
@@ -151,50 +151,61 @@ sf_status failWith(sf_status st, const std::string& msg) {
     return st;
 }
 
-// Is p still a device address of `device`? After cudaDeviceReset (or any
-// teardown of the primary context) the module is loaded again and a cached
-// address may be stale; the runtime then no longer knows it as device memory.
-bool stillDeviceAddress(const void* p, int device) {
+// What the runtime knows about p on the current device: its type and device.
+cudaPointerAttributes attributesOf(const void* p) {
     cudaPointerAttributes a{};
-    const cudaError_t e = cudaPointerGetAttributes(&a, p);
-    if (e != cudaSuccess) {
+    a.type = cudaMemoryTypeUnregistered;
+    if (p && cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();  // not sticky: clear it so later checks see only their own errors
-        return false;
+        a.type = cudaMemoryTypeUnregistered;
     }
-    return a.type == cudaMemoryTypeDevice && a.device == device;
+    return a;
 }
 
-// Device address of the scratch on the current device, and the device's report
-// words: looked up on the first call on a device and again whenever the cached
-// address went stale (a reset of the context frees the pinned memory as well).
-unsigned int* scratchAddress(int device, Report*& report, std::string& why) {
+// What a call uses of a device.
+struct Scratch {
+    unsigned int* words = nullptr;    // g_noallocScratch
+    Report* report = nullptr;         // host address of the report page
+    Report* reportOnDevice = nullptr;
+};
+
+// The scratch of the current device: looked up on the first call on a device
+// and again after its context was reset (cudaDeviceReset or any teardown of
+// the primary context), when the module is loaded again and cached addresses
+// may be stale. A reset frees pinned memory, so the report page is not the
+// runtime's: it is a page of this library's own that stays allocated, and is
+// registered with the context. The host may therefore always write it, no
+// other allocation can be found at its address, and that the runtime no longer
+// knows it as registered is what tells of a reset. (The device address alone
+// does not: by the next call the module, or another allocation, may have taken
+// the same place.)
+bool scratchOf(int device, Scratch& out, std::string& why) {
     static std::mutex mu;
-    static unsigned int* addr[kMaxDevices] = {};
-    static Report* reports[kMaxDevices] = {};
+    static Scratch known[kMaxDevices];
     std::lock_guard<std::mutex> lock(mu);
-    if (device < 0 || device >= kMaxDevices) {
-        why = "device index out of range";
-        return nullptr;
+    if (device < 0 || device >= kMaxDevices) return why = "device index out of range", false;
+    Scratch& k = known[device];
+    const cudaPointerAttributes w = attributesOf(k.words);
+    if (attributesOf(k.report).type != cudaMemoryTypeHost || w.type != cudaMemoryTypeDevice || w.device != device) {
+        const size_t page = size_t(sysconf(_SC_PAGESIZE));
+        void* p = k.report;
+        if (!p && posix_memalign(&p, page, page) != 0) return why = "no host memory for the report page", false;
+        k.report = static_cast<Report*>(p);
+        k.words = nullptr;
+        cudaError_t e = cudaSuccess;
+        if (attributesOf(p).type != cudaMemoryTypeHost &&
+            (e = cudaHostRegister(p, page, cudaHostRegisterMapped)) != cudaSuccess)
+            return why = std::string("cudaHostRegister: ") + cudaGetErrorString(e), false;
+        void *d = nullptr, *s = nullptr;
+        if ((e = cudaHostGetDevicePointer(&d, p, 0)) != cudaSuccess)
+            return why = std::string("cudaHostGetDevicePointer: ") + cudaGetErrorString(e), false;
+        if ((e = cudaGetSymbolAddress(&s, g_noallocScratch)) != cudaSuccess)
+            return why = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e), false;
+        k.reportOnDevice = static_cast<Report*>(d);
+        k.words = static_cast<unsigned int*>(s);
     }
-    if (addr[device] && !stillDeviceAddress(addr[device], device)) addr[device] = nullptr;
-    if (!addr[device]) {
-        void* p = nullptr;
-        const cudaError_t e = cudaGetSymbolAddress(&p, g_noallocScratch);
-        if (e != cudaSuccess) {
-            why = std::string("cudaGetSymbolAddress: ") + cudaGetErrorString(e);
-            return nullptr;
-        }
-        void* r = nullptr;
-        const cudaError_t he = cudaHostAlloc(&r, sizeof(Report), cudaHostAllocPortable | cudaHostAllocMapped);
-        if (he != cudaSuccess) {
-            why = std::string("cudaHostAlloc: ") + cudaGetErrorString(he);
-            return nullptr;
-        }
-        reports[device] = static_cast<Report*>(r);
-        addr[device] = static_cast<unsigned int*>(p);
-    }
-    report = reports[device];
-    return addr[device];
+    out = k;
+    return true;
 }
 
 }  // namespace
@@ -217,9 +228,10 @@ extern "C" sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const 
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return failWith(SF_ERR_CUDA, std::string("cudaGetDevice: ") + cudaGetErrorString(e));
     std::string why;
-    Report* report = nullptr;
-    unsigned int* base = scratchAddress(device, report, why);
-    if (!base) return failWith(SF_ERR_CUDA, "sf_cell_sort_noalloc: " + why);
+    Scratch scratch;
+    if (!scratchOf(device, scratch, why)) return failWith(SF_ERR_CUDA, "sf_cell_sort_noalloc: " + why);
+    unsigned int* base = scratch.words;
+    volatile Report* report = scratch.report;
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int ncell = int(cells);
     if (n == 0) {
@@ -246,11 +258,12 @@ extern "C" sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const 
         const int shift = countTileShift(ncell), tiles = ((ncell - 1) >> shift) + 1;
         if ((e = cudaMemsetAsync(table, 0, sizeof(int32_t) * size_t(ncell), s)) != cudaSuccess)
             return failWith(SF_ERR_CUDA, std::string("cudaMemsetAsync: ") + cudaGetErrorString(e));
-        kNoAllocCount<<<blocks, kThreads, 0, s>>>(S, pos_dev, int(n), table, keyRank, report);
+        kNoAllocCount<<<blocks, kThreads, 0, s>>>(S, pos_dev, int(n), table, keyRank, scratch.reportOnDevice);
         kNoAllocScan<<<tiles, kThreads, 0, s>>>(table, ncell, shift, tileSum);
         kNoAllocAddTiles<<<tiles, kThreads, 0, s>>>(table, ncell, int(n), shift, tileSum);
         kNoAllocScatter<<<blocks, kThreads, 0, s>>>(int(n), table, keyRank, arrived);
-        kNoAllocOrder<<<blocks, kThreads, 0, s>>>(int(n), table, keyRank, arrived, perm_out_dev, report);
+        kNoAllocOrder<<<blocks, kThreads, 0, s>>>(int(n), table, keyRank, arrived, perm_out_dev,
+                                                  scratch.reportOnDevice);
         if ((e = cudaGetLastError()) != cudaSuccess)
             return failWith(SF_ERR_CUDA, std::string("sf_cell_sort_noalloc launch: ") + cudaGetErrorString(e));
         if ((e = cudaStreamSynchronize(s)) != cudaSuccess)
@@ -268,7 +281,7 @@ extern "C" sf_status sf_cell_sort_noalloc(const sf_boundary_params* grid, const 
         sc.tiles = sortTiles(int(n));
         int bits = 1;
         while ((int64_t(1) << bits) <= int64_t(ncell)) ++bits;
-        kNoAllocKeys<<<blocks, kThreads, 0, s>>>(S, pos_dev, int(n), keys, report);
+        kNoAllocKeys<<<blocks, kThreads, 0, s>>>(S, pos_dev, int(n), keys, scratch.reportOnDevice);
         unsigned int *sortedKeys = nullptr, *perm = nullptr;
         radixSort(s, int(n), bits, keys, sc, &sortedKeys, &perm);
         launchCellStart(s, int(n), ncell, sortedKeys, table);
