@@ -216,7 +216,7 @@ struct sf_handle {
     unsigned int* sortedKeys = nullptr;  // points into keys/scratch after a sort
     SortScratch sc{};
     bool countingSort = false;  // by cell count and slot count (useCountingSort), else the radix sort
-    unsigned int *cellCount = nullptr, *tileCount = nullptr, *parkedBefore = nullptr;
+    unsigned int *cellCount = nullptr, *tileCount = nullptr, *parkedBefore = nullptr, *parkedTile = nullptr;
     uint2* keyRank = nullptr;
     unsigned char* parkedInWarp = nullptr;
     // the keys and counts of the counting sort: none (counts zero), of the
@@ -352,8 +352,8 @@ struct sf_handle {
         if (counts == kCountsReady) counts = kCountsStale;
     }
     CountScratch countScratch() const {
-        return CountScratch{cellCount, tileCount, keyRank, parkedInWarp, parkedBefore, sc.vals, keys,
-                            countTileShift(totalCells)};
+        return CountScratch{cellCount, tileCount, keyRank, parkedInWarp, parkedBefore, parkedTile, sc.vals, keys,
+                            countTileShift(totalCells), parkedTileShift(totalSlots)};
     }
     void setLanes(int all) { lanes = adjLanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
     void setAutomaticLanes(int smCount) {
@@ -445,6 +445,7 @@ struct sf_handle {
         devFree(tileCount);
         devFree(parkedInWarp);
         devFree(parkedBefore);
+        devFree(parkedTile);
         devFree(bpos);
         devFree(blabel);
         devFree(dScenes);
@@ -820,6 +821,7 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
         SF_ALLOC(h->keyRank, sizeof(uint2) * M);
         SF_ALLOC(h->parkedInWarp, M / 32);
         SF_ALLOC(h->parkedBefore, sizeof(unsigned) * M / kSlotAlign);
+        SF_ALLOC(h->parkedTile, sizeof(unsigned) * kMaxParkedTiles);
     } else {
         SF_ALLOC(h->sc.keysAlt, sizeof(unsigned) * M);
         SF_ALLOC(h->sc.valsAlt, sizeof(unsigned) * M);

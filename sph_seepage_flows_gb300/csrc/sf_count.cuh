@@ -7,8 +7,10 @@
 
 namespace sfg {
 
-// Set in the place of a slot that is parked (p.w is 0): its place in keyRank is
-// then its number among the parked slots of its warp (see parkedPlace).
+// Set in the place of a slot that is parked (p.w is 0). The place then holds its
+// number among the parked slots of its warp and, above those five bits, the
+// first block of kSlotAlign slots of its scene (at most 2^22 of them): what the
+// scatter needs for parkedPlace without another chain of loads.
 constexpr unsigned int kParkedBit = 0x80000000u;
 
 // Counts slot (position p, parked when p.w is 0) into its cell and writes its
@@ -35,7 +37,8 @@ __device__ __forceinline__ void countSlot(const SceneDev& S, int slot, float4 p,
     at = __shfl_sync(0xffffffffu, at, leader) + (lane - unsigned(leader));
     const unsigned int parked = __ballot_sync(0xffffffffu, !live);
     if (lane == 0u) cc.parkedInWarp[slot >> 5] = static_cast<unsigned char>(__popc(parked));
-    cc.keyRank[slot] = make_uint2(key, live ? at : kParkedBit | unsigned(__popc(parked & ((1u << lane) - 1u))));
+    const unsigned int park = kParkedBit | unsigned(S.slot_off / kSlotAlign) << 5 | unsigned(__popc(parked & ((1u << lane) - 1u)));
+    cc.keyRank[slot] = make_uint2(key, live ? at : park);
     const int blockParked = __syncthreads_count(!live);
     if (threadIdx.x == 0 && blockParked) atomicAdd(&cc.count[S.cell_off + S.ncell], unsigned(blockParked));
 }
@@ -53,11 +56,12 @@ __device__ __forceinline__ unsigned int parkedInWarps(const CountScratch& cc, in
     return __dp4a(w.x, 0x01010101u, __dp4a(w.y, 0x01010101u, 0u));
 }
 
-// Place of a parked slot, whose keyRank entry is rank, among its scene's parked slots.
-__device__ __forceinline__ unsigned int parkedPlace(const CountScratch& cc, const SceneDev& S, int slot,
-                                                    unsigned int rank) {
-    return cc.parkedBefore[slot / kSlotAlign] - cc.parkedBefore[S.slot_off / kSlotAlign] +
-           parkedInWarps(cc, slot / kSlotAlign, (slot >> 5) & 7) + (rank & ~kParkedBit);
+// Place of a parked slot, whose place in keyRank is park, among its scene's parked slots.
+__device__ __forceinline__ unsigned int parkedPlace(const CountScratch& cc, int slot, unsigned int park) {
+    const int block = slot / kSlotAlign, first = int((park & ~kParkedBit) >> 5);
+    unsigned int place = cc.parkedBefore[block] - cc.parkedBefore[first] + parkedInWarps(cc, block, (slot >> 5) & 7) + (park & 31u);
+    for (int t = first >> cc.parkedShift; t < block >> cc.parkedShift; ++t) place += cc.parkedTile[t];
+    return place;
 }
 
 }  // namespace sfg

@@ -181,10 +181,12 @@ struct CountScratch {
     unsigned int* tileCount;   // kMaxCountTiles: slots per table tile
     uint2* keyRank;            // n: key of each slot before the sort, place among the slots counted into its cell
     unsigned char* parkedInWarp;  // n / 32: parked slots of each 32
-    unsigned int* parkedBefore;   // n / 256: parked slots before each block of 256
+    unsigned int* parkedBefore;   // n / 256: parked slots before each block of 256, within its tile of blocks
+    unsigned int* parkedTile;     // kMaxParkedTiles: parked slots of each tile of blocks
     unsigned int* arrived;     // n: slots of each cell, in arrival order
     unsigned int* sortedKeys;  // n: keys after the sort
     int tileShift;             // log2 of the cells per table tile (countTileShift)
+    int parkedShift;           // log2 of the blocks of 256 slots per tile (parkedTileShift)
 };
 // timeArgDev: when not null, the kernel reads timeArg from this device scalar
 // (graph-replayed steps whose render interval changes from call to call).
@@ -245,6 +247,11 @@ bool useCountingSort(int slots, int cells);
 // log2 of the cells per table tile: 1024 cells, doubled until at most
 // kMaxCountTiles tiles are left (every block of the scatter scans the tile sums).
 int countTileShift(int cells);
+// log2 of the blocks of slots per tile of the scan of the parked slots: 1024,
+// doubled until at most kMaxParkedTiles tiles are left (a parked slot adds the
+// sums of those of its scene before it).
+constexpr int kMaxParkedTiles = 64;
+int parkedTileShift(int slots);
 // Keys and counts of n slots at pos, into zero counts.
 void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc);
 // The sort stage from the keys and counts: cell table, stable order and gather

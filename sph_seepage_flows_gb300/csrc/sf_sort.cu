@@ -442,6 +442,12 @@ int countTileShift(int cells) {
     return shift;
 }
 
+int parkedTileShift(int slots) {
+    int shift = 10;
+    while ((slots / kSlotAlign >> shift) >= kMaxParkedTiles) ++shift;
+    return shift;
+}
+
 __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restrict__ scenes,
                                                          const int* __restrict__ blockScene,
                                                          const float4* __restrict__ pos4, CountScratch cc,
@@ -450,32 +456,32 @@ __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restr
     countSlot(scenes[blockScene[blockIdx.x]], slot, pos4[slot], cc, errWord);
 }
 
-// Exclusive prefix of the parked slots over the blocks of kSlotAlign slots, by
-// one block of threads, 4096 blocks a turn (a million slots).
-__device__ __forceinline__ void scanParked(const CountScratch& cc, int blocks) {
-    constexpr int kItems = 16;
+// Tile t of the blocks of kSlotAlign slots: exclusive prefix of their parked slots, and its sum.
+__device__ __forceinline__ void scanParked(const CountScratch& cc, int t, int blocks) {
     unsigned int carry = 0u, total;
-    for (int base = 0; base < blocks; base += kSortThreads * kItems) {
-        const int first = base + int(threadIdx.x) * kItems;
-        unsigned int v[kItems], sum = 0u;
+    const int end = min((t + 1) << cc.parkedShift, blocks);
+    for (int base = t << cc.parkedShift; base < end; base += kScanChunk) {
+        const int first = base + int(threadIdx.x) * kScanItems;
+        unsigned int v[kScanItems], sum = 0u;
 #pragma unroll
-        for (int u = 0; u < kItems; ++u) sum += v[u] = first + u < blocks ? parkedInWarps(cc, first + u, 8) : 0u;
+        for (int u = 0; u < kScanItems; ++u) sum += v[u] = first + u < end ? parkedInWarps(cc, first + u, 8) : 0u;
         unsigned int a = carry + blockScan(sum, total);
 #pragma unroll
-        for (int u = 0; u < kItems; ++u) {
-            if (first + u < blocks) cc.parkedBefore[first + u] = a;
+        for (int u = 0; u < kScanItems; ++u) {
+            if (first + u < end) cc.parkedBefore[first + u] = a;
             a += v[u];
         }
         carry += total;
     }
+    if (threadIdx.x == 0) cc.parkedTile[t] = carry;
 }
 
 // Block b scans table tile b (2^tileShift cells, a multiple of kScanChunk) in
-// place and writes its sum; the block behind the tiles scans the parked slots.
-__global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int n, int nCells) {
+// place and writes its sum; the blocks behind the tiles scan the parked slots.
+__global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int n, int nCells, int tiles) {
     unsigned int carry = 0u, total;
     const int tile = afterPrevious(int(blockIdx.x));
-    if (tile == int(gridDim.x) - 1) return scanParked(cc, n / kSlotAlign);
+    if (tile >= tiles) return scanParked(cc, tile - tiles, n / kSlotAlign);
     const int tileBeg = tile << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
     for (int base = tileBeg; base < tileEnd; base += kScanChunk) {
         const int c = base + int(threadIdx.x) * kScanItems;
@@ -489,9 +495,7 @@ __global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int n
     if (threadIdx.x == 0) cc.tileCount[blockIdx.x] = carry;
 }
 
-__global__ void __launch_bounds__(kSortThreads) kCountScatter(const SceneDev* __restrict__ scenes,
-                                                              const int* __restrict__ blockScene, CountScratch cc,
-                                                              int n, int nCells, int tiles,
+__global__ void __launch_bounds__(kSortThreads) kCountScatter(CountScratch cc, int n, int nCells, int tiles,
                                                               unsigned int* __restrict__ cs) {
     // every block scans the (at most kMaxCountTiles) tile sums
     __shared__ unsigned int before[kMaxCountTiles];
@@ -507,7 +511,7 @@ __global__ void __launch_bounds__(kSortThreads) kCountScatter(const SceneDev* __
     const int first = blockIdx.x * kSortThreads + tid, threads = gridDim.x * kSortThreads;
     for (int i = first; i < n; i += threads) {
         uint2 kr = cc.keyRank[i];
-        if (kr.y & kParkedBit) kr.y = parkedPlace(cc, scenes[blockScene[i / kSlotAlign]], i, kr.y);
+        if (kr.y & kParkedBit) kr.y = parkedPlace(cc, i, kr.y);
         cc.arrived[cc.count[kr.x] + before[kr.x >> cc.tileShift] + kr.y] = unsigned(i);
     }
     for (int c = first; c < nCells; c += threads) cs[c] = cc.count[c] + before[c >> cc.tileShift];
@@ -557,9 +561,10 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
                        float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
                        unsigned int* cellStart, float4* pairXY, float2* pairZ) {
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
-    launchChained(c.stream, tiles + 1, kSortThreads, 0, kCellScan, cc, n, nCells);
-    launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, c.scenes, c.blockScene,
-                  cc, n, nCells, tiles, cellStart);
+    const int parkedTiles = ((blocks - 1) >> cc.parkedShift) + 1;
+    launchChained(c.stream, tiles + parkedTiles, kSortThreads, 0, kCellScan, cc, n, nCells, tiles);
+    launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
+                  cellStart);
     launchChained(c.stream, blocks, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
                   pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
                   reinterpret_cast<float*>(pairZ));

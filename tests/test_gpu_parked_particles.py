@@ -24,7 +24,7 @@ def park(n, rng):
 
 @pytest.mark.parametrize("sizes, side, spare", [
     ((5,), 0.4, 0), ((255, 256, 257), 0.4, 0), ((1000,), 0.4, 5000), ((20011,), 1.3, 0), ((900, 3000), 0.4, 40),
-    ((1500,), 6.0, 300)])
+    ((1000, 700), 0.4, 400000), ((1500,), 6.0, 300)])
 def test_parked_particles_stay_in_slot_order(cuda_lib, sizes, side, spare):
     from sph_seepage_flows_gb300.capi import Simulation
     scs = [make_scene(n, side, 20 + k) for k, n in enumerate(sizes)]
