@@ -21,10 +21,9 @@ constexpr unsigned int kParkedBit = 0x80000000u;
 // one per block. Its slots are not ordered by those atomics: a particle whose
 // mass was set to 0 is parked too, keeps its id and has to stay in slot order
 // before the blank slots, so each warp leaves the number of its parked slots.
-__device__ __forceinline__ void countSlot(const SceneDev& S, int slot, float4 p, const CountScratch& cc,
-                                          unsigned int* errWord) {
+__device__ __forceinline__ void countSlot(const SceneDev& S, int slot, float4 p, const CountScratch& cc) {
     const bool live = p.w != 0.f;
-    const unsigned int key = slotKey(S, p, errWord);
+    const unsigned int key = slotKey(S, p);
     const unsigned int lane = threadIdx.x & 31u;
     const unsigned int prev = __shfl_up_sync(0xffffffffu, key, 1);
     const unsigned int heads = __ballot_sync(0xffffffffu, lane == 0u || prev != key);

@@ -1200,8 +1200,7 @@ __global__ void kIntegrate(const SceneDev* __restrict__ scenes, const int* __res
                            int adaptive,
                            const unsigned int* __restrict__ bcs, const float4* __restrict__ bpos4,
                            float4* __restrict__ pos4, float4* __restrict__ vel4, float4* __restrict__ acc4,
-                           float4* __restrict__ adh4, float4* __restrict__ avgadh4, CountScratch cc,
-                           unsigned int* errWord) {
+                           float4* __restrict__ adh4, float4* __restrict__ avgadh4, CountScratch cc) {
     SF_SLOT_PROLOGUE
     if (timeArgDev) timeArg = *timeArgDev;  // a graph-replayed step reads the time from the device
     float dt = timeArg;
@@ -1266,7 +1265,7 @@ __global__ void kIntegrate(const SceneDev* __restrict__ scenes, const int* __res
         avgadh4[slot] = make_float4(0.f, 0.f, 0.f, 0.f);
     }
     // the next sort's keys and counts
-    if (cc.keyRank) countSlot(S, slot, p4, cc, errWord);
+    if (cc.keyRank) countSlot(S, slot, p4, cc);
 }
 
 // ------------------------------------------------- neighbour-count probe
@@ -1391,7 +1390,7 @@ void launchIntegrate(const LaunchCtx& c, const PassBuffers& b, float timeArg, in
                      const CountScratch& cc) {
     launchChained(c.stream, grid(c, kPassIntegrate), c.block[kPassIntegrate], 0, kIntegrate, c.scenes, c.blockScene,
                   c.state, timeArg, timeArgDev, adaptive, b.lists.bcs, b.bpos4, b.pos4, b.vel4, b.acc4, b.adh4,
-                  b.avgadh4, cc, c.errWord);
+                  b.avgadh4, cc);
 }
 
 }  // namespace sfg

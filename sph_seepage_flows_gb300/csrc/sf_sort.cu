@@ -94,7 +94,8 @@ __global__ void __launch_bounds__(kSortThreads) kKeysHist(const SceneDev* __rest
         for (int u = 0; u < kGroup; ++u) {
             const int slot = base + (r0 + u) * kSortThreads + threadIdx.x;
             if (slot < n) {
-                const unsigned int k = slotKey(scenes[sid[u]], p[u], errWord);
+                const unsigned int k = slotKey(scenes[sid[u]], p[u]);
+                checkPosition(p[u], errWord);
                 keys[slot] = k;
                 atomicAdd(&h[k & unsigned(R - 1)], 1u);
             }
@@ -420,7 +421,9 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 //                  slots in slot order)
 //   kCellReorder   the place of each slot within its cell by slot number (the
 //                  stable order), the gather of the persistent arrays, and the
-//                  counts cleared for the next sort
+//                  counts cleared for the next sort; a non-finite position is
+//                  reported here and not where it was counted, since a caller
+//                  may still replace what the integrator wrote
 // The particles are nearly in cell order from the substep before, so a warp
 // counts its runs of equal keys with one atomic each, and a cell's slots are
 // next to each other in memory. Atomics on few addresses are kept out: a count
@@ -450,10 +453,9 @@ int parkedTileShift(int slots) {
 
 __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restrict__ scenes,
                                                          const int* __restrict__ blockScene,
-                                                         const float4* __restrict__ pos4, CountScratch cc,
-                                                         unsigned int* errWord) {
+                                                         const float4* __restrict__ pos4, CountScratch cc) {
     const int slot = blockIdx.x * kSlotAlign + afterPrevious(threadIdx.x);
-    countSlot(scenes[blockScene[blockIdx.x]], slot, pos4[slot], cc, errWord);
+    countSlot(scenes[blockScene[blockIdx.x]], slot, pos4[slot], cc);
 }
 
 // Tile t of the blocks of kSlotAlign slots: exclusive prefix of their parked slots, and its sum.
@@ -524,7 +526,7 @@ __global__ void __launch_bounds__(kSortThreads)
                  const float2* __restrict__ amc, const int* __restrict__ pid, float4* __restrict__ posOut,
                  float4* __restrict__ velOut, float4* __restrict__ colOut, float4* __restrict__ matOut,
                  float2* __restrict__ amcOut, int* __restrict__ pidOut, float* __restrict__ pairXY,
-                 float* __restrict__ pairZ) {
+                 float* __restrict__ pairZ, unsigned int* errWord) {
     const int i = blockIdx.x * kSortThreads + afterPrevious(threadIdx.x);
     for (int c = i; c < ((nCells + 3) & ~3); c += gridDim.x * kSortThreads) cc.count[c] = 0u;
     if (i >= n) return;
@@ -534,6 +536,7 @@ __global__ void __launch_bounds__(kSortThreads)
     const int id = pid[o];
     const unsigned int key = cc.keyRank[o].x;
     unsigned int d = unsigned(i);
+    checkPosition(p, errWord);
     if (p.w != 0.f) {  // the parked slots are listed in slot order
         const unsigned int beg = cs[key], end = cs[key + 1];
         d = beg;
@@ -553,7 +556,7 @@ __global__ void __launch_bounds__(kSortThreads)
 }
 
 void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc) {
-    launchChained(c.stream, n / kSlotAlign, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc, c.errWord);
+    launchChained(c.stream, n / kSlotAlign, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc);
 }
 
 int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch& cc, const float4* pos,
@@ -567,7 +570,7 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
                   cellStart);
     launchChained(c.stream, blocks, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
                   pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
-                  reinterpret_cast<float*>(pairZ));
+                  reinterpret_cast<float*>(pairZ), c.errWord);
     return 3;
 }
 
