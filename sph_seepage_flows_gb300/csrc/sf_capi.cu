@@ -1805,10 +1805,12 @@ __global__ void __launch_bounds__(kSlotAlign) kResetOrder(const SceneDev* __rest
                                                           float4* __restrict__ pos2, float4* __restrict__ vel2,
                                                           float4* __restrict__ col2, float4* __restrict__ mat2,
                                                           float2* __restrict__ amc2, int* __restrict__ pid2,
-                                                          unsigned int* __restrict__ cellCount, int nCells) {
+                                                          unsigned int* __restrict__ cellCount, int nCells,
+                                                          int slots) {
     const int s = blockIdx.x * kSlotAlign + threadIdx.x;
     if (cellCount)  // the counts were those of the old order
         for (int c = s; c < nCells; c += gridDim.x * kSlotAlign) cellCount[c] = 0u;
+    if (s >= slots) return;
     const int id = from.pid[s];
     const int d = id >= 0 ? scenes[blockScene[blockIdx.x]].slot_off + id : s;
     pos2[d] = from.pos[s];
@@ -1824,10 +1826,11 @@ __global__ void __launch_bounds__(kSlotAlign) kResetOrder(const SceneDev* __rest
 sf_status sf_reset_order(sf_handle* h) {
     if (!h) return SF_ERR_INVALID;
     const int t = 1 - h->cur;
-    kResetOrder<<<h->slotBlocks, kSlotAlign, 0, h->stream>>>(h->dScenes, h->dBlockScene, fieldArrays(h), h->pos[t],
-                                                             h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t],
-                                                             h->counts != sf_handle::kCountsZero ? h->cellCount : nullptr,
-                                                             h->totalCells + 4);
+    unsigned int* counts = h->counts != sf_handle::kCountsZero ? h->cellCount : nullptr;
+    const int cells = counts ? h->totalCells + 4 : 1;
+    kResetOrder<<<tableBlocks(h->slotBlocks, cells), kSlotAlign, 0, h->stream>>>(
+        h->dScenes, h->dBlockScene, fieldArrays(h), h->pos[t], h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t],
+        counts, cells, h->totalSlots);
     h->launches += 1;
     h->cur = t;
     h->sorted = false;

@@ -445,6 +445,10 @@ int countTileShift(int cells) {
     return shift;
 }
 
+int tableBlocks(int slotBlocks, int cells) {
+    return std::max(slotBlocks, std::min((cells - 1) / (4 * kSortThreads) + 1, kScatterBlocks));
+}
+
 int parkedTileShift(int slots) {
     int shift = 10;
     while ((slots / kSlotAlign >> shift) >= kMaxParkedTiles) ++shift;
@@ -566,9 +570,10 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
     const int parkedTiles = ((blocks - 1) >> cc.parkedShift) + 1;
     launchChained(c.stream, tiles + parkedTiles, kSortThreads, 0, kCellScan, cc, n, nCells, tiles);
-    launchChained(c.stream, std::min(blocks, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
+    const int all = tableBlocks(blocks, nCells);
+    launchChained(c.stream, std::min(all, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
                   cellStart);
-    launchChained(c.stream, blocks, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
+    launchChained(c.stream, all, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
                   pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
                   reinterpret_cast<float*>(pairZ), c.errWord);
     return 3;
