@@ -2406,13 +2406,14 @@ sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t che
                 "parameter gradient D2H") ||
         h->cuda(cudaStreamSynchronize(h->stream), "adjoint sync"))
         return SF_ERR_CUDA;
-    // packed gradients: positions, then velocities
+    // packed gradients: positions, then velocities, in the snapshots (76 B per
+    // slot at least), which nothing needs any more: no memory is taken for them
     const size_t gradBytes = sizeof(float) * 3 * size_t(off);
     float *gx = nullptr, *gv = nullptr;
     if (off > 0 && (grad_pos0_out || grad_vel0_out)) {
-        if (ensureStage(h, 2 * gradBytes)) return SF_ERR_CUDA;
-        if (grad_pos0_out) gx = static_cast<float*>(h->stage);
-        if (grad_vel0_out) gv = static_cast<float*>(h->stage) + 3 * size_t(off);
+        float* packed = reinterpret_cast<float*>(h->snap);
+        if (grad_pos0_out) gx = packed;
+        if (grad_vel0_out) gv = packed + 3 * size_t(off);
     }
     off = 0;
     for (int s = 0; s < h->nScenes; ++s) {
