@@ -1226,6 +1226,17 @@ struct FieldList {
 // one before it on the SMs (afterPrevious). 64 scenes of about 17k particles, a
 // call each: four fields set 532 -> 277 us, three fields read 318 -> 205 us.
 constexpr int kFieldBatch = 4;
+// Most particles of a scene for which a list is read in one launch, and for
+// which its vector fields in sorted order are set with the others. Beyond, the
+// launches no longer count and what bounds is memory: the registers of a batch
+// halve the threads in flight, and whole words through shared memory
+// (kGetVec3, kSetVec3) beat strided ones. One launch / one per field, us: get
+// four vectors by id at 1M 41 / 40, 1.5M 67 / 57, 4M 150 / 126; two scalars at
+// 1M 7.6 / 7.0, 4M 42 / 32; set two sorted vectors at 0.7M 12 / 14, 1M 28 / 17,
+// 4M 111 / 82, while scalars and fields by id are set as fast or faster in one
+// launch at every size. A list of one field has a kernel of its own, without
+// the batch's registers (12 instead of 50: get one vector by id at 4M 46 -> 31).
+constexpr int64_t kListGetParticles = 1000000, kListSetParticles = 800000;
 
 // Field's value of slot s, in as many components as the field has words
 // (integers as their bits).
@@ -1282,6 +1293,19 @@ __global__ void kGetFields(FieldList list, int n, int slotOff, int cellOff, int 
             if (w > 2) out[2] = v[k].z;
         }
     }
+}
+
+// A list of one field.
+__global__ void kGetField(FieldList list, int n, int slotOff, int cellOff, int order, FieldArrays A) {
+    const int i = blockIdx.x * blockDim.x + afterPrevious(threadIdx.x);
+    if (i >= n) return;
+    const int s = slotOff + i, w = list.width[0];
+    const int o = order == SF_ORDER_ID ? A.pid[s] : i;
+    const float3 v = getField(list.field[0], s, cellOff, A);
+    float* out = static_cast<float*>(list.buf[0]) + size_t(w) * size_t(o);
+    out[0] = v.x;
+    if (w > 1) out[1] = v.y;
+    if (w > 2) out[2] = v.z;
 }
 
 // The values the passes derive from a slot's fields for later passes (the
@@ -1380,6 +1404,19 @@ __global__ void kSetFields(FieldList list, int n, int slotOff, int order, FieldA
         }
     }
     if (derived)
+        refreshDerived(s, A.pos, A.vel, A.aux, A.flow, A.avgadh, A.drag, A.dp, A.vrec2, A.grec4, *scene);
+}
+
+// A list of one field.
+__global__ void kSetField(FieldList list, int n, int slotOff, int order, FieldArrays A,
+                          const SceneDev* __restrict__ scene) {
+    const int i = blockIdx.x * blockDim.x + afterPrevious(threadIdx.x);
+    if (i >= n) return;
+    const int s = slotOff + i, w = list.width[0];
+    const int o = order == SF_ORDER_ID ? A.pid[s] : i;
+    const float* in = static_cast<const float*>(list.buf[0]) + size_t(w) * size_t(o);
+    setField(list.field[0], s, A, make_float3(in[0], w > 1 ? in[1] : 0.f, w > 2 ? in[2] : 0.f));
+    if (hasDerived(list.field[0]))
         refreshDerived(s, A.pos, A.vel, A.aux, A.flow, A.avgadh, A.drag, A.dp, A.vrec2, A.grec4, *scene);
 }
 
@@ -1533,8 +1570,8 @@ FieldList oneField(int field, const void* buf) {
 
 sf_status launchGetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
     const SceneDev& S = h->hScenes[scene];
-    launchChained(h->stream, int((n + 255) / 256), 256, 0, kGetFields, list, int(n), S.slot_off, S.cell_off, order,
-                  fieldArrays(h));
+    launchChained(h->stream, int((n + 255) / 256), 256, 0, list.n == 1 ? kGetField : kGetFields, list,
+                  int(n), S.slot_off, S.cell_off, order, fieldArrays(h));
     return h->cuda(cudaGetLastError(), "get_field launch");
 }
 
@@ -1587,13 +1624,14 @@ sf_status sf_get_field(sf_handle* h, int32_t scene, int32_t field, int32_t order
 sf_status sf_get_fields(sf_handle* h, int32_t scene, int32_t n_fields, const int32_t* fields, int32_t order,
                         void* const* dsts, int64_t count, int32_t dst_on_device) {
     if (!h || n_fields < 0 || (n_fields > 0 && (!fields || !dsts))) return SF_ERR_INVALID;
-    // device buffers: one launch for (up to kFieldsPerLaunch) fields
+    // device buffers: one launch for (up to kFieldsPerLaunch) fields, unless the scene is large
     if (dst_on_device) {
         FieldList list;
         for (int32_t k = 0; k < n_fields; ++k) {
             size_t bytes = 0;
             sf_status st = checkField(h, scene, fields[k], order, dsts[k], count, false, &bytes);
-            const bool own = st == SF_OK && fields[k] >= SF_BFIELD_POS;  // boundary fields
+            // boundary fields, and any of many particles
+            const bool own = st == SF_OK && (fields[k] >= SF_BFIELD_POS || (n_fields > 1 && count > kListGetParticles));
             if (!own && st == SF_OK) {
                 list.add(fields[k], fieldWidth(fields[k]), dsts[k]);
             }
@@ -1624,8 +1662,8 @@ bool movesParticles(int field) {
 sf_status launchSetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
     for (int k = 0; k < list.n; ++k)
         if (movesParticles(list.field[k])) h->positionsChanged();
-    launchChained(h->stream, int((n + 255) / 256), 256, 0, kSetFields, list, int(n), h->hScenes[scene].slot_off, order,
-                  fieldArrays(h), h->dScenes + scene);
+    launchChained(h->stream, int((n + 255) / 256), 256, 0, list.n == 1 ? kSetField : kSetFields, list,
+                  int(n), h->hScenes[scene].slot_off, order, fieldArrays(h), h->dScenes + scene);
     return h->cuda(cudaGetLastError(), "set_field launch");
 }
 
@@ -1670,22 +1708,26 @@ sf_status sf_set_field(sf_handle* h, int32_t scene, int32_t field, int32_t order
 sf_status sf_set_fields(sf_handle* h, int32_t scene, int32_t n_fields, const int32_t* fields, int32_t order,
                         const void* const* srcs, int64_t count, int32_t src_on_device) {
     if (!h || n_fields < 0 || (n_fields > 0 && (!fields || !srcs))) return SF_ERR_INVALID;
-    // device buffers: one launch for (up to kFieldsPerLaunch) fields
+    // device buffers: one launch for (up to kFieldsPerLaunch) fields; large vector fields in their own
     if (src_on_device) {
         FieldList list;
         for (int32_t k = 0; k < n_fields; ++k) {
             size_t bytes = 0;
-            const sf_status st = checkField(h, scene, fields[k], order, srcs[k], count, true, &bytes);
-            if (st == SF_OK) {
+            sf_status st = checkField(h, scene, fields[k], order, srcs[k], count, true, &bytes);
+            // vector fields of many particles
+            const bool own = st == SF_OK && n_fields > 1 && count > kListSetParticles && order == SF_ORDER_SORTED &&
+                             vec3Array(h, fields[k]) && (reinterpret_cast<uintptr_t>(srcs[k]) & 15u) == 0;
+            if (!own && st == SF_OK) {
                 list.add(fields[k], fieldWidth(fields[k]), srcs[k]);
             }
             // the fields before an invalid one are set, as by calls of their own
-            if (list.n > 0 && (st || list.n == kFieldsPerLaunch || k == n_fields - 1)) {
+            if (list.n > 0 && (st || own || list.n == kFieldsPerLaunch || k == n_fields - 1)) {
                 const sf_status ls = count > 0 ? launchSetFields(h, scene, list, order, count) : SF_OK;
                 list.n = 0;
                 if (ls) return ls;
             }
             if (st) return st;
+            if (own && (st = setFieldQueued(h, scene, fields[k], order, srcs[k], count, 1))) return st;
         }
         return SF_OK;
     }
