@@ -342,18 +342,21 @@ sf_status sf_get_density_staging(const sf_handle* h, int32_t* staged);
 /* Autotuner (no reference counterpart). Sizes the neighbour lists for the
  * current state (list capacity = largest neighbour count + 25%, a multiple of
  * 32 in [64, 256]; sf_create does this once for the initial state), then
- * times on the current state, with CUDA events: the radix sort with 8, 4, 2
- * and 1 keys per thread (tile size) and with 8-bit or wider digits, and, for
- * 1, 2, 4 and 8 threads per
+ * times on the current state, with CUDA events, for 1, 2, 4 and 8 threads per
  * particle, each neighbour pass with 64, 128 and 256 threads per block
- * (density, average flow, voidage/adhesion, sand momentum, water momentum;
- * the integrator keeps its size; with one thread per particle the density
- * pass with and without its shared-memory staging); it keeps the fastest sort tiles, the
- * fastest lane count of each pass up to voidage/adhesion (their results do
- * not depend on it) and the lane count with the smaller sum of the two
- * momentum passes, with those block sizes. The state is not advanced. block_sizes_out (6 entries, in
- * that pass order then the integrator) and list_capacity_out may be NULL;
- * sf_get_tuning reads every choice back. */
+ * (density, average flow, voidage/adhesion, sand momentum, water momentum; the
+ * integrator keeps its size), each in the form that substeps run. It keeps the
+ * fastest thread count of each pass up to voidage/adhesion (their results do
+ * not depend on it) and, for the two momentum passes, the one with the smaller
+ * sum, with those block sizes. With one thread per particle the density pass is
+ * also timed with its shared-memory staging, which is kept where it is faster
+ * together with the average flow that it leads to (which then sums the sand
+ * volume). Where the grid has so many more cells than the handle has particles
+ * that the radix sort runs, that is timed with 8, 4, 2 and 1 keys per thread
+ * (tile size) and with 8-bit or wider digits; the counting sort has nothing to
+ * choose, and the threads per particle of the adjoint kernels stay as they are.
+ * The state is not advanced. block_sizes_out (6 entries, in that pass order then
+ * the integrator) and list_capacity_out may be NULL. */
 sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t* list_capacity_out);
 
 /* The current launch configuration (no reference counterpart): block sizes

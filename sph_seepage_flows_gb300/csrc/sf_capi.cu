@@ -2011,60 +2011,67 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
     const int stages[kTunedPasses - 1] = {SF_STAGE_DENSITY, SF_STAGE_AVGFLOW, SF_STAGE_VOIDAGE_ADHESION,
                                           SF_STAGE_SAND_MOMENTUM, SF_STAGE_WATER_MOMENTUM};
     for (int s = SF_STAGE_DENSITY; s <= SF_STAGE_WATER_MOMENTUM && st == SF_OK; ++s) st = runStage(h, s, dt, 0);
-    // (with one lane the density pass is timed with and without its
-    // shared-memory staging as well). The passes up to voidage / adhesion give
-    // the same results for every lane count, so each keeps its own fastest;
-    // the two momentum passes share the one of their smaller sum.
-    constexpr int kFirstMomentum = kPassSand;
-    float bestMomentum = 0.f, bestList[kFirstMomentum] = {};
-    const int adjLanes = h->adjLanes;  // not timed here: stays as it is
-    int bestLanes = h->lanes, bestListLanes[kFirstMomentum], bestBlock[kTunedPasses - 1], bestStaged = 0;
-    for (int p = 0; p < kTunedPasses - 1; ++p) bestBlock[p] = h->block[p];
-    for (int p = 0; p < kFirstMomentum; ++p) bestListLanes[p] = h->listLanes[p];
-    for (int lanes : {1, 2, 4, 8}) {
-        if (st) break;
-        h->setLanes(lanes);
-        float momentum = 0.f;
-        int block[kTunedPasses - 1], staged = 0;
-        for (int p = 0; p < kTunedPasses - 1 && st == SF_OK; ++p) {
-            float best = 0.f;
-            block[p] = h->block[p];
-            const int forms = (p == kPassDensity && lanes == 1) ? 2 : 1;
-            for (int f = 0; f < forms && st == SF_OK; ++f) {
-                h->densityStaged = f;
-                for (int bs : candidates) {
-                    h->block[p] = bs;
-                    float ms = 0.f;
-                    if ((st = timed([&] { return runStage(h, stages[p], dt, 0); }, ms))) break;
-                    if (best == 0.f || ms < best) {
-                        best = ms;
-                        block[p] = bs;
-                        if (p == kPassDensity) staged = f;
-                    }
-                }
-            }
-            h->densityStaged = 0;
-            h->block[p] = block[p];
-            if (p >= kFirstMomentum) {
-                momentum += best;
-            } else if (st == SF_OK && (bestList[p] == 0.f || best < bestList[p])) {
-                bestList[p] = best;
-                bestListLanes[p] = lanes;
-                bestBlock[p] = block[p];
-                if (p == kPassDensity) bestStaged = staged;
-            }
+    // The passes up to voidage / adhesion give the same results for every lane
+    // count, so each keeps its own fastest; the two momentum passes share the
+    // one of their smaller sum. The average flow is timed as substeps run it,
+    // behind a density pass that summed the sand volume.
+    struct Choice {
+        float ms = 0.f;
+        int lanes = 0, block = 0;
+        void offer(float t, int l, int b) {
+            if (ms == 0.f || t < ms) *this = Choice{t, l, b};
         }
-        if (st == SF_OK && (bestMomentum == 0.f || momentum < bestMomentum)) {
-            bestMomentum = momentum;
-            bestLanes = lanes;
-            for (int p = kFirstMomentum; p < kTunedPasses - 1; ++p) bestBlock[p] = block[p];
+    };
+    const auto kept = h->ctx();
+    const int adjLanes = h->adjLanes;  // not timed here: stays as it is
+    Choice best[kTunedPasses - 1];     // of the momentum passes: with the lanes that are kept
+    // pass p at `lanes` and every block size; chained: as a part of a whole substep
+    auto tunePass = [&](int p, int lanes, bool chained, Choice& c) {
+        h->setLanes(lanes);
+        for (int bs : candidates) {
+            h->block[p] = bs;
+            float ms = 0.f;
+            if (st == SF_OK && (st = timed([&] { return runStage(h, stages[p], dt, 0, chained); }, ms)) == SF_OK)
+                c.offer(ms, lanes, bs);
+        }
+        h->block[p] = kept.block[p];
+    };
+    h->densityStaged = 0;
+    for (int lanes : {1, 2, 4, 8}) {
+        for (int p = kPassDensity; p <= kPassVoidage; ++p) tunePass(p, lanes, true, best[p]);
+        Choice sand, water;
+        tunePass(kPassSand, lanes, true, sand);
+        tunePass(kPassWater, lanes, true, water);
+        if (lanes == 1 || sand.ms + water.ms < best[kPassSand].ms + best[kPassWater].ms) {
+            best[kPassSand] = sand;
+            best[kPassWater] = water;
         }
     }
-    h->lanes = bestLanes;
+    // the density pass staged in shared memory (one lane) does not sum the sand
+    // volume, so the average flow does: the two forms are compared by the sum
+    Choice staged, flow;
+    h->densityStaged = 1;
+    tunePass(kPassDensity, 1, true, staged);
+    h->densityStaged = 0;
+    if (staged.ms < best[kPassDensity].ms)
+        for (int lanes : {1, 2, 4, 8}) tunePass(kPassAvgFlow, lanes, false, flow);
+    const bool useStaged =
+        flow.ms > 0.f && staged.ms + flow.ms < best[kPassDensity].ms + best[kPassAvgFlow].ms;
+    if (useStaged) {
+        best[kPassDensity] = staged;
+        best[kPassAvgFlow] = flow;
+    }
+    if (st == SF_OK) {
+        for (int p = 0; p < kTunedPasses - 1; ++p) h->block[p] = best[p].block;
+        for (int p = kPassDensity; p <= kPassVoidage; ++p) h->listLanes[p] = best[p].lanes;
+        h->lanes = best[kPassSand].lanes;
+        h->densityStaged = useStaged;
+    } else {
+        for (int p = kPassDensity; p <= kPassVoidage; ++p) h->listLanes[p] = kept.lanes[p];
+        h->lanes = kept.lanes[kPassSand];
+        h->densityStaged = kept.densityStaged;
+    }
     h->adjLanes = adjLanes;
-    for (int p = 0; p < kFirstMomentum; ++p) h->listLanes[p] = bestListLanes[p];
-    h->densityStaged = bestStaged;
-    for (int p = 0; p < kTunedPasses - 1; ++p) h->block[p] = bestBlock[p];
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     if (st) return st;
