@@ -223,6 +223,13 @@ struct sf_handle {
     // positions as they are (left by the integrator or the key kernel), or of
     // positions that have changed since
     enum { kCountsZero, kCountsReady, kCountsStale } counts = kCountsZero;
+    // Both are what the calls so far left on the device. A caller may also
+    // capture calls into a graph of its own and replay it at any time, which no
+    // call here sees, so the calls that rely on the two begin with track():
+    // they hold within one capture, and between calls only while the caller has
+    // captured none.
+    unsigned long long captureId = 0;  // of the caller's capture that the last tracked call was part of
+    bool callerCaptures = false;
     float4* bpos = nullptr;
     int* blabel = nullptr;
     // staging for field access
@@ -345,6 +352,22 @@ struct sf_handle {
         b.vrec2 = vrec2;
         b.grec4 = grec4;
         return b;
+    }
+    void track() {
+        cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+        unsigned long long id = 0;
+        if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) (void)cudaGetLastError();
+        trackIn(status == cudaStreamCaptureStatusActive ? id : 0);
+    }
+    // id: of the capture that the call is part of, 0 where it can be part of
+    // none (it launches a graph or waits, which a capture refuses)
+    void trackIn(unsigned long long id) {
+        if (id) callerCaptures = true;
+        if (callerCaptures && (id == 0 || id != captureId)) {
+            pairsFresh = false;
+            counts = kCountsStale;
+        }
+        captureId = id;
     }
     // positions or buffers changed outside the substep's passes
     void positionsChanged() {
@@ -989,6 +1012,7 @@ sf_status sf_run_stage(sf_handle* h, int32_t stage, float time_arg, int32_t adap
     if (!h) return SF_ERR_INVALID;
     if (stage < 0 || stage >= SF_STAGE_COUNT) return h->fail(SF_ERR_INVALID, "unknown stage");
     if (stage != SF_STAGE_SORT && !h->sorted) return h->fail(SF_ERR_INVALID, "run the sort stage first");
+    h->track();
     return runStage(h, stage, time_arg, adaptive);
 }
 
@@ -1046,6 +1070,7 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
         h->timeArg = t;
     }
     GraphCache& g = h->graphStep[h->cur];
+    h->trackIn(0);
     sf_status st = ensureCounts(h);
     if (st != SF_OK || (st = ensureStepGraph(h, g)) != SF_OK) return st;
     if (h->cuda(cudaGraphLaunch(g.exec, h->stream), "graph launch")) return SF_ERR_CUDA;
@@ -1170,6 +1195,7 @@ sf_status sf_substeps_fixed(sf_handle* h, float dt, int64_t n) {
     sf_status st = growListsIfFull(h, n > kListCheckEvery ? 0 : -1);
     if (st == SF_OK && n > kListCheckEvery) st = growListsIfFull(h, 1);
     if (st) return st;
+    h->trackIn(0);
     int prevSlot = -1;
     for (int64_t done = 0; done < n;) {
         const int64_t m = std::min(kListCheckEvery, n - done);
@@ -1660,6 +1686,7 @@ bool movesParticles(int field) {
 }
 
 sf_status launchSetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
+    h->track();
     for (int k = 0; k < list.n; ++k)
         if (movesParticles(list.field[k])) h->positionsChanged();
     launchChained(h->stream, int((n + 255) / 256), 256, 0, list.n == 1 ? kSetField : kSetFields, list,
@@ -1689,6 +1716,7 @@ sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
     float4* vec = order == SF_ORDER_SORTED ? vec3Array(h, field) : nullptr;
     if (!vec || (reinterpret_cast<uintptr_t>(from) & 15u) != 0)
         return launchSetFields(h, scene, oneField(field, from), order, n);
+    h->track();
     if (movesParticles(field)) h->positionsChanged();
     kSetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
         int(n), h->hScenes[scene].slot_off, vec, static_cast<const float4*>(from),
@@ -1867,6 +1895,7 @@ __global__ void __launch_bounds__(kSlotAlign) kResetOrder(const SceneDev* __rest
 
 sf_status sf_reset_order(sf_handle* h) {
     if (!h) return SF_ERR_INVALID;
+    h->track();
     const int t = 1 - h->cur;
     unsigned int* counts = h->counts != sf_handle::kCountsZero ? h->cellCount : nullptr;
     const int cells = counts ? h->totalCells + 4 : 1;
@@ -1957,6 +1986,7 @@ sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t*
     if (!h) return SF_ERR_INVALID;
     if (!(dt > 0.f) || !std::isfinite(dt)) return h->fail(SF_ERR_INVALID, "dt must be finite and > 0");
     sf_status st = SF_OK;
+    h->trackIn(0);
     if (!h->sorted && (st = runSort(h))) return st;
     if ((st = probeListCapacity(h))) return st;
     if (h->slab) {  // stored-substep slabs depend on the list capacity
@@ -2382,6 +2412,7 @@ sf_status sf_adjoint_run(sf_handle* h, float dt, int64_t n_substeps, int64_t che
     const int64_t T = n_substeps, K = std::min(checkpoint_every, n_substeps);
     const int64_t nSeg = (T + K - 1) / K;
     const int64_t lastLen = T - (nSeg - 1) * K;
+    h->trackIn(0);
     // lists found full by earlier calls grow first (the stored substeps are sized by the capacity)
     if (sf_status gs = growListsIfFull(h, -1)) return gs;
     // snapshots: segment starts [0, nSeg - 1) and the final state; slabs: one segment
