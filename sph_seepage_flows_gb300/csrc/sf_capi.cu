@@ -1261,7 +1261,9 @@ constexpr int kFieldBatch = 4;
 // 1M 7.6 / 7.0, 4M 42 / 32; set two sorted vectors at 0.7M 12 / 14, 1M 28 / 17,
 // 4M 111 / 82, while scalars and fields by id are set as fast or faster in one
 // launch at every size. A list of one field has a kernel of its own, without
-// the batch's registers (12 instead of 50: get one vector by id at 4M 46 -> 31).
+// the batch's registers (12 instead of 50: get one vector by id at 4M 46 -> 31);
+// pinned host memory off the 16-byte grid is left to the batch's, whose fewer
+// threads in flight suit the link (a vector of 119k particles 21 us, 31 without).
 constexpr int64_t kListGetParticles = 1000000, kListSetParticles = 800000;
 
 // Field's value of slot s, in as many components as the field has words
@@ -1594,9 +1596,10 @@ FieldList oneField(int field, const void* buf) {
     return l;
 }
 
-sf_status launchGetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
+sf_status launchGetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n,
+                          bool toHost = false) {
     const SceneDev& S = h->hScenes[scene];
-    launchChained(h->stream, int((n + 255) / 256), 256, 0, list.n == 1 ? kGetField : kGetFields, list,
+    launchChained(h->stream, int((n + 255) / 256), 256, 0, list.n == 1 && !toHost ? kGetField : kGetFields, list,
                   int(n), S.slot_off, S.cell_off, order, fieldArrays(h));
     return h->cuda(cudaGetLastError(), "get_field launch");
 }
@@ -1628,7 +1631,7 @@ sf_status getFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
             int(n), S.slot_off, vec, static_cast<float4*>(target));
     } else if (bfield) {
         kGetBoundary<<<int((n + 255) / 256), 256, 0, h->stream>>>(field, int(n), S.b_off, h->bpos, h->blabel, target);
-    } else if (launchGetFields(h, scene, oneField(field, target), order, n)) {
+    } else if (launchGetFields(h, scene, oneField(field, target), order, n, mapped != nullptr)) {
         return SF_ERR_CUDA;
     }
     if (h->cuda(cudaGetLastError(), "get_field launch")) return SF_ERR_CUDA;
