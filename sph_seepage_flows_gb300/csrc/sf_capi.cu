@@ -175,7 +175,7 @@ sf_status exportBgeoSlots(cudaStream_t s, int64_t n, const float4* pos4, const f
 struct sf_handle {
     cudaStream_t stream = nullptr;
     bool ownStream = false;
-    int device = 0;
+    int device = 0, smCount = 0;
     int nScenes = 0;
     std::vector<sf_params> P;
     std::vector<sf_boundary_params> B;
@@ -308,6 +308,7 @@ struct sf_handle {
         c.lanes[kPassSand] = c.lanes[kPassWater] = lanes;
         c.lanes[kPassIntegrate] = 1;
         c.densityStaged = densityStaged;
+        c.smCount = smCount;
         return c;
     }
     PassBuffers buffers() const {
@@ -379,7 +380,7 @@ struct sf_handle {
                             countTileShift(totalCells), parkedTileShift(totalSlots)};
     }
     void setLanes(int all) { lanes = adjLanes = listLanes[0] = listLanes[1] = listLanes[2] = all; }
-    void setAutomaticLanes(int smCount) {
+    void setAutomaticLanes() {
         setLanes(lanesForSlots(totalSlots, smCount));
         listLanes[0] = densityLanesForSlots(totalSlots, smCount);
         listLanes[1] = flowLanesForSlots(totalSlots, smCount);
@@ -824,14 +825,10 @@ sf_status sf_create_batched(int32_t n_scenes, const sf_params* params, const sf_
     SF_ALLOC(h->cnbrCnt, sizeof(int) * M);
     SF_ALLOC(h->cnbr, sizeof(unsigned) * M * kMaxContact);
     SF_ALLOC(h->sc.vals, sizeof(unsigned) * M);
-    {
-        int dev = 0, sms = 0;
-        if (h->cuda(cudaGetDevice(&dev), "cudaGetDevice") ||
-            h->cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"))
-            return bail(SF_ERR_CUDA);
-        h->sc.items = sortItemsFor(h->totalSlots, sms);
-        h->setAutomaticLanes(sms);
-    }
+    if (h->cuda(cudaDeviceGetAttribute(&h->smCount, cudaDevAttrMultiProcessorCount, h->device), "SM count"))
+        return bail(SF_ERR_CUDA);
+    h->sc.items = sortItemsFor(h->totalSlots, h->smCount);
+    h->setAutomaticLanes();
     h->sc.tiles = sortTiles(h->totalSlots, h->sc.items);
     // digits of 8 bits, or 9-11 when that saves a pass; room for the widest
     // digits and the smallest tiles, so that the tuner can change both
@@ -1902,7 +1899,7 @@ sf_status sf_reset_order(sf_handle* h) {
     const int t = 1 - h->cur;
     unsigned int* counts = h->counts != sf_handle::kCountsZero ? h->cellCount : nullptr;
     const int cells = counts ? h->totalCells + 4 : 1;
-    kResetOrder<<<tableBlocks(h->slotBlocks, cells), kSlotAlign, 0, h->stream>>>(
+    kResetOrder<<<tableBlocks(h->slotBlocks, cells, h->smCount), kSlotAlign, 0, h->stream>>>(
         h->dScenes, h->dBlockScene, fieldArrays(h), h->pos[t], h->vel[t], h->col[t], h->mat[t], h->amc[t], h->pid[t],
         counts, cells, h->totalSlots);
     h->launches += 1;
@@ -1973,11 +1970,7 @@ sf_status sf_set_lanes(sf_handle* h, int32_t lanes) {
     if (lanes != 0 && lanes != 1 && lanes != 2 && lanes != 4 && lanes != 8)
         return h->fail(SF_ERR_INVALID, "lanes must be 0 (automatic), 1, 2, 4 or 8");
     if (lanes == 0) {
-        int dev = 0, sms = 0;
-        if (h->cuda(cudaGetDevice(&dev), "cudaGetDevice") ||
-            h->cuda(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev), "SM count"))
-            return SF_ERR_CUDA;
-        h->setAutomaticLanes(sms);
+        h->setAutomaticLanes();
     } else {
         h->setLanes(lanes);
     }

@@ -309,8 +309,8 @@ __device__ __forceinline__ float sandVolumeTerm(const SceneDev& S, float wj, flo
 // Hits of one slot waiting to be appended: (first candidate, hit mask) of up
 // to kHitChunks chunks of 32 candidates, per thread.
 constexpr int kHitChunks = 12;
-// Most slots for the form of the one-lane density pass that loads ahead.
-constexpr int kAheadSlots = 600000;
+// Most slots per SM for the form of the one-lane density pass that loads ahead.
+constexpr long long kAheadSlotsPerSM = 2048;
 
 // Builds the neighbour lists (sand / water / boundary, each in stencil
 // order, plus the sand-sand contact list) and computes the density, fused
@@ -352,9 +352,12 @@ constexpr int kAheadSlots = 600000;
 //
 // kAhead: the hit phase loads the position of the next hit before it uses this
 // one's, with 64 registers (4 blocks of kSlotAlign threads per SM). That pays
-// while there are few waves of blocks (kAheadSlots): 40k 48 -> 43 us, 120k
-// 67 -> 63, 252k 90 -> 85, 306k of 12 scenes 147 -> 141; at a million the
-// occupancy is worth more (1M embankment 283 -> 286, 64 scenes 295 -> 306).
+// while there are two waves of blocks at most (kAheadSlotsPerSM): 40k 48 -> 43
+// us, 120k 67 -> 63, columns of 200k 115 -> 107 and 300k 134 -> 128, embankments of
+// 200k 79 -> 76 and 252k 90 -> 85 (but 300k 94 -> 100), 306k of 12 scenes 147 ->
+// 141. Beyond, the occupancy is worth more: columns of 400k 152 -> 154, 600k 195
+// -> 201, 800k 247 -> 261, embankments of 400k 118 -> 120, 600k 166 -> 171, 1M 260
+// -> 269.
 template <bool kAhead>
 __global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
     kDensity(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, SceneState* __restrict__ state,
@@ -1344,7 +1347,7 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
                 c.scenes, c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4, cap);
         } else {
             const size_t hits = size_t(kHitChunks) * c.block[kPassDensity] * sizeof(uint2);
-            const auto kernel = c.slotBlocks <= kAheadSlots / kSlotAlign ? kDensity<true> : kDensity<false>;
+            const auto kernel = c.slotBlocks <= kAheadSlotsPerSM * c.smCount / kSlotAlign ? kDensity<true> : kDensity<false>;
             launchChained(c.stream, grid(c, kPassDensity), c.block[kPassDensity], hits, kernel, c.scenes,
                           c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4);
         }

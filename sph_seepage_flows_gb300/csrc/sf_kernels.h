@@ -46,6 +46,7 @@ struct LaunchCtx {
     int block[kTunedPasses];  // threads per block of each tuned pass
     int lanes[kTunedPasses];  // threads per slot of each neighbour pass (1, 2, 4 or 8)
     int densityStaged;        // 1: the one-lane density pass stages its candidates in shared memory
+    int smCount;              // SMs of the device
 };
 
 // Largest shared staging of the density pass, in positions (16 B each): with
@@ -141,7 +142,15 @@ struct PassBuffers {
 
 // Threads per slot of the voidage / adhesion and momentum passes for
 // totalSlots slots on a GPU with smCount SMs: doubled, up to 8, while fewer
-// than 2048 threads per SM would run.
+// than 2048 threads per SM would run. The two momentum passes in us with 1, 2, 4
+// and 8 lanes, columns / embankments: 20k 47 30 21 17 / 35 22 17 14, 50k 55 34
+// 26 25 / 36 24 21 22, 75k 51 34 28 32 / 37 26 26 29, 100k 58 39 35 39 / 39 28 29
+// 36, 150k 59 43 44 53 / 43 37 39 51, 200k 82 51 54 69 / 46 41 49 67, 300k 79 68
+// 76 100 / 65 60 73 99, 340k 83 72 85 111 / 69 65 80 112, 420k 91 85 102 134 / 74
+// 75 98 137. The line dates from 48 registers a thread (five blocks per SM);
+// with the 64 of today 4 lanes are the better by a tenth from 55k to 78k slots, and 2
+// to 400k. It stays, as other lanes group the momentum sums differently, so
+// that results would differ from before in their rounding.
 int lanesForSlots(long long totalSlots, int smCount);
 // The same for the adjoint pair kernels, but 2 up to 4096 threads per SM: with
 // 24 warps per SM at most, one lane per particle leaves their last wave short
@@ -255,10 +264,10 @@ int parkedTileShift(int slots);
 // Blocks of 256 threads for a kernel that passes over the slots (slotBlocks) and
 // over the cell table: with the slots' blocks alone, a few slots in a large grid
 // leave the table to a few threads. Four cells per thread, and up to 8 blocks per
-// SM of 152 for the table. Sort stage with the blocks of the slots / with these:
+// SM for the table. Sort stage with the blocks of the slots / with these:
 // 250 slots in 97k cells 94 / 9 us, in 1M 895 / 12; 2000 in 97k 20 / 11, in 1M 121 /
 // 14; 6750 in 1M 45 / 14; 100k in 1M 15.7 / 15.0 (the radix form: 35, 90, 33, 72, 71, 74).
-int tableBlocks(int slotBlocks, int cells);
+int tableBlocks(int slotBlocks, int cells, int smCount);
 // Keys and counts of n slots at pos, into zero counts.
 void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc);
 // The sort stage from the keys and counts: cell table, stable order and gather

@@ -435,7 +435,7 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 // its launches count: 40k 28.8 -> 8.3.
 constexpr int kScanItems = 4;
 constexpr int kScanChunk = kSortThreads * kScanItems;
-constexpr int kScatterBlocks = 1216;  // 8 per SM: each scans the tile sums once
+constexpr int kTableBlocksPerSM = 8;  // each block of the scatter scans the tile sums once
 
 bool useCountingSort(int slots, int cells) { return cells <= max(8LL * slots, 1LL << 20); }
 
@@ -445,8 +445,8 @@ int countTileShift(int cells) {
     return shift;
 }
 
-int tableBlocks(int slotBlocks, int cells) {
-    return std::max(slotBlocks, std::min((cells - 1) / (4 * kSortThreads) + 1, kScatterBlocks));
+int tableBlocks(int slotBlocks, int cells, int smCount) {
+    return std::max(slotBlocks, std::min((cells - 1) / (4 * kSortThreads) + 1, kTableBlocksPerSM * smCount));
 }
 
 int parkedTileShift(int slots) {
@@ -570,8 +570,8 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
     const int parkedTiles = ((blocks - 1) >> cc.parkedShift) + 1;
     launchChained(c.stream, tiles + parkedTiles, kSortThreads, 0, kCellScan, cc, n, nCells, tiles);
-    const int all = tableBlocks(blocks, nCells);
-    launchChained(c.stream, std::min(all, kScatterBlocks), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
+    const int all = tableBlocks(blocks, nCells, c.smCount);
+    launchChained(c.stream, std::min(all, kTableBlocksPerSM * c.smCount), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
                   cellStart);
     launchChained(c.stream, all, kSortThreads, 0, kCellReorder, cc, n, nCells, cellStart, pos, vel, col, mat, amc,
                   pid, posOut, velOut, colOut, matOut, amcOut, pidOut, reinterpret_cast<float*>(pairXY),
