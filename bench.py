@@ -64,7 +64,7 @@ BYTES_PER_SUBSTEP = sum(STAGE_BYTES.values())  # 753
 # csrc_digest(KERNEL_SOURCES[stage])) at the capture. When those sources have
 # changed since, the figure no longer describes the running kernel and is
 # reported as null.
-KERNEL_SOURCES = {"density": ("sf_kernels.cu", "sf_kernels.h", "sf_device.cuh", "sf_neighbors.cuh")}
+KERNEL_SOURCES = {"density": ("sf_kernels.cu", "sf_kernels.h", "sf_count.cuh", "sf_device.cuh", "sf_neighbors.cuh")}
 NCU_TRAFFIC = {"density": (282.0e6, "0abe114f76e1")}
 
 

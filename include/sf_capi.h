@@ -129,7 +129,7 @@ enum {
     SF_FIELD_COL = 3,            /* f32 x3 */
     SF_FIELD_LABEL = 4,          /* i32 */
     SF_FIELD_RADIUS = 5,         /* f32 */
-    SF_FIELD_MASS = 6,           /* f32 */
+    SF_FIELD_MASS = 6,           /* f32; 0 parks the particle: no pass sees it, its id and fields stay */
     SF_FIELD_DENSITY = 7,        /* f32 */
     SF_FIELD_PRESSURE = 8,       /* f32 */
     SF_FIELD_VOIDAGE = 9,        /* f32 */
@@ -236,7 +236,10 @@ sf_status sf_reset_order(sf_handle* h);
 sf_status sf_frame_adaptive(sf_handle* h, float render_interval, int64_t* n_calls_out);
 
 /* Run one pass of the substep (parity testing; the reference's per-pass
- * solver methods). time_arg is the render interval when adaptive != 0, else dt. */
+ * solver methods). time_arg is the render interval when adaptive != 0, else dt.
+ * Like the field calls on device buffers and sf_reset_order it only queues work,
+ * so a caller may capture it into a CUDA graph of its own (with an even number
+ * of sorts and order resets, which swap the buffers that the graph holds). */
 sf_status sf_run_stage(sf_handle* h, int32_t stage, float time_arg, int32_t adaptive);
 
 /* Copy a field of one scene to dst (device pointer when dst_on_device, else
@@ -320,13 +323,16 @@ sf_status sf_get_list_capacity(const sf_handle* h, int32_t* capacity, int64_t* g
 sf_status sf_set_tuning(sf_handle* h, int32_t block_size, int32_t items_per_thread);
 
 /* Threads per particle of the neighbour passes and of the adjoint pair
- * kernels (no reference counterpart): 1, 2, 4 or 8, or 0 for the automatic
- * choice (doubled up to 8 while fewer than 2048 threads per SM would run,
- * i.e. 1 for large scenes; the density pass uses 8 while no more than 1152
- * threads per SM run, else 1, the average-flow pass 8, 2 or 1). The density, average-flow and voidage/adhesion
- * results and the neighbour lists are the same for every value; the
- * momentum sums are grouped differently (FP32 rounding only). Takes effect
- * at the next substep (captured graphs are dropped). */
+ * kernels (no reference counterpart): 1, 2, 4 or 8 for all of them, or 0 for
+ * the automatic choice by the handle's slots: doubled up to 8 while fewer than
+ * 2048 threads per SM would run, i.e. 1 for large scenes; the density pass
+ * uses 8 while no more than 1152 threads per SM run, 4 while no more than 2304,
+ * else 1; the average-flow pass the same, but 2 instead of 1 up to 4096 slots
+ * per SM, and so do the adjoint pair kernels where the first rule gives 1. The
+ * density, average-flow and voidage/adhesion results and the neighbour lists
+ * are the same for every value; the momentum and adjoint sums are grouped
+ * differently (FP32 rounding only). Takes effect at the next substep (captured
+ * graphs are dropped). */
 sf_status sf_set_lanes(sf_handle* h, int32_t lanes);
 
 /* Shared-memory staging of the density pass (no reference counterpart), for
@@ -360,8 +366,8 @@ sf_status sf_get_density_staging(const sf_handle* h, int32_t* staged);
 sf_status sf_autotune(sf_handle* h, float dt, int32_t* block_sizes_out, int32_t* list_capacity_out);
 
 /* The current launch configuration (no reference counterpart): block sizes
- * (6 entries, as sf_autotune), threads per particle of the momentum passes,
- * keys per thread of the radix sort tiles and bits per radix digit (8, or
+ * (6 entries, as sf_autotune), threads per particle of the momentum passes (the
+ * passes before them and the adjoint kernels have their own), keys per thread of the radix sort tiles and bits per radix digit (8, or
  * 9-11 where wider digits save a pass). Any pointer may be NULL. */
 sf_status sf_get_tuning(const sf_handle* h, int32_t* block_sizes_out, int32_t* lanes_out, int32_t* sort_items_out,
                         int32_t* sort_digit_bits_out);

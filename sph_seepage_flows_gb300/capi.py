@@ -323,7 +323,7 @@ class Simulation:
         self._check(self.lib.sf_set_tuning(self.h, int(block_size), int(items_per_thread)))
 
     def set_lanes(self, lanes: int):
-        """sf_set_lanes: threads per particle of the neighbour passes (0 = automatic)."""
+        """sf_set_lanes: threads per particle of all neighbour passes and adjoint pair kernels (0 = automatic)."""
         self._check(self.lib.sf_set_lanes(self.h, int(lanes)))
 
     def autotune(self, dt: float) -> dict:
@@ -335,8 +335,8 @@ class Simulation:
         return {"block_sizes": dict(zip(names, list(bs))), "list_capacity": cap.value, **self.tuning()}
 
     def tuning(self) -> dict:
-        """sf_get_tuning: threads per particle of the neighbour passes, keys per
-        thread of the sort tiles and bits per radix digit currently in use."""
+        """sf_get_tuning: threads per particle of the momentum passes, keys per
+        thread of the radix sort's tiles and bits per digit currently in use."""
         lanes, items, digit = ctypes.c_int32(), ctypes.c_int32(), ctypes.c_int32()
         self._check(self.lib.sf_get_tuning(self.h, None, ctypes.byref(lanes), ctypes.byref(items),
                                            ctypes.byref(digit)))

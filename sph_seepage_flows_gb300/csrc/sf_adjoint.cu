@@ -30,7 +30,8 @@
 //
 // The pair kernels wait on their gathers (position, fields and cotangents of
 // each neighbour), so they walk the lists with the next neighbour's data and
-// the index after it in flight (forLabelNeighbors) within 80 registers. On 12
+// the index after it in flight (forLabelNeighbors), in 48 to 77 registers (held to
+// 80, the voidage and flow pairs to 64). On 12
 // calibration scenes (306k particles, one lane): water 131 -> 100 us, sand
 // pairs 137 -> 95, voidage 101 -> 62, average flow 74 -> 46, density 43 -> 34;
 // with 48 registers the reverse sweep takes 6.1 ms of 10 substeps instead of

@@ -88,8 +88,11 @@ struct SceneState {
 // Programmatic dependent launch: the passes of a substep are a chain of short
 // kernels, each launched while the one before drains (launchChained in
 // sf_kernels.h) and held here until it has finished. Returns i unchanged; what
-// a kernel reads is addressed through it, so that no load, not even one from
-// memory that the kernel itself never writes, can move ahead of the wait.
+// a kernel reads of other kernels' results is addressed through it, so that no
+// such load, not even one from memory that the kernel itself never writes, can
+// move ahead of the wait. (The scenes' descriptions and the table of the blocks'
+// scenes may be loaded earlier: only copies write them, which a launch behind
+// them waits for.)
 __device__ __forceinline__ int afterPrevious(int i) {
     asm volatile("griddepcontrol.wait;" : "+r"(i) : : "memory");
     return i;

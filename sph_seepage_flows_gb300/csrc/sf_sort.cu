@@ -17,7 +17,7 @@
 // the warp leaders of each round). The first pass takes its tile histograms
 // from the key kernel (kKeysHist), and the reorder writes the cell table
 // (cellStart[c] = lower bound of c) as it gathers, so a sort stage of two
-// digit passes is six launches.
+// digit passes is seven launches.
 #include <algorithm>
 
 #include "sf_count.cuh"
@@ -409,7 +409,7 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 
 // ------------------------------------------------- counting sort by cell
 // The sort stage where the cell table is not much larger than the particle
-// arrays (useCountingSort): three or four launches instead of seven or eight.
+// arrays (useCountingSort): three or four launches instead of seven (two digits) or ten.
 //   kCountKeys     the key of every slot and its place among the slots counted
 //                  into its cell (in arrival order); the integrator leaves the
 //                  same for the positions it writes, so this runs only after
