@@ -1358,8 +1358,12 @@ __device__ void refreshDerived(int s, const float4* pos, const float4* vel, cons
     }
 }
 
+// In a list: velocities whose copy in the gather records is all that follows
+// them, as kSetVec3 leaves it.
+constexpr int kVelocityRecords = -1;
+
 // Whether the passes' derived values of a slot depend on a field.
-__device__ __forceinline__ bool hasDerived(int field) {
+__host__ __device__ __forceinline__ bool hasDerived(int field) {
     switch (field) {
     case SF_FIELD_VEL: case SF_FIELD_LABEL: case SF_FIELD_MASS: case SF_FIELD_DENSITY: case SF_FIELD_PRESSURE:
     case SF_FIELD_VOIDAGE: case SF_FIELD_SATURATION:
@@ -1397,12 +1401,15 @@ __device__ __forceinline__ void setField(int field, int s, const FieldArrays& A,
     case SF_FIELD_AVG_ADHESION: set3(A.avgadh); break;
     case SF_FIELD_CDA0ASAT: set3(A.mat); break;
     case SF_FIELD_AMCAMCP: A.amc[s] = make_float2(v.x, v.y); break;
+    case kVelocityRecords: set3(A.vel); set3(A.grec4); break;
     default: break;
     }
 }
 
-// The fields of the list in order, each as if set by a call of its own (what
-// the passes derive from them is no field, so it follows once, at the end).
+// The fields of the list in order, each as if set by a call of its own: what
+// the passes derive from them is no field and a function of all of them, so it
+// follows once, at the end (a list ends before a label or mass that would
+// change which values those are: sf_set_fields).
 __global__ void kSetFields(FieldList list, int n, int slotOff, int order, FieldArrays A,
                            const SceneDev* __restrict__ scene) {
     const int i = blockIdx.x * blockDim.x + afterPrevious(threadIdx.x);
@@ -1745,18 +1752,27 @@ sf_status sf_set_fields(sf_handle* h, int32_t scene, int32_t n_fields, const int
             // vector fields of many particles
             const bool own = st == SF_OK && n_fields > 1 && count > kListSetParticles && order == SF_ORDER_SORTED &&
                              vec3Array(h, fields[k]) && (reinterpret_cast<uintptr_t>(srcs[k]) & 15u) == 0;
-            if (!own && st == SF_OK) {
-                list.add(fields[k], fieldWidth(fields[k]), srcs[k]);
-            }
+            // a label or a mass of 0 changes which derived values a slot has:
+            // those of the fields before it follow first
+            const bool ends = fields[k] == SF_FIELD_LABEL || fields[k] == SF_FIELD_MASS;
+            bool pending = false;
+            for (int q = 0; q < list.n; ++q) pending |= hasDerived(list.field[q]);
             // the fields before an invalid one are set, as by calls of their own
-            if (list.n > 0 && (st || own || list.n == kFieldsPerLaunch || k == n_fields - 1)) {
+            if (list.n > 0 && (st || own || list.n == kFieldsPerLaunch || (ends && pending))) {
                 const sf_status ls = count > 0 ? launchSetFields(h, scene, list, order, count) : SF_OK;
                 list.n = 0;
                 if (ls) return ls;
             }
             if (st) return st;
-            if (own && (st = setFieldQueued(h, scene, fields[k], order, srcs[k], count, 1))) return st;
+            if (own) {
+                if ((st = setFieldQueued(h, scene, fields[k], order, srcs[k], count, 1))) return st;
+                continue;
+            }
+            const bool records = fields[k] == SF_FIELD_VEL && order == SF_ORDER_SORTED &&
+                                 (reinterpret_cast<uintptr_t>(srcs[k]) & 15u) == 0;
+            list.add(records ? kVelocityRecords : fields[k], fieldWidth(fields[k]), srcs[k]);
         }
+        if (list.n > 0 && count > 0) return launchSetFields(h, scene, list, order, count);
         return SF_OK;
     }
     for (int32_t k = 0; k < n_fields; ++k)
