@@ -432,7 +432,7 @@ __global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
         // the list overflows when its two parts meet: from then on
         // nothing reads it, so the order of the two appends is free
         const bool room = cS + cW < L.cap;
-        if (pj.w < 0.f) {
+        if (__float_as_int(pj.w) < 0) {  // by the sign, as the other forms: that of a parked one (-0) too
             if (room) entry(L.nbr, cS) = j;
             ++cS;
             if (!water) {
