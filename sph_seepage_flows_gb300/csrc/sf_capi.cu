@@ -554,7 +554,7 @@ sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive, bool ch
             h->launches += 1;
             h->pairsFresh = true;
         }
-        launchDensity(c, b);
+        launchDensity(c, b, chained);
         break;
     case SF_STAGE_AVGFLOW: launchAvgFlow(c, b, chained); break;
     case SF_STAGE_VOIDAGE_ADHESION: launchVoidageAdhesion(c, b); break;

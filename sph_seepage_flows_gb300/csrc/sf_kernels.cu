@@ -363,7 +363,7 @@ __global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
     kDensity(const SceneDev* __restrict__ scenes, const int* __restrict__ blockScene, SceneState* __restrict__ state,
              NbrListsW L, const float4* __restrict__ pos4, const float4* __restrict__ pairXY,
              const float2* __restrict__ pairZ, const float4* __restrict__ bpos4, float4* __restrict__ vel4,
-             float4* __restrict__ aux4) {
+             float4* __restrict__ aux4, bool chained) {
     SF_SLOT_PROLOGUE
     extern __shared__ uint2 sHits[];
     if (slot == S.slot_off) state[sid].amax_bits = 0u;
@@ -562,7 +562,7 @@ __global__ void __launch_bounds__(kSlotAlign, kAhead ? 4 : 5)
     }
     vel4[slot].w = density;
     float4& aux = aux4[slot];
-    if (water)
+    if (water || !chained)
         aux.x = pressure;
     else
         *reinterpret_cast<float2*>(&aux) = make_float2(pressure, 1.f - sum);
@@ -741,7 +741,8 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
                                                             SceneState* __restrict__ state, NbrListsW L,
                                                             const float4* __restrict__ pos4,
                                                             const float4* __restrict__ bpos4,
-                                                            float4* __restrict__ vel4, float4* __restrict__ aux4) {
+                                                            float4* __restrict__ vel4, float4* __restrict__ aux4,
+                                                            bool chained) {
     SF_SLOT_PROLOGUE_G
     if (part == 0 && slot == S.slot_off) state[sid].amax_bits = 0u;
     const float4 pi4 = pos4[slot];
@@ -967,7 +968,7 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
     if (water) pressure = pressureOf(S, density);
     vel4[slot].w = density;
     aux4[slot].x = pressure;
-    if (!water) aux4[slot].y = 1.f - sandVolume;
+    if (!water && chained) aux4[slot].y = 1.f - sandVolume;
 }
 
 // ------------------------------------------------------------ avg-flow stage
@@ -979,7 +980,7 @@ __global__ void __launch_bounds__(kSlotAlign) kDensityLanes(const SceneDev* __re
 // stay bit-identical. kSummed: the density pass, run just before on the same
 // state, left the fluid voidage of sand in aux.y, so sand has no sand
 // neighbours to visit (a stage run by itself sums them from the densities it
-// finds). That was most of this pass's work: 93 -> 30 us on
+// finds, and a density stage run by itself leaves aux.y alone). That was most of this pass's work: 93 -> 30 us on
 // the 1M embankment, for 26 us more in the density pass.
 template <int G, bool kSummed>
 __global__ void __launch_bounds__(kSlotAlign, 4) kAvgFlow(const SceneDev* __restrict__ scenes,
@@ -1329,15 +1330,15 @@ void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, co
     kBoundaryVolume<<<(nb + 255) / 256, 256, 0, c.stream>>>(c.scenes, sid, bpos4, blabel, bcs);
 }
 
-template <int G> void launchDensityLanes(const LaunchCtx& c, const PassBuffers& b) {
+template <int G> void launchDensityLanes(const LaunchCtx& c, const PassBuffers& b, bool chained) {
     launchChained(c.stream, grid(c, kPassDensity) * G, c.block[kPassDensity], 0, kDensityLanes<G>, c.scenes,
-                  c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4);
+                  c.blockScene, c.state, b.listsW, b.pos4, b.bpos4, b.vel4, b.aux4, chained);
 }
-void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
+void launchDensity(const LaunchCtx& c, const PassBuffers& b, bool chained) {
     switch (c.lanes[kPassDensity]) {
-    case 2: launchDensityLanes<2>(c, b); break;
-    case 4: launchDensityLanes<4>(c, b); break;
-    case 8: launchDensityLanes<8>(c, b); break;
+    case 2: launchDensityLanes<2>(c, b, chained); break;
+    case 4: launchDensityLanes<4>(c, b, chained); break;
+    case 8: launchDensityLanes<8>(c, b, chained); break;
     default:
         if (c.densityStaged) {
             // 14 positions per thread (a block of 128 consecutive slots
@@ -1349,7 +1350,7 @@ void launchDensity(const LaunchCtx& c, const PassBuffers& b) {
             const size_t hits = size_t(kHitChunks) * c.block[kPassDensity] * sizeof(uint2);
             const auto kernel = c.slotBlocks <= kAheadSlotsPerSM * c.smCount / kSlotAlign ? kDensity<true> : kDensity<false>;
             launchChained(c.stream, grid(c, kPassDensity), c.block[kPassDensity], hits, kernel, c.scenes,
-                          c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4);
+                          c.blockScene, c.state, b.listsW, b.pos4, b.pairXY, b.pairZ, b.bpos4, b.vel4, b.aux4, chained);
         }
         break;
     }

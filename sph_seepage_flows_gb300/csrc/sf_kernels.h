@@ -178,8 +178,9 @@ int flowLanesForSlots(long long totalSlots, int smCount);
 
 void launchBoundaryVolume(const LaunchCtx& c, int sid, int nb, float4* bpos4, const int* blabel,
                           const unsigned int* bcs);
-void launchDensity(const LaunchCtx& c, const PassBuffers& b);
-// chained: the density pass ran just before, with nothing set in between
+// chained: the average flow follows at once, and takes the sand volume summed here
+void launchDensity(const LaunchCtx& c, const PassBuffers& b, bool chained);
+// chained: the density pass ran just before (chained), with nothing set in between
 void launchAvgFlow(const LaunchCtx& c, const PassBuffers& b, bool chained);
 void launchVoidageAdhesion(const LaunchCtx& c, const PassBuffers& b);
 void launchSandMomentum(const LaunchCtx& c, const PassBuffers& b);
