@@ -432,7 +432,8 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 // Sort stage against the radix sort: 1M embankment 77.5 -> 51.6 us (keys 10,
 // scan 3, scatter 8, reorder 27 of 190 MB through L2), and 42 behind an integrator
 // that counted; 252k 40.9 -> 13.6, 64-scene ensemble 86 -> 49; on small scenes
-// its launches count: 40k 28.8 -> 8.3.
+// its launches count: 40k 28.8 -> 8.3. (Ranking the parked slots has since added
+// 0.2 to 0.7 us.)
 constexpr int kScanItems = 4;
 constexpr int kScanChunk = kSortThreads * kScanItems;
 constexpr int kTableBlocksPerSM = 8;  // each block of the scatter scans the tile sums once
