@@ -223,10 +223,13 @@ struct sf_handle {
     // positions as they are (left by the integrator or the key kernel), or of
     // positions that have changed since
     enum { kCountsZero, kCountsReady, kCountsStale } counts = kCountsZero;
-    // Both are what the calls so far left on the device. A caller may also
-    // capture calls into a graph of its own and replay it at any time, which no
-    // call here sees, so the calls that rely on the two begin with track():
-    // they hold within one capture, and between calls only while the caller has
+    // whether a caller ever set masses (a mass of 0 parks a particle), and whether
+    // no slot was parked, taken back or added since the last sort
+    bool massesSet = false, parkedInPlace = false;
+    // All of these are what the calls so far left on the device. A caller may
+    // also capture calls into a graph of its own and replay it at any time, which
+    // no call here sees, so the calls that rely on them begin with track(): they
+    // hold within one capture, and between calls only while the caller has
     // captured none.
     unsigned long long captureId = 0;  // of the caller's capture that the last tracked call was part of
     bool callerCaptures = false;
@@ -357,22 +360,34 @@ struct sf_handle {
     void track() {
         cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
         unsigned long long id = 0;
-        if (cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess) (void)cudaGetLastError();
-        trackIn(status == cudaStreamCaptureStatusActive ? id : 0);
+        if (cudaStreamIsCapturing(stream, &status) != cudaSuccess ||
+            (status == cudaStreamCaptureStatusActive && cudaStreamGetCaptureInfo(stream, &status, &id) != cudaSuccess))
+            (void)cudaGetLastError();
+        trackIn(id);
     }
     // id: of the capture that the call is part of, 0 where it can be part of
     // none (it launches a graph or waits, which a capture refuses)
     void trackIn(unsigned long long id) {
         if (id) callerCaptures = true;
         if (callerCaptures && (id == 0 || id != captureId)) {
-            pairsFresh = false;
+            positionsChanged();
             counts = kCountsStale;
         }
         captureId = id;
     }
+    // a captured substep was replayed, integrator included
+    void replayed() {
+        sorted = true;
+        pairsFresh = false;
+        parkedInPlace = true;
+        if (countingSort) counts = kCountsReady;
+    }
+    // whether there may be particles that a mass of 0 parked
+    bool parkedParticles() const { return massesSet || callerCaptures; }
     // positions or buffers changed outside the substep's passes
     void positionsChanged() {
         pairsFresh = false;
+        parkedInPlace = false;
         if (counts == kCountsReady) counts = kCountsStale;
     }
     CountScratch countScratch() const {
@@ -503,8 +518,7 @@ sf_status ensureCounts(sf_handle* h) {
     if (!h->countingSort || h->counts == sf_handle::kCountsReady) return SF_OK;
     if (h->counts == sf_handle::kCountsStale)
         if (sf_status st = clearCounts(h)) return st;
-    launchCountKeys(h->ctx(), h->totalSlots, h->pos[h->cur], h->countScratch());
-    h->launches += 1;
+    h->launches += launchCountKeys(h->ctx(), h->totalSlots, h->pos[h->cur], h->countScratch(), h->parkedParticles());
     h->counts = sf_handle::kCountsReady;
     return h->cuda(cudaGetLastError(), "count keys launch");
 }
@@ -523,7 +537,7 @@ sf_status runSort(sf_handle* h) {
                                           h->amc[t], h->pid[t], h->cs, h->pairXY, h->pairZ);
         h->counts = sf_handle::kCountsZero;
         h->sortedKeys = cc.sortedKeys;
-        h->pairsFresh = true;
+        h->pairsFresh = h->parkedInPlace = true;
         h->cur = t;
         h->sorted = true;
         return h->cuda(cudaGetLastError(), "sort stage launch");
@@ -560,14 +574,20 @@ sf_status runStage(sf_handle* h, int stage, float timeArg, int adaptive, bool ch
     case SF_STAGE_VOIDAGE_ADHESION: launchVoidageAdhesion(c, b); break;
     case SF_STAGE_SAND_MOMENTUM: launchSandMomentum(c, b); break;
     case SF_STAGE_WATER_MOMENTUM: launchWaterMomentum(c, b); break;
-    case SF_STAGE_INTEGRATE:
-        if (h->countingSort && h->counts != sf_handle::kCountsZero)  // no sort since the last count
+    case SF_STAGE_INTEGRATE: {
+        // (slots parked since the last sort are not where the integrator takes them to go)
+        const bool count = h->countingSort && (h->parkedInPlace || !h->parkedParticles());
+        if (count && h->counts != sf_handle::kCountsZero)  // no sort since the last count
             if (sf_status st = clearCounts(h)) return st;
         launchIntegrate(c, b, timeArg, adaptive, h->captureStep ? h->dTimeArg : nullptr,
-                        h->countingSort ? h->countScratch() : CountScratch{});
+                        count ? h->countScratch() : CountScratch{});
         h->pairsFresh = false;
-        if (h->countingSort) h->counts = sf_handle::kCountsReady;
+        if (count)
+            h->counts = sf_handle::kCountsReady;
+        else if (h->counts == sf_handle::kCountsReady)
+            h->counts = sf_handle::kCountsStale;
         break;
+    }
     default: return h->fail(SF_ERR_INVALID, "unknown stage");
     }
     h->launches += 1;
@@ -1035,6 +1055,7 @@ static sf_status ensureStepGraph(sf_handle* h, GraphCache& g) {
     const cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
     h->cur = curBefore;
     h->counts = countsBefore;
+    h->parkedInPlace = false;
     g.nodes = int(h->launches - launchesBefore);
     h->launches = launchesBefore;
     if (st != SF_OK) {
@@ -1073,9 +1094,7 @@ sf_status sf_step(sf_handle* h, float render_interval, int64_t* n_substeps_out, 
     if (h->cuda(cudaGraphLaunch(g.exec, h->stream), "graph launch")) return SF_ERR_CUDA;
     h->launches += g.nodes;
     h->cur = 1 - h->cur;
-    h->sorted = true;
-    h->pairsFresh = false;
-    if (h->countingSort) h->counts = sf_handle::kCountsReady;
+    h->replayed();
     const int copy = queueStateCopy(h);
     if (ms_out) {
         cudaEventRecord(e1, h->stream);
@@ -1136,6 +1155,7 @@ static sf_status ensureGraph(sf_handle* h, GraphCache& g, int nsub, float dt) {
     cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
     h->cur = curBefore;
     h->counts = countsBefore;
+    h->parkedInPlace = false;
     g.nodes = int(h->launches - launchesBefore);
     h->launches = launchesBefore;
     if (st != SF_OK) {
@@ -1171,9 +1191,7 @@ sf_status queueSubstepsFixed(sf_handle* h, float dt, int64_t n) {
             h->launches += g.nodes;
         }
     }
-    h->sorted = true;
-    h->pairsFresh = false;
-    if (h->countingSort) h->counts = sf_handle::kCountsReady;
+    h->replayed();
     return SF_OK;
 }
 
@@ -1693,9 +1711,15 @@ bool movesParticles(int field) {
 }
 
 sf_status launchSetFields(sf_handle* h, int32_t scene, const FieldList& list, int32_t order, int64_t n) {
-    h->track();
-    for (int k = 0; k < list.n; ++k)
-        if (movesParticles(list.field[k])) h->positionsChanged();
+    bool moves = false;
+    for (int k = 0; k < list.n; ++k) {
+        moves |= movesParticles(list.field[k]);
+        h->massesSet |= list.field[k] == SF_FIELD_MASS;
+    }
+    if (moves) {
+        h->track();
+        h->positionsChanged();
+    }
     launchChained(h->stream, int((n + 255) / 256), 256, 0, list.n == 1 ? kSetField : kSetFields, list,
                   int(n), h->hScenes[scene].slot_off, order, fieldArrays(h), h->dScenes + scene);
     return h->cuda(cudaGetLastError(), "set_field launch");
@@ -1723,8 +1747,10 @@ sf_status setFieldQueued(sf_handle* h, int32_t scene, int32_t field, int32_t ord
     float4* vec = order == SF_ORDER_SORTED ? vec3Array(h, field) : nullptr;
     if (!vec || (reinterpret_cast<uintptr_t>(from) & 15u) != 0)
         return launchSetFields(h, scene, oneField(field, from), order, n);
-    h->track();
-    if (movesParticles(field)) h->positionsChanged();
+    if (movesParticles(field)) {
+        h->track();
+        h->positionsChanged();
+    }
     kSetVec3<<<int((n + kVecParticles - 1) / kVecParticles), kVecParticles, 0, h->stream>>>(
         int(n), h->hScenes[scene].slot_off, vec, static_cast<const float4*>(from),
         field == SF_FIELD_VEL ? h->grec4 : nullptr);
@@ -1921,7 +1947,7 @@ sf_status sf_reset_order(sf_handle* h) {
     h->launches += 1;
     h->cur = t;
     h->sorted = false;
-    h->pairsFresh = false;
+    h->positionsChanged();
     h->counts = sf_handle::kCountsZero;
     return h->cuda(cudaGetLastError(), "reset order launch");
 }
@@ -2299,6 +2325,7 @@ sf_status runSubstepStoreGraphed(sf_handle* h, float dt, int64_t t) {
         cudaError_t ce = cudaStreamEndCapture(h->stream, &graph);
         h->cur = curBefore;
         h->counts = countsBefore;
+        h->parkedInPlace = false;
         g.nodes = int(h->launches - launchesBefore);
         h->launches = launchesBefore;
         if (st != SF_OK) {
@@ -2315,9 +2342,7 @@ sf_status runSubstepStoreGraphed(sf_handle* h, float dt, int64_t t) {
     if (h->cuda(cudaGraphLaunch(g.exec, h->stream), "graph launch")) return SF_ERR_CUDA;
     h->launches += g.nodes;
     h->cur = 1 - h->cur;
-    h->sorted = true;
-    h->pairsFresh = false;
-    if (h->countingSort) h->counts = sf_handle::kCountsReady;
+    h->replayed();
     return SF_OK;
 }
 

@@ -190,6 +190,7 @@ struct CountScratch {
     unsigned int* count;       // nCells rounded up to a multiple of 4
     unsigned int* tileCount;   // kMaxCountTiles: slots per table tile
     uint2* keyRank;            // n: key of each slot before the sort, place among the slots counted into its cell
+                               // (of a parked slot: the slot it goes to)
     unsigned char* parkedInWarp;  // n / 32: parked slots of each 32
     unsigned int* parkedBefore;   // n / 256: parked slots before each block of 256, within its tile of blocks
     unsigned int* parkedTile;     // kMaxParkedTiles: parked slots of each tile of blocks
@@ -269,8 +270,9 @@ int parkedTileShift(int slots);
 // 250 slots in 97k cells 94 / 9 us, in 1M 895 / 12; 2000 in 97k 20 / 11, in 1M 121 /
 // 14; 6750 in 1M 45 / 14; 100k in 1M 15.7 / 15.0 (the radix form: 35, 90, 33, 72, 71, 74).
 int tableBlocks(int slotBlocks, int cells, int smCount);
-// Keys and counts of n slots at pos, into zero counts.
-void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc);
+// Keys and counts of n slots at pos, into zero counts. ranked: parked slots may
+// have to go to another place (countSlot). Returns kernels launched.
+int launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc, bool ranked);
 // The sort stage from the keys and counts: cell table, stable order and gather
 // of the persistent arrays (with the slot-pair positions); the counts are zero
 // afterwards. Returns kernels launched.

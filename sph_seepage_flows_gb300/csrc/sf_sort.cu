@@ -414,11 +414,13 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 //                  into its cell (in arrival order); the integrator leaves the
 //                  same for the positions it writes, so this runs only after
 //                  positions came from elsewhere
-//   kCellScan      exclusive scan of the counts within each table tile, and of
-//                  the parked slots over the blocks of slots
+//   kScanParked,   after masses were set and the slots counted anew: where the
+//   kRankParked    parked slots go, in slot order, as the atomics that count
+//                  them have none
+//   kCellScan      exclusive scan of the counts within each table tile
 //   kCountScatter  adds the slots of the tiles before (the cell table), and
-//                  lists the slots of each cell in arrival order (the parked
-//                  slots in slot order)
+//                  lists the slots of each cell in arrival order, the parked
+//                  slots where they go
 //   kCellReorder   the place of each slot within its cell by slot number (the
 //                  stable order), the gather of the persistent arrays, and the
 //                  counts cleared for the next sort; a non-finite position is
@@ -432,8 +434,7 @@ void launchReorder(cudaStream_t s, int n, const unsigned int* perm, const float4
 // Sort stage against the radix sort: 1M embankment 77.5 -> 51.6 us (keys 10,
 // scan 3, scatter 8, reorder 27 of 190 MB through L2), and 42 behind an integrator
 // that counted; 252k 40.9 -> 13.6, 64-scene ensemble 86 -> 49; on small scenes
-// its launches count: 40k 28.8 -> 8.3. (Ranking the parked slots has since added
-// 0.2 to 0.7 us.)
+// its launches count: 40k 28.8 -> 8.3.
 constexpr int kScanItems = 4;
 constexpr int kScanChunk = kSortThreads * kScanItems;
 constexpr int kTableBlocksPerSM = 8;  // each block of the scatter scans the tile sums once
@@ -458,15 +459,34 @@ int parkedTileShift(int slots) {
 
 __global__ void __launch_bounds__(kSlotAlign) kCountKeys(const SceneDev* __restrict__ scenes,
                                                          const int* __restrict__ blockScene,
-                                                         const float4* __restrict__ pos4, CountScratch cc) {
+                                                         const float4* __restrict__ pos4, CountScratch cc, bool ranked) {
     const int slot = blockIdx.x * kSlotAlign + afterPrevious(threadIdx.x);
-    countSlot(scenes[blockScene[blockIdx.x]], slot, pos4[slot], cc);
+    const float4 p = pos4[slot];
+    countSlot(scenes[blockScene[blockIdx.x]], slot, p, cc);
+    if (ranked) {
+        const unsigned int parked = __ballot_sync(0xffffffffu, p.w == 0.f);
+        if ((threadIdx.x & 31u) == 0u) cc.parkedInWarp[slot >> 5] = static_cast<unsigned char>(__popc(parked));
+    }
 }
 
-// Tile t of the blocks of kSlotAlign slots: exclusive prefix of their parked slots, and its sum.
-__device__ __forceinline__ void scanParked(const CountScratch& cc, int t, int blocks) {
+// Parked slots of the first `warps` warps of a block of kSlotAlign slots.
+__device__ __forceinline__ unsigned int parkedInWarps(const CountScratch& cc, int block, int warps) {
+    static_assert(kSlotAlign == 256, "the counts of a block's warps are one 8-byte word");
+    uint2 w = reinterpret_cast<const uint2*>(cc.parkedInWarp)[block];
+    if (warps < 4) {
+        w.x &= (1u << (8 * warps)) - 1u;
+        w.y = 0u;
+    } else if (warps < 8) {
+        w.y &= (1u << (8 * (warps - 4))) - 1u;
+    }
+    return __dp4a(w.x, 0x01010101u, __dp4a(w.y, 0x01010101u, 0u));
+}
+
+// Block t: tile t of the blocks of kSlotAlign slots, the exclusive prefix of
+// their parked slots and its sum.
+__global__ void __launch_bounds__(kSortThreads) kScanParked(CountScratch cc, int blocks) {
     unsigned int carry = 0u, total;
-    const int end = min((t + 1) << cc.parkedShift, blocks);
+    const int t = afterPrevious(int(blockIdx.x)), end = min((t + 1) << cc.parkedShift, blocks);
     for (int base = t << cc.parkedShift; base < end; base += kScanChunk) {
         const int first = base + int(threadIdx.x) * kScanItems;
         unsigned int v[kScanItems], sum = 0u;
@@ -483,13 +503,27 @@ __device__ __forceinline__ void scanParked(const CountScratch& cc, int t, int bl
     if (threadIdx.x == 0) cc.parkedTile[t] = carry;
 }
 
+// Where each parked slot goes: its scene's parked slots fill the end of the
+// scene's slots in slot order.
+__global__ void __launch_bounds__(kSlotAlign) kRankParked(const SceneDev* __restrict__ scenes,
+                                                          const int* __restrict__ blockScene, CountScratch cc) {
+    const int block = blockIdx.x, slot = block * kSlotAlign + afterPrevious(threadIdx.x);
+    const bool parked = (cc.keyRank[slot].y & kParkedBit) != 0u;
+    const unsigned int warp = __ballot_sync(0xffffffffu, parked);
+    if (!parked) return;
+    const SceneDev& S = scenes[blockScene[block]];
+    const int first = S.slot_off / kSlotAlign;
+    unsigned int place = cc.parkedBefore[block] - cc.parkedBefore[first] + parkedInWarps(cc, block, int(threadIdx.x >> 5)) +
+                         unsigned(__popc(warp & ((1u << (threadIdx.x & 31u)) - 1u)));
+    for (int t = first >> cc.parkedShift; t < block >> cc.parkedShift; ++t) place += cc.parkedTile[t];
+    cc.keyRank[slot].y = kParkedBit | (unsigned(S.slot_off + S.slot_cap) - cc.count[S.cell_off + S.ncell] + place);
+}
+
 // Block b scans table tile b (2^tileShift cells, a multiple of kScanChunk) in
-// place and writes its sum; the blocks behind the tiles scan the parked slots.
-__global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int n, int nCells, int tiles) {
+// place and writes its sum.
+__global__ void __launch_bounds__(kSortThreads) kCellScan(CountScratch cc, int nCells) {
     unsigned int carry = 0u, total;
-    const int tile = afterPrevious(int(blockIdx.x));
-    if (tile >= tiles) return scanParked(cc, tile - tiles, n / kSlotAlign);
-    const int tileBeg = tile << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
+    const int tileBeg = afterPrevious(int(blockIdx.x)) << cc.tileShift, tileEnd = min(tileBeg + (1 << cc.tileShift), nCells);
     for (int base = tileBeg; base < tileEnd; base += kScanChunk) {
         const int c = base + int(threadIdx.x) * kScanItems;
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -517,9 +551,10 @@ __global__ void __launch_bounds__(kSortThreads) kCountScatter(CountScratch cc, i
     __syncthreads();
     const int first = blockIdx.x * kSortThreads + tid, threads = gridDim.x * kSortThreads;
     for (int i = first; i < n; i += threads) {
-        uint2 kr = cc.keyRank[i];
-        if (kr.y & kParkedBit) kr.y = parkedPlace(cc, i, kr.y);
-        cc.arrived[cc.count[kr.x] + before[kr.x >> cc.tileShift] + kr.y] = unsigned(i);
+        const uint2 kr = cc.keyRank[i];
+        const unsigned int at = kr.y & kParkedBit ? kr.y & ~kParkedBit
+                                                  : cc.count[kr.x] + before[kr.x >> cc.tileShift] + kr.y;
+        cc.arrived[at] = unsigned(i);
     }
     for (int c = first; c < nCells; c += threads) cs[c] = cc.count[c] + before[c >> cc.tileShift];
     if (first == 0) cs[nCells] = unsigned(n);
@@ -542,7 +577,7 @@ __global__ void __launch_bounds__(kSortThreads)
     const unsigned int key = cc.keyRank[o].x;
     unsigned int d = unsigned(i);
     checkPosition(p, errWord);
-    if (p.w != 0.f) {  // the parked slots are listed in slot order
+    if (p.w != 0.f) {  // the parked slots are listed where they go
         const unsigned int beg = cs[key], end = cs[key + 1];
         d = beg;
         for (unsigned int q = beg; q < end; ++q) d += cc.arrived[q] < o ? 1u : 0u;
@@ -560,8 +595,13 @@ __global__ void __launch_bounds__(kSortThreads)
     pairZ[d] = p.z;
 }
 
-void launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc) {
-    launchChained(c.stream, n / kSlotAlign, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc);
+int launchCountKeys(const LaunchCtx& c, int n, const float4* pos, const CountScratch& cc, bool ranked) {
+    const int blocks = n / kSlotAlign;
+    launchChained(c.stream, blocks, kSlotAlign, 0, kCountKeys, c.scenes, c.blockScene, pos, cc, ranked);
+    if (!ranked) return 1;
+    launchChained(c.stream, ((blocks - 1) >> cc.parkedShift) + 1, kSortThreads, 0, kScanParked, cc, blocks);
+    launchChained(c.stream, blocks, kSlotAlign, 0, kRankParked, c.scenes, c.blockScene, cc);
+    return 3;
 }
 
 int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch& cc, const float4* pos,
@@ -569,8 +609,7 @@ int launchCountingSort(const LaunchCtx& c, int n, int nCells, const CountScratch
                        float4* posOut, float4* velOut, float4* colOut, float4* matOut, float2* amcOut, int* pidOut,
                        unsigned int* cellStart, float4* pairXY, float2* pairZ) {
     const int blocks = n / kSlotAlign, tiles = ((nCells - 1) >> cc.tileShift) + 1;
-    const int parkedTiles = ((blocks - 1) >> cc.parkedShift) + 1;
-    launchChained(c.stream, tiles + parkedTiles, kSortThreads, 0, kCellScan, cc, n, nCells, tiles);
+    launchChained(c.stream, tiles, kSortThreads, 0, kCellScan, cc, nCells);
     const int all = tableBlocks(blocks, nCells, c.smCount);
     launchChained(c.stream, std::min(all, kTableBlocksPerSM * c.smCount), kSortThreads, 0, kCountScatter, cc, n, nCells, tiles,
                   cellStart);

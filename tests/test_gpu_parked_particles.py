@@ -86,3 +86,33 @@ def test_parked_particles_through_substeps(cuda_lib, block):
     for o in outs[1:]:
         for k, v in o.items():
             assert np.array_equal(v, outs[0][k]), k
+
+
+@pytest.mark.parametrize("side", [0.4, 6.0])
+def test_particles_parked_between_stages_by_hand(cuda_lib, side):
+    """Masses set, taken back and particles added right before an integration run by hand: the sort after it is numpy's
+    stable order of what the integration left, in both forms."""
+    from sph_seepage_flows_gb300.capi import Simulation
+    sc = make_scene(2000, side, 7)
+    sim = Simulation(sc, capacity=sc.n + 200)
+    rng = np.random.default_rng(3)
+    for turn in range(5):
+        sim.stage("sort")
+        n = sim.size()
+        if turn:
+            mass = sim.field("mass", order="id")
+            mass[:sc.n] = np.where(park(sc.n, rng) & (turn < 4), np.float32(0), sc.mass)
+            sim.set_field("mass", mass, order="id")
+        if turn in (0, 2):
+            sim.add_sph_particles(rng.uniform(0.05, 0.35, (30, 3)), [0, 0, 1], [0, 0, 0], float(sc.params.sph_mass), 0.01)
+        ids = sim.field("id")
+        assert np.array_equal(np.sort(ids), np.arange(sim.size())) and sim.size() - n == 30 * (turn in (0, 2))
+        sim.stage("integrate", 1e-6)
+        mass = sim.field("mass", order="id")
+        sim.stage("sort")
+        keys, cells = keys_of(sc, sim.field("pos", order="id"))
+        keys = np.where(mass == 0, cells, keys)
+        want = ids[np.argsort(keys[ids], kind="stable")]
+        assert np.array_equal(sim.field("id"), want), turn
+        assert np.array_equal(sim.field("key"), keys[want]), turn
+        assert np.array_equal(sim.cell_table(0), np.searchsorted(keys[want], np.arange(cells + 1))), turn
