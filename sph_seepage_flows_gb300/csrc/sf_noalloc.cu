@@ -151,15 +151,15 @@ sf_status failWith(sf_status st, const std::string& msg) {
     return st;
 }
 
-// What the runtime knows about p on the current device: its type and device.
-cudaPointerAttributes attributesOf(const void* p) {
+// Whether the runtime knows p as registered host memory.
+bool isRegistered(const void* p) {
     cudaPointerAttributes a{};
-    a.type = cudaMemoryTypeUnregistered;
-    if (p && cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    if (!p) return false;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
         (void)cudaGetLastError();  // not sticky: clear it so later checks see only their own errors
-        a.type = cudaMemoryTypeUnregistered;
+        return false;
     }
-    return a;
+    return a.type == cudaMemoryTypeHost;
 }
 
 // What a call uses of a device.
@@ -185,15 +185,14 @@ bool scratchOf(int device, Scratch& out, std::string& why) {
     std::lock_guard<std::mutex> lock(mu);
     if (device < 0 || device >= kMaxDevices) return why = "device index out of range", false;
     Scratch& k = known[device];
-    const cudaPointerAttributes w = attributesOf(k.words);
-    if (attributesOf(k.report).type != cudaMemoryTypeHost || w.type != cudaMemoryTypeDevice || w.device != device) {
+    if (!k.words || !isRegistered(k.report)) {
         const size_t page = size_t(sysconf(_SC_PAGESIZE));
         void* p = k.report;
         if (!p && posix_memalign(&p, page, page) != 0) return why = "no host memory for the report page", false;
         k.report = static_cast<Report*>(p);
         k.words = nullptr;
         cudaError_t e = cudaSuccess;
-        if (attributesOf(p).type != cudaMemoryTypeHost &&
+        if (!isRegistered(p) &&
             (e = cudaHostRegister(p, page, cudaHostRegisterMapped)) != cudaSuccess)
             return why = std::string("cudaHostRegister: ") + cudaGetErrorString(e), false;
         void *d = nullptr, *s = nullptr;
